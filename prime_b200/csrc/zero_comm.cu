@@ -112,12 +112,32 @@ __global__ void allreduce_scalars_kernel(PeerTable flag_pads, PeerTable data_pad
 template <typename G>
 __device__ __forceinline__ float ld_grad(const G* p) { return float(*p); }
 
-// Sum of `nvec` 8-element bf16 vectors over the W ranks (rank order), scaled, written as fp32; returns this
-// thread's sum of squares. UNR vectors per thread and step with every peer load issued before the first add:
+// elements of one 16-byte gradient vector as fp32
+template <typename G>
+struct GradVec;
+template <>
+struct GradVec<__nv_bfloat16> {
+    static constexpr int N = 8;
+    static __device__ __forceinline__ void unpack(const uint4& v, float (&f)[8]) {
+        const float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y), c = unpack_bf16x2(v.z), d = unpack_bf16x2(v.w);
+        f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+    }
+};
+template <>
+struct GradVec<float> {
+    static constexpr int N = 4;
+    static __device__ __forceinline__ void unpack(const uint4& v, float (&f)[4]) {
+        f[0] = __uint_as_float(v.x); f[1] = __uint_as_float(v.y); f[2] = __uint_as_float(v.z); f[3] = __uint_as_float(v.w);
+    }
+};
+
+// Sum of `nvec` 16-byte gradient vectors (8 bf16 or 4 fp32) over the W ranks (rank order), scaled, written as fp32; returns
+// this thread's sum of squares. UNR vectors per thread and step with every peer load issued before the first add:
 // enough bytes in flight for HBM (one rank) and for NVLink (several ranks) alike.
-template <int WMAX, int UNR>
+template <typename G, int WMAX, int UNR>
 __device__ __forceinline__ float reduce_vectors(const PeerTable& peers, int W, long long fo, long long nvec, float scale,
                                                 float* __restrict__ dst, long long b, long long nb) {
+    constexpr int E = GradVec<G>::N;
     float ss = 0.f;
     const long long stride = nb * blockDim.x;
     for (long long i0 = b * blockDim.x + threadIdx.x; i0 < nvec; i0 += UNR * stride) {
@@ -127,30 +147,35 @@ __device__ __forceinline__ float reduce_vectors(const PeerTable& peers, int W, l
             const long long i = i0 + u * stride;
 #pragma unroll
             for (int r = 0; r < WMAX; ++r)
-                if (r < W && i < nvec) v[u][r] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(peers.ptr[r]) + fo) + i);
+                if (r < W && i < nvec) v[u][r] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const G*>(peers.ptr[r]) + fo) + i);
         }
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
             const long long i = i0 + u * stride;
             if (i < nvec) {
-                float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                float acc[E] = {};
 #pragma unroll
                 for (int r = 0; r < WMAX; ++r)
                     if (r < W) {
-                        const float2 a = unpack_bf16x2(v[u][r].x), b = unpack_bf16x2(v[u][r].y), c = unpack_bf16x2(v[u][r].z), d = unpack_bf16x2(v[u][r].w);
-                        acc[0] += a.x; acc[1] += a.y; acc[2] += b.x; acc[3] += b.y; acc[4] += c.x; acc[5] += c.y; acc[6] += d.x; acc[7] += d.y;
+                        float f[E];
+                        GradVec<G>::unpack(v[u][r], f);
+#pragma unroll
+                        for (int k = 0; k < E; ++k) acc[k] += f[k];
                     }
 #pragma unroll
-                for (int k = 0; k < 8; ++k) { acc[k] *= scale; ss += acc[k] * acc[k]; }
-                reinterpret_cast<float4*>(dst)[2 * i] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-                reinterpret_cast<float4*>(dst)[2 * i + 1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+                for (int k = 0; k < E; ++k) { acc[k] *= scale; ss += acc[k] * acc[k]; }
+#pragma unroll
+                for (int k = 0; k < E; k += 4)
+                    reinterpret_cast<float4*>(dst)[(E / 4) * i + k / 4] = make_float4(acc[k], acc[k + 1], acc[k + 2], acc[k + 3]);
             }
         }
     }
     return ss;
 }
 
-// Reduce-scatter by pull + cast/scale + sum of squares. grid-stride over the segment elements.
+// Reduce-scatter by pull + cast/scale + sum of squares. grid-stride over the segment elements. Bound by HBM (one rank) or
+// NVLink: fp32 gradients take the same 16-byte vectors as bf16 ones (element by element the 1.92 G fp32 gradients
+// of four 10B blocks took 31.2 ms on one rank).
 template <typename G>
 __global__ void __launch_bounds__(256) zero_reduce_grads_kernel(PeerTable peers, SegTable segs, float* __restrict__ grad_shard,
                                                                 float scale, float* __restrict__ sumsq_partial) {
@@ -161,16 +186,16 @@ __global__ void __launch_bounds__(256) zero_reduce_grads_kernel(PeerTable peers,
     long long b, nb;
     my_segment(segs, s, b, nb);
     if (nb > 0) {
+        constexpr int E = GradVec<G>::N;
         const long long n = segs.numel[s];
         const long long fo = segs.full_off[s];
         float* dst = grad_shard + segs.shard_off[s];
-        // vector path: 8 elements per thread per step when everything is 16-byte aligned
-        const bool vec_ok = (fo % 8 == 0) && (segs.shard_off[s] % 4 == 0) && sizeof(G) == 2;
-        const long long nvec = vec_ok ? n / 8 : 0;
-        if (W <= 4) ss += reduce_vectors<4, 4>(peers, W, fo, nvec, scale, dst, b, nb);
-        else if (W <= 8) ss += reduce_vectors<8, 2>(peers, W, fo, nvec, scale, dst, b, nb);
-        else ss += reduce_vectors<MAX_RANKS, 1>(peers, W, fo, nvec, scale, dst, b, nb);
-        for (long long i = nvec * 8 + b * blockDim.x + threadIdx.x; i < n; i += nb * blockDim.x) {
+        const bool vec_ok = (fo % E == 0) && (segs.shard_off[s] % 4 == 0);      // 16-byte aligned on both sides
+        const long long nvec = vec_ok ? n / E : 0;
+        if (W <= 4) ss += reduce_vectors<G, 4, 4>(peers, W, fo, nvec, scale, dst, b, nb);
+        else if (W <= 8) ss += reduce_vectors<G, 8, 2>(peers, W, fo, nvec, scale, dst, b, nb);
+        else ss += reduce_vectors<G, MAX_RANKS, 1>(peers, W, fo, nvec, scale, dst, b, nb);
+        for (long long i = nvec * E + b * blockDim.x + threadIdx.x; i < n; i += nb * blockDim.x) {
             float acc = 0.f;
             for (int r = 0; r < W; ++r) acc += ld_grad(reinterpret_cast<const G*>(peers.ptr[r]) + fo + i);
             acc *= scale;
@@ -188,6 +213,69 @@ __global__ void __launch_bounds__(256) zero_reduce_grads_kernel(PeerTable peers,
     }
 }
 
+// Squared global norm of one rank's own gradient buffer, for runs without peers: one read of the gradients, no fp32 copy.
+// The last CTA to finish adds the per-CTA partials in a fixed tree (thread t takes partials t, t + 256, ...), so the result
+// is bit-reproducible and needs no second launch. `counter` is zero between launches.
+template <typename G>
+__global__ void __launch_bounds__(256) grad_sumsq_kernel(const G* __restrict__ grads, SegTable segs, float* __restrict__ partial,
+                                                         unsigned* counter, float* __restrict__ out) {
+    __shared__ float red[8];
+    __shared__ bool last;
+    constexpr int E = GradVec<G>::N, UNR = 8;
+    float ss = 0.f;
+    int s;
+    long long b, nb;
+    my_segment(segs, s, b, nb);
+    if (nb > 0) {
+        const long long n = segs.numel[s], fo = segs.full_off[s];
+        const long long nvec = fo % E == 0 ? n / E : 0;
+        const long long stride = nb * blockDim.x;
+        const uint4* src = reinterpret_cast<const uint4*>(grads + fo);
+        for (long long i0 = b * blockDim.x + threadIdx.x; i0 < nvec; i0 += UNR * stride) {
+            uint4 v[UNR];
+#pragma unroll
+            for (int u = 0; u < UNR; ++u) v[u] = i0 + u * stride < nvec ? __ldg(src + i0 + u * stride) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int u = 0; u < UNR; ++u) {
+                float f[E];
+                GradVec<G>::unpack(v[u], f);
+#pragma unroll
+                for (int k = 0; k < E; ++k) ss += f[k] * f[k];
+            }
+        }
+        for (long long i = nvec * E + b * blockDim.x + threadIdx.x; i < n; i += stride) {
+            const float f = float(grads[fo + i]);
+            ss += f * f;
+        }
+    }
+    auto block_sum = [&](float v) {
+        v = warp_sum(v);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t += red[i];
+        __syncthreads();
+        return t;
+    };
+    const float mine = block_sum(ss);
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x] = mine;
+        __threadfence();
+        last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    float t = 0.f;
+    for (int i = threadIdx.x; i < int(gridDim.x); i += 256) t += __ldcg(partial + i);
+    t = block_sum(t);
+    if (threadIdx.x == 0) {
+        out[0] = t;
+        *counter = 0u;
+    }
+}
+
 // fixed-order sum of `n` partials -> out[0] (+)=
 __global__ void reduce_partials_kernel(const float* __restrict__ partial, int n, float* __restrict__ out, int accumulate) {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
@@ -197,9 +285,13 @@ __global__ void reduce_partials_kernel(const float* __restrict__ partial, int n,
     }
 }
 
-// Sharded AdamW + push all-gather. gnorm_sq: device scalar with the GLOBAL sum of squared grads.
+// Sharded AdamW + push all-gather. gnorm_sq: device scalar with the GLOBAL sum of squared grads. HBM-bound. FULL: the
+// gradients are read from the rank's own full gradient buffer (bf16 or fp32, at the segment's full offset) instead of the
+// reduced fp32 shard: without peers there is nothing to reduce, which saves the fp32 copy's write and read (28 instead of
+// 36 bytes per bf16-gradient parameter over the whole update).
+template <typename G, bool FULL>
 __global__ void __launch_bounds__(256) zero_adamw_gather_kernel(PeerTable params, SegTable segs, float* __restrict__ master,
-                                                                const float* __restrict__ grad_shard, float* __restrict__ m,
+                                                                const G* __restrict__ grad, float* __restrict__ m,
                                                                 float* __restrict__ v, float lr, float beta1, float beta2, float eps,
                                                                 float wd, float bc1, float bc2, const float* __restrict__ gnorm_sq,
                                                                 float max_norm) {
@@ -214,7 +306,8 @@ __global__ void __launch_bounds__(256) zero_adamw_gather_kernel(PeerTable params
     my_segment(segs, s, b, nb);
     if (nb > 0) {
         const long long n = segs.numel[s], fo = segs.full_off[s], so = segs.shard_off[s];
-        const bool vec_ok = (fo % 8 == 0) && (so % 4 == 0);
+        const G* gsrc = grad + (FULL ? fo : so);
+        const bool vec_ok = (fo % 8 == 0) && (so % 4 == 0);      // covers the gradients: 8 elements of fo, or 4 fp32 of so
         const long long nvec = vec_ok ? n / 8 : 0;
         // two 8-element vectors per thread and step: sixteen 16-byte streaming loads are issued before the first use
         const long long stride = nb * blockDim.x;
@@ -227,10 +320,11 @@ __global__ void __launch_bounds__(256) zero_adamw_gather_kernel(PeerTable params
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         *reinterpret_cast<float4*>(p[u] + 4 * h) = __ldcs(reinterpret_cast<const float4*>(master + so) + 2 * i + h);
-                        *reinterpret_cast<float4*>(g[u] + 4 * h) = __ldcs(reinterpret_cast<const float4*>(grad_shard + so) + 2 * i + h);
+                        if constexpr (sizeof(G) == 4) *reinterpret_cast<float4*>(g[u] + 4 * h) = __ldcs(reinterpret_cast<const float4*>(gsrc) + 2 * i + h);
                         *reinterpret_cast<float4*>(mm[u] + 4 * h) = __ldcs(reinterpret_cast<const float4*>(m + so) + 2 * i + h);
                         *reinterpret_cast<float4*>(vv[u] + 4 * h) = __ldcs(reinterpret_cast<const float4*>(v + so) + 2 * i + h);
                     }
+                    if constexpr (sizeof(G) == 2) GradVec<__nv_bfloat16>::unpack(__ldcs(reinterpret_cast<const uint4*>(gsrc) + i), g[u]);
                 }
             }
 #pragma unroll
@@ -263,7 +357,7 @@ __global__ void __launch_bounds__(256) zero_adamw_gather_kernel(PeerTable params
             }
         }
         for (long long i = nvec * 8 + b * blockDim.x + threadIdx.x; i < n; i += nb * blockDim.x) {
-            const float gi = grad_shard[so + i] * clip;
+            const float gi = float(gsrc[i]) * clip;
             float pi = master[so + i] * (1.f - lr * wd);
             const float mi = beta1 * m[so + i] + (1.f - beta1) * gi;
             const float vi = beta2 * v[so + i] + (1.f - beta2) * gi * gi;
@@ -411,18 +505,39 @@ extern "C" int pb_zero_reduce_grads(void* const* peer_grads, int world, int rank
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }
 
+// grad: fp32 shard (grad_kind 0, indexed by shard_off), or the rank's full gradient buffer in bf16 (1) or fp32 (2), indexed by
+// full_off.
 extern "C" int pb_zero_adamw_gather(void* const* peer_params, int world, int rank, int nseg, const long long* full_off,
-                                    const long long* shard_off, const long long* numel, float* master, const float* grad_shard,
+                                    const long long* shard_off, const long long* numel, float* master, const void* grad, int grad_kind,
                                     float* m, float* v, float lr, float beta1, float beta2, float eps, float wd, int step,
                                     const float* gnorm_sq, float max_norm, int ctas, void* stream) {
-    if (world > MAX_RANKS || nseg > MAX_SEGS) return -1;
+    if (world > MAX_RANKS || nseg > MAX_SEGS || grad_kind < 0 || grad_kind > 2) return -1;
     const float bc1 = 1.f - powf(beta1, float(step));
     const float bc2 = sqrtf(1.f - powf(beta2, float(step)));
     if (ctas < nseg) ctas = nseg;
     const SegTable sg = make_segs(nseg, full_off, shard_off, numel, ctas);
     if (sg.cta_begin[nseg] <= 0) return 0;
-    zero_adamw_gather_kernel<<<sg.cta_begin[nseg], 256, 0, ST(stream)>>>(make_peers(peer_params, world, rank), sg, master, grad_shard, m, v,
-                                                                         lr, beta1, beta2, eps, wd, bc1, bc2, gnorm_sq, max_norm);
+    const PeerTable pt = make_peers(peer_params, world, rank);
+    auto launch = [&](auto kern, auto* g) {
+        kern<<<sg.cta_begin[nseg], 256, 0, ST(stream)>>>(pt, sg, master, g, m, v, lr, beta1, beta2, eps, wd, bc1, bc2, gnorm_sq, max_norm);
+    };
+    if (grad_kind == 0) launch(zero_adamw_gather_kernel<float, false>, reinterpret_cast<const float*>(grad));
+    else if (grad_kind == 1) launch(zero_adamw_gather_kernel<__nv_bfloat16, true>, reinterpret_cast<const __nv_bfloat16*>(grad));
+    else launch(zero_adamw_gather_kernel<float, true>, reinterpret_cast<const float*>(grad));
+    return cudaGetLastError() == cudaSuccess ? 0 : -30;
+}
+
+// out[0] = sum of squares of the gradients in these segments of one rank's full buffer. scratch: >= ctas floats;
+// counter: one zero-initialised unsigned that concurrent launches do not share.
+extern "C" int pb_grad_sumsq(const void* grads, int grad_fp32, int nseg, const long long* full_off, const long long* numel, float* scratch,
+                             unsigned* counter, float* out, int ctas, void* stream) {
+    if (nseg > MAX_SEGS || nseg < 1) return -1;
+    if (ctas < nseg) ctas = nseg;
+    const SegTable sg = make_segs(nseg, full_off, full_off, numel, ctas);
+    ctas = sg.cta_begin[nseg];
+    if (ctas <= 0) return -1;
+    if (grad_fp32) grad_sumsq_kernel<float><<<ctas, 256, 0, ST(stream)>>>(reinterpret_cast<const float*>(grads), sg, scratch, counter, out);
+    else grad_sumsq_kernel<__nv_bfloat16><<<ctas, 256, 0, ST(stream)>>>(reinterpret_cast<const __nv_bfloat16*>(grads), sg, scratch, counter, out);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }
 
