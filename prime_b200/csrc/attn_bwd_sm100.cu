@@ -144,6 +144,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_sync();
 
     if (warp < 4) {
         reg_dealloc_64();
@@ -542,6 +543,7 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
                                                             long long do_stride) {
     constexpr int LPR = HD / 8;                       // lanes per row
     constexpr int ROWS_PER_BLOCK = 256 / LPR;
+    pdl_sync();
     const int sub = threadIdx.x % LPR;
     const long long total = M * H;
     const long long stride = (long long)gridDim.x * ROWS_PER_BLOCK;
@@ -582,6 +584,7 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
 __global__ void attn_bwd_finish_kernel(const float* __restrict__ dq_acc, __nv_bfloat16* __restrict__ dqkv,
                                        const float* __restrict__ table, long long M, int T, int H, int KV, int HD,
                                        long long stride, int apply_rope) {
+    pdl_sync();
     const int vph = HD / 8;
     const long long total = M * (H + KV) * vph;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -626,6 +629,7 @@ __global__ void attn_bwd_finish_kernel(const float* __restrict__ dq_acc, __nv_bf
 // row's sequence starts at or before the tile's last kv row (seq_start is non-decreasing). One warp per kv tile, 32
 // candidate tiles per step (one load latency per 32 tiles instead of one per tile). Also zeroes the work counter.
 __global__ void attn_bwd_span_kernel(const int* __restrict__ seq_start, int n_tiles, int* __restrict__ nq, int* counter) {
+    pdl_sync();
     if (blockIdx.x == 0 && threadIdx.x == 0) *counter = 0;
     const int kv_tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (kv_tile >= n_tiles) return;
@@ -659,8 +663,8 @@ static int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const 
         configured = true;
     }
     const int grid = p.n_items < sm_count() ? p.n_items : sm_count();     // one CTA per SM draws items until none are left
-    attn_bwd_span_kernel<<<(p.n_tiles * 32 + 255) / 256, 256, 0, st>>>(p.seq_start, p.n_tiles, p.nq, p.counter);
-    kern<<<grid, 512, Cfg::SMEM_BYTES, st>>>(tq, tdo, tdq, p);
+    launch_pdl(attn_bwd_span_kernel, LaunchCfg((p.n_tiles * 32 + 255) / 256, 256, 0, st), p.seq_start, p.n_tiles, p.nq, p.counter);
+    launch_pdl(kern, LaunchCfg(grid, 512, Cfg::SMEM_BYTES, st), tq, tdo, tdq, p);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }
 
@@ -693,10 +697,10 @@ extern "C" int pb_attn_bwd(const void* qkv, const void* o, const void* dout, con
         long long blocks = (rows + 4LL * rows_per_block - 1) / (4LL * rows_per_block);
         if (blocks < 1) blocks = 1;
         if (HD == 64)
-            attn_bwd_prep_kernel<64><<<unsigned(blocks), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, D, M, H,
+            launch_pdl(attn_bwd_prep_kernel<64>, LaunchCfg(unsigned(blocks), 256, 0, st), (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, D, M, H,
                                                                          o_stride, do_stride);
         else
-            attn_bwd_prep_kernel<128><<<unsigned(blocks), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, D, M, H,
+            launch_pdl(attn_bwd_prep_kernel<128>, LaunchCfg(unsigned(blocks), 256, 0, st), (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, D, M, H,
                                                                           o_stride, do_stride);
     }
     AttnBwdParams p;
@@ -710,7 +714,7 @@ extern "C" int pb_attn_bwd(const void* qkv, const void* o, const void* dout, con
     const long long total = (long long)M * (H + KV) * (HD / 8);
     long long blocks = (total + 255) / 256;
     if (blocks > 148 * 8) blocks = 148 * 8;
-    attn_bwd_finish_kernel<<<unsigned(blocks), 256, 0, st>>>(dq_acc, (__nv_bfloat16*)dqkv, rope_table, M, T, H, KV, HD, dqkv_stride,
+    launch_pdl(attn_bwd_finish_kernel, LaunchCfg(unsigned(blocks), 256, 0, st), dq_acc, (__nv_bfloat16*)dqkv, rope_table, M, T, H, KV, HD, dqkv_stride,
                                                               rope_table != nullptr);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }

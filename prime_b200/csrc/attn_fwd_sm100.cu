@@ -103,6 +103,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tS = tmem_base, tO = tmem_base + 128, tP = tmem_base + Cfg::T_P;
+    pdl_sync();
 
     // kv tile range: from the tile holding the first row's sequence start up to the diagonal
     const int first_start = p.seq_start[min(q0, p.M - 1)];
@@ -364,7 +365,7 @@ static int launch_attn_fwd(const CUtensorMap& tm, const AttnFwdParams& p, cudaSt
         configured = true;
     }
     dim3 grid((p.M + 127) / 128, p.H);
-    kern<<<grid, 256, Cfg::SMEM_BYTES, st>>>(tm, p);
+    launch_pdl(kern, LaunchCfg(grid, 256, Cfg::SMEM_BYTES, st), tm, p);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }
 

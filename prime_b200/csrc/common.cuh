@@ -147,6 +147,38 @@ struct ItemRing {
     }
 };
 
+// ----------------------------------------------------------------------------
+// Programmatic dependent launch. A training step is a chain of launches on one stream; without it every kernel pays its launch
+// latency and its set-up (barrier init, tensor-memory allocation, cluster rendezvous, descriptor fetch: 3-5 us for the
+// GEMM and attention kernels) after the previous kernel has drained. A kernel launched with launch_pdl() may become resident
+// while its predecessor still runs, does whatever touches no global memory, and then calls pdl_sync(): that returns when the
+// predecessor has completed and its writes are visible, and only then lets the successor start, so at most one kernel waits at
+// a time and everything before the predecessor is complete as well. Rules: no global memory access before pdl_sync(),
+// every thread calls it, and kernels that talk to other GPUs are launched the ordinary way.
+// (pdl_sync() does nothing in an ordinary launch.) Measured: forward pass of the 150M model over 3 x 777 tokens, 87 launches,
+// 2.10 -> 1.91 ms; 70M step of 32 x 1024 tokens, 388 launches, 13.5 -> 13.1 ms; nothing on steps of 100 ms and more.
+// ----------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_sync() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+struct LaunchCfg {
+    cudaLaunchConfig_t c{};
+    LaunchCfg(dim3 grid, dim3 block, size_t smem, cudaStream_t st) {
+        c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = st;
+    }
+};
+template <typename... P, typename... A>
+static inline cudaError_t launch_pdl(void (*kern)(P...), LaunchCfg cfg, A&&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.c.attrs = at;
+    cfg.c.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg.c, kern, static_cast<P>(args)...);
+}
+
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }

@@ -22,6 +22,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
                                                           const __nv_bfloat16* __restrict__ w,
                                                           __nv_bfloat16* __restrict__ y, float* __restrict__ rstd,
                                                           int M, int N, float eps) {
+    pdl_sync();
     const int warps_per_block = blockDim.x >> 5;
     const int lane = threadIdx.x & 31;
     for (long long row = (long long)blockIdx.x * warps_per_block + (threadIdx.x >> 5); row < M;
@@ -56,6 +57,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fwd_kernel(const __nv_bfloat16* _
 // ----------------------------------------------------------------------------
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __restrict__ table, long long M, int T,
                             int n_rot_heads, int hd, int row_stride, float sign) {
+    pdl_sync();
     // one thread handles 8 consecutive elements (4 pairs)
     const int vec_per_head = hd / 8;
     const long long total = M * n_rot_heads * vec_per_head;
@@ -88,6 +90,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ qkv, const float* __rest
 // ----------------------------------------------------------------------------
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ h13, __nv_bfloat16* __restrict__ act,
                                   long long M, int F) {
+    pdl_sync();
     const int vpr = F / 8;
     const long long total = M * vpr;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -106,6 +109,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ h13, __nv_bf
 // (dh13 may alias h13: each thread reads its inputs before writing the same locations).
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* h13, const __nv_bfloat16* __restrict__ dact,
                                   __nv_bfloat16* dh13, long long M, int F) {
+    pdl_sync();
     const int vpr = F / 8;
     const long long total = M * vpr;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -132,6 +136,7 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* h13, const __nv_bfloat16*
 // ----------------------------------------------------------------------------
 __global__ void embedding_fwd_kernel(const long long* __restrict__ tok, const __nv_bfloat16* __restrict__ E,
                                      __nv_bfloat16* __restrict__ out, long long M, int D) {
+    pdl_sync();
     const int vpr = D / 8;
     const long long total = M * vpr;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -143,6 +148,7 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ tok, const __
 }
 __global__ void embedding_bwd_kernel(const long long* __restrict__ tok, const __nv_bfloat16* __restrict__ dout,
                                      void* __restrict__ dE, long long M, int D, int grad_fp32) {
+    pdl_sync();
     const int vpr = D / 8;
     const long long total = M * vpr;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -179,6 +185,7 @@ __global__ void __launch_bounds__(512) cross_entropy_kernel(__nv_bfloat16* logit
                                                             const float* __restrict__ inv_count, float grad_scale,
                                                             int V, long long ld, int ignore_index, int z_mode,
                                                             float z_weight, int write_grad) {
+    pdl_sync();
     __shared__ float s_m[16], s_s[16];
     __shared__ int s_arg[16];
     const long long row = blockIdx.x;
@@ -271,6 +278,7 @@ __global__ void __launch_bounds__(512) cross_entropy_kernel(__nv_bfloat16* logit
 // count of labels != ignore_index -> inv_count = 1/max(count,1) ; single CTA, fixed order
 __global__ void count_valid_kernel(const long long* __restrict__ labels, long long n, int ignore_index,
                                    float* __restrict__ inv_count) {
+    pdl_sync();
     __shared__ long long s[32];
     long long c = 0;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) c += (labels[i] != ignore_index);
@@ -288,6 +296,7 @@ __global__ void count_valid_kernel(const long long* __restrict__ labels, long lo
 
 // out[0] (+)= scale * sum(x[0:n]) — two-stage fixed-order sum of fp32 values
 __global__ void sum_stage1_kernel(const float* __restrict__ x, long long n, float* __restrict__ partial) {
+    pdl_sync();
     __shared__ float s[32];
     float a = 0.f;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -303,6 +312,7 @@ __global__ void sum_stage1_kernel(const float* __restrict__ x, long long n, floa
 }
 __global__ void sum_stage2_kernel(const float* __restrict__ partial, int nb, const float* __restrict__ scale_ptr,
                                   float scale, float* __restrict__ out, int accumulate) {
+    pdl_sync();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         float t = 0.f;
         for (int i = 0; i < nb; ++i) t += partial[i];
@@ -316,6 +326,7 @@ __global__ void sum_stage2_kernel(const float* __restrict__ partial, int nb, con
 // ----------------------------------------------------------------------------
 template <typename T>
 __global__ void sumsq_kernel(const T* __restrict__ x, long long n, float* __restrict__ partial) {
+    pdl_sync();
     __shared__ float s[32];
     float a = 0.f;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -342,6 +353,7 @@ __global__ void adamw_kernel(float* __restrict__ p, const G* __restrict__ g, flo
                              __nv_bfloat16* __restrict__ p_bf16, long long n, float lr, float beta1, float beta2,
                              float eps, float wd, float bc1, float bc2, const float* __restrict__ gnorm,
                              float max_norm, float gscale) {
+    pdl_sync();
     float clip = gscale;
     if (gnorm) {
         const float c = max_norm / (*gnorm + 1e-6f);
@@ -363,6 +375,7 @@ __global__ void adamw_kernel(float* __restrict__ p, const G* __restrict__ g, flo
 }
 
 __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long n) {
+    pdl_sync();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         dst[i] = __float2bfloat16(src[i]);
 }
@@ -370,6 +383,7 @@ __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ src, __nv_bflo
 // residual add: out = a + b (bf16)
 __global__ void add_bf16_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                                 __nv_bfloat16* __restrict__ out, long long n8) {
+    pdl_sync();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
         float x[8], y[8];
         load8(a + i * 8, x);
@@ -394,7 +408,7 @@ using namespace pb;
 
 extern "C" int pb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int M, int N, float eps, void* stream) {
     if (N % 8) return -1;
-    rmsnorm_fwd_kernel<<<grid_for(M, 8), 256, 0, ST(stream)>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+    launch_pdl(rmsnorm_fwd_kernel, LaunchCfg(grid_for(M, 8), 256, 0, ST(stream)), (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
                                                                 (__nv_bfloat16*)y, rstd, M, N, eps);
     return CHECK_LAUNCH();
 }
@@ -410,50 +424,50 @@ extern "C" int pb_rmsnorm_bwd(const void* x, const void* w, const float* rstd, c
     auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w; auto DY = (const __nv_bfloat16*)dy;
     auto DR = (const __nv_bfloat16*)dres; auto DX = (__nv_bfloat16*)dx;
     // rows wider than 1024 are shared by two or four warps (at most four 256-column chunks per warp)
-#define RB(NCH, WPR) case NCH: rmsnorm_bwd_kernel<NCH, WPR><<<ctas, 256, 0, ST(stream)>>>(X, W, rstd, DY, DR, DX, dw_partial, M); break;
+#define RB(NCH, WPR) case NCH: launch_pdl(rmsnorm_bwd_kernel<NCH, WPR>, LaunchCfg(ctas, 256, 0, ST(stream)), X, W, rstd, DY, DR, DX, dw_partial, M); break;
     switch (N / 256) {
         RB(1, 1) RB(2, 1) RB(3, 1) RB(4, 1) RB(6, 2) RB(8, 2) RB(12, 4) RB(16, 4)
         default: return -1;
     }
 #undef RB
     if (cudaGetLastError() != cudaSuccess) return -30;
-    colsum_partials_kernel<<<(N + 31) / 32, 256, 0, ST(stream)>>>(dw_partial, dw, ctas, N, dw_fp32, dw_accumulate);
+    launch_pdl(colsum_partials_kernel, LaunchCfg((N + 31) / 32, 256, 0, ST(stream)), dw_partial, dw, ctas, N, dw_fp32, dw_accumulate);
     return CHECK_LAUNCH();
 }
 
 extern "C" int pb_rope(void* qkv, const float* table, long long M, int T, int n_rot_heads, int hd, int row_stride,
                        int backward, void* stream) {
     if (hd % 8 || row_stride % 8) return -1;
-    rope_kernel<<<grid_for(M * n_rot_heads * (hd / 8), 256), 256, 0, ST(stream)>>>(
+    launch_pdl(rope_kernel, LaunchCfg(grid_for(M * n_rot_heads * (hd / 8), 256), 256, 0, ST(stream)), 
         (__nv_bfloat16*)qkv, table, M, T, n_rot_heads, hd, row_stride, backward ? -1.f : 1.f);
     return CHECK_LAUNCH();
 }
 
 extern "C" int pb_swiglu_fwd(const void* h13, void* act, long long M, int F, void* stream) {
     if (F % 8) return -1;
-    swiglu_fwd_kernel<<<grid_for(M * (F / 8), 256), 256, 0, ST(stream)>>>((const __nv_bfloat16*)h13, (__nv_bfloat16*)act, M, F);
+    launch_pdl(swiglu_fwd_kernel, LaunchCfg(grid_for(M * (F / 8), 256), 256, 0, ST(stream)), (const __nv_bfloat16*)h13, (__nv_bfloat16*)act, M, F);
     return CHECK_LAUNCH();
 }
 extern "C" int pb_swiglu_bwd(const void* h13, const void* dact, void* dh13, long long M, int F, void* stream) {
     if (F % 8) return -1;
-    swiglu_bwd_kernel<<<grid_for(M * (F / 8), 256), 256, 0, ST(stream)>>>((const __nv_bfloat16*)h13, (const __nv_bfloat16*)dact,
+    launch_pdl(swiglu_bwd_kernel, LaunchCfg(grid_for(M * (F / 8), 256), 256, 0, ST(stream)), (const __nv_bfloat16*)h13, (const __nv_bfloat16*)dact,
                                                                           (__nv_bfloat16*)dh13, M, F);
     return CHECK_LAUNCH();
 }
 
 extern "C" int pb_embedding_fwd(const long long* tok, const void* E, void* out, long long M, int D, void* stream) {
     if (D % 8) return -1;
-    embedding_fwd_kernel<<<grid_for(M * (D / 8), 256), 256, 0, ST(stream)>>>(tok, (const __nv_bfloat16*)E, (__nv_bfloat16*)out, M, D);
+    launch_pdl(embedding_fwd_kernel, LaunchCfg(grid_for(M * (D / 8), 256), 256, 0, ST(stream)), tok, (const __nv_bfloat16*)E, (__nv_bfloat16*)out, M, D);
     return CHECK_LAUNCH();
 }
 extern "C" int pb_embedding_bwd(const long long* tok, const void* dout, void* dE, long long M, int D, int grad_fp32, void* stream) {
     if (D % 8) return -1;
-    embedding_bwd_kernel<<<grid_for(M * (D / 8), 256), 256, 0, ST(stream)>>>(tok, (const __nv_bfloat16*)dout, dE, M, D, grad_fp32);
+    launch_pdl(embedding_bwd_kernel, LaunchCfg(grid_for(M * (D / 8), 256), 256, 0, ST(stream)), tok, (const __nv_bfloat16*)dout, dE, M, D, grad_fp32);
     return CHECK_LAUNCH();
 }
 
 extern "C" int pb_count_valid(const long long* labels, long long n, int ignore_index, float* inv_count, void* stream) {
-    count_valid_kernel<<<1, 1024, 0, ST(stream)>>>(labels, n, ignore_index, inv_count);
+    launch_pdl(count_valid_kernel, LaunchCfg(1, 1024, 0, ST(stream)), labels, n, ignore_index, inv_count);
     return CHECK_LAUNCH();
 }
 
@@ -464,7 +478,7 @@ extern "C" int pb_cross_entropy(void* logits, const long long* labels, float* lo
     if (ld % 8) return -1;
     // 256 threads per row: more resident CTAs per SM overlap one row's exponentials with another's loads (260 us
     // against 296 us with 512 threads for 8192 x 32000)
-    cross_entropy_kernel<<<(unsigned)rows, 256, 0, ST(stream)>>>((__nv_bfloat16*)logits, labels, loss_rows, z_rows, inv_count,
+    launch_pdl(cross_entropy_kernel, LaunchCfg((unsigned)rows, 256, 0, ST(stream)), (__nv_bfloat16*)logits, labels, loss_rows, z_rows, inv_count,
                                                                  grad_scale, V, ld, ignore_index, z_mode, z_weight, write_grad);
     return CHECK_LAUNCH();
 }
@@ -473,17 +487,17 @@ extern "C" int pb_cross_entropy(void* logits, const long long* labels, float* lo
 extern "C" int pb_sum_f32(const float* x, long long n, float* scratch, const float* scale_ptr, float scale, float* out,
                           int accumulate, void* stream) {
     const int nb = grid_for(n, 256, 1024);
-    sum_stage1_kernel<<<nb, 256, 0, ST(stream)>>>(x, n, scratch);
-    sum_stage2_kernel<<<1, 32, 0, ST(stream)>>>(scratch, nb, scale_ptr, scale, out, accumulate);
+    launch_pdl(sum_stage1_kernel, LaunchCfg(nb, 256, 0, ST(stream)), x, n, scratch);
+    launch_pdl(sum_stage2_kernel, LaunchCfg(1, 32, 0, ST(stream)), scratch, nb, scale_ptr, scale, out, accumulate);
     return CHECK_LAUNCH();
 }
 
 // out (+)= sum(x^2) ; scratch >= 1024 floats
 extern "C" int pb_sumsq(const void* x, long long n, int is_fp32, float* scratch, float* out, int accumulate, void* stream) {
     const int nb = grid_for(n, 256, 1024);
-    if (is_fp32) sumsq_kernel<float><<<nb, 256, 0, ST(stream)>>>((const float*)x, n, scratch);
-    else sumsq_kernel<__nv_bfloat16><<<nb, 256, 0, ST(stream)>>>((const __nv_bfloat16*)x, n, scratch);
-    sum_stage2_kernel<<<1, 32, 0, ST(stream)>>>(scratch, nb, nullptr, 1.f, out, accumulate);
+    if (is_fp32) launch_pdl(sumsq_kernel<float>, LaunchCfg(nb, 256, 0, ST(stream)), (const float*)x, n, scratch);
+    else launch_pdl(sumsq_kernel<__nv_bfloat16>, LaunchCfg(nb, 256, 0, ST(stream)), (const __nv_bfloat16*)x, n, scratch);
+    launch_pdl(sum_stage2_kernel, LaunchCfg(1, 32, 0, ST(stream)), scratch, nb, nullptr, 1.f, out, accumulate);
     return CHECK_LAUNCH();
 }
 
@@ -495,23 +509,23 @@ extern "C" int pb_adamw(float* p, const void* g, int g_fp32, float* m, float* v,
     const float bc2 = sqrtf(1.f - powf(beta2, float(step)));
     const int nb = grid_for(n, 256, 148 * 16);
     if (g_fp32)
-        adamw_kernel<float><<<nb, 256, 0, ST(stream)>>>(p, (const float*)g, m, v, (__nv_bfloat16*)p_bf16, n, lr, beta1, beta2, eps,
+        launch_pdl(adamw_kernel<float>, LaunchCfg(nb, 256, 0, ST(stream)), p, (const float*)g, m, v, (__nv_bfloat16*)p_bf16, n, lr, beta1, beta2, eps,
                                                          wd, bc1, bc2, gnorm, max_norm, gscale);
     else
-        adamw_kernel<__nv_bfloat16><<<nb, 256, 0, ST(stream)>>>(p, (const __nv_bfloat16*)g, m, v, (__nv_bfloat16*)p_bf16, n, lr,
+        launch_pdl(adamw_kernel<__nv_bfloat16>, LaunchCfg(nb, 256, 0, ST(stream)), p, (const __nv_bfloat16*)g, m, v, (__nv_bfloat16*)p_bf16, n, lr,
                                                                  beta1, beta2, eps, wd, bc1, bc2, gnorm, max_norm, gscale);
     return CHECK_LAUNCH();
 }
 
 extern "C" int pb_cast_f32_bf16(const float* src, void* dst, long long n, void* stream) {
     if (n <= 0) return 0;
-    cast_f32_to_bf16_kernel<<<grid_for(n, 256, 148 * 16), 256, 0, ST(stream)>>>(src, (__nv_bfloat16*)dst, n);
+    launch_pdl(cast_f32_to_bf16_kernel, LaunchCfg(grid_for(n, 256, 148 * 16), 256, 0, ST(stream)), src, (__nv_bfloat16*)dst, n);
     return CHECK_LAUNCH();
 }
 
 extern "C" int pb_add_bf16(const void* a, const void* b, void* out, long long n, void* stream) {
     if (n % 8) return -1;
-    add_bf16_kernel<<<grid_for(n / 8, 256), 256, 0, ST(stream)>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)out, n / 8);
+    launch_pdl(add_bf16_kernel, LaunchCfg(grid_for(n / 8, 256), 256, 0, ST(stream)), (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)out, n / 8);
     return CHECK_LAUNCH();
 }
 
@@ -519,6 +533,7 @@ extern "C" int pb_add_bf16(const void* a, const void* b, void* out, long long n,
 template <bool OUT_FP32>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ ws, int slices, long long M, int N, const void* res,
                                                             long long ld_res, void* out, long long ld_out) {
+    pdl_sync();
     const int vpr = N / 4;
     const long long total = M * vpr;
     const long long slice_stride = M * (long long)N;
@@ -554,7 +569,7 @@ extern "C" int pb_splitk_reduce(const float* ws, int slices, long long M, int N,
                                 long long ld_out, int out_fp32, void* stream) {
     if (N % 4 || ld_out % 4 || (res && ld_res % 4)) return -1;
     const unsigned grid = grid_for(M * (N / 4), 256);
-    if (out_fp32) splitk_reduce_kernel<true><<<grid, 256, 0, ST(stream)>>>(ws, slices, M, N, res, ld_res, out, ld_out);
-    else splitk_reduce_kernel<false><<<grid, 256, 0, ST(stream)>>>(ws, slices, M, N, res, ld_res, out, ld_out);
+    if (out_fp32) launch_pdl(splitk_reduce_kernel<true>, LaunchCfg(grid, 256, 0, ST(stream)), ws, slices, M, N, res, ld_res, out, ld_out);
+    else launch_pdl(splitk_reduce_kernel<false>, LaunchCfg(grid, 256, 0, ST(stream)), ws, slices, M, N, res, ld_res, out, ld_out);
     return CHECK_LAUNCH();
 }

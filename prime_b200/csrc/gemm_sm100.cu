@@ -74,6 +74,7 @@ gemm_bf16_tcgen05(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_sync();
 
     const int num_kb = (p.K + BK - 1) / BK;
 
@@ -269,7 +270,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParam
     p.num_tiles = tiles_m * p.tiles_n;
     int grid = p.num_tiles < sm_count() ? p.num_tiles : sm_count();
     if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-    kern<<<grid, 192, Cfg::SMEM_BYTES, st>>>(tmA, tmB, p);
+    launch_pdl(kern, LaunchCfg(grid, 192, Cfg::SMEM_BYTES, st), tmA, tmB, p);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }
 

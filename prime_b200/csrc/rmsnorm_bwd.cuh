@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(256, 2) rmsnorm_bwd_kernel(const __nv_bfloat16
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = warp % WPR, rslot = warp / WPR;
     const int col0 = sub * CPW * 256 + lane * 8;
+    pdl_sync();
     for (int c = threadIdx.x; c < N; c += blockDim.x) s_w[c] = __bfloat162float(w[c]);
     float dwacc[CPW][8];
 #pragma unroll
@@ -150,6 +151,7 @@ static __global__ void __launch_bounds__(256) colsum_partials_kernel(const float
     const int cx = threadIdx.x & 31, g = threadIdx.x >> 5;
     const int c = blockIdx.x * 32 + cx;
     float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+    pdl_sync();
     if (c < N) {
         int b = g;
         for (; b + 24 < nb; b += 32) {

@@ -223,6 +223,7 @@ __global__ void __launch_bounds__(256) grad_sumsq_kernel(const G* __restrict__ g
     __shared__ bool last;
     constexpr int E = GradVec<G>::N, UNR = 8;
     float ss = 0.f;
+    pdl_sync();
     int s;
     long long b, nb;
     my_segment(segs, s, b, nb);
@@ -296,6 +297,7 @@ __global__ void __launch_bounds__(256) zero_adamw_gather_kernel(PeerTable params
                                                                 float wd, float bc1, float bc2, const float* __restrict__ gnorm_sq,
                                                                 float max_norm) {
     float clip = 1.f;
+    pdl_sync();
     if (gnorm_sq && max_norm > 0.f) {
         const float c = max_norm / (sqrtf(*gnorm_sq) + 1e-6f);
         clip = c < 1.f ? c : 1.f;
@@ -519,7 +521,9 @@ extern "C" int pb_zero_adamw_gather(void* const* peer_params, int world, int ran
     if (sg.cta_begin[nseg] <= 0) return 0;
     const PeerTable pt = make_peers(peer_params, world, rank);
     auto launch = [&](auto kern, auto* g) {
-        kern<<<sg.cta_begin[nseg], 256, 0, ST(stream)>>>(pt, sg, master, g, m, v, lr, beta1, beta2, eps, wd, bc1, bc2, gnorm_sq, max_norm);
+        const LaunchCfg cfg(sg.cta_begin[nseg], 256, 0, ST(stream));
+        if (world == 1) launch_pdl(kern, cfg, pt, sg, master, g, m, v, lr, beta1, beta2, eps, wd, bc1, bc2, gnorm_sq, max_norm);
+        else kern<<<cfg.c.gridDim, 256, 0, ST(stream)>>>(pt, sg, master, g, m, v, lr, beta1, beta2, eps, wd, bc1, bc2, gnorm_sq, max_norm);
     };
     if (grad_kind == 0) launch(zero_adamw_gather_kernel<float, false>, reinterpret_cast<const float*>(grad));
     else if (grad_kind == 1) launch(zero_adamw_gather_kernel<__nv_bfloat16, true>, reinterpret_cast<const __nv_bfloat16*>(grad));
@@ -536,8 +540,8 @@ extern "C" int pb_grad_sumsq(const void* grads, int grad_fp32, int nseg, const l
     const SegTable sg = make_segs(nseg, full_off, full_off, numel, ctas);
     ctas = sg.cta_begin[nseg];
     if (ctas <= 0) return -1;
-    if (grad_fp32) grad_sumsq_kernel<float><<<ctas, 256, 0, ST(stream)>>>(reinterpret_cast<const float*>(grads), sg, scratch, counter, out);
-    else grad_sumsq_kernel<__nv_bfloat16><<<ctas, 256, 0, ST(stream)>>>(reinterpret_cast<const __nv_bfloat16*>(grads), sg, scratch, counter, out);
+    if (grad_fp32) launch_pdl(grad_sumsq_kernel<float>, LaunchCfg(ctas, 256, 0, ST(stream)), reinterpret_cast<const float*>(grads), sg, scratch, counter, out);
+    else launch_pdl(grad_sumsq_kernel<__nv_bfloat16>, LaunchCfg(ctas, 256, 0, ST(stream)), reinterpret_cast<const __nv_bfloat16*>(grads), sg, scratch, counter, out);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }
 
