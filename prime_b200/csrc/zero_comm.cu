@@ -289,15 +289,17 @@ __global__ void reduce_partials_kernel(const float* __restrict__ partial, int n,
 // Sharded AdamW + push all-gather. gnorm_sq: device scalar with the GLOBAL sum of squared grads. HBM-bound. FULL: the
 // gradients are read from the rank's own full gradient buffer (bf16 or fp32, at the segment's full offset) instead of the
 // reduced fp32 shard: without peers there is nothing to reduce, which saves the fp32 copy's write and read (28 instead of
-// 36 bytes per bf16-gradient parameter over the whole update).
+// 36 bytes per bf16-gradient parameter over the whole update). hyper (optional): {lr, bc1, bc2} in device memory instead of the
+// arguments, for launches that are replayed from a graph.
 template <typename G, bool FULL>
 __global__ void __launch_bounds__(256) zero_adamw_gather_kernel(PeerTable params, SegTable segs, float* __restrict__ master,
                                                                 const G* __restrict__ grad, float* __restrict__ m,
                                                                 float* __restrict__ v, float lr, float beta1, float beta2, float eps,
                                                                 float wd, float bc1, float bc2, const float* __restrict__ gnorm_sq,
-                                                                float max_norm) {
+                                                                float max_norm, const float* __restrict__ hyper) {
     float clip = 1.f;
     pdl_sync();
+    if (hyper) { lr = hyper[0]; bc1 = hyper[1]; bc2 = hyper[2]; }
     if (gnorm_sq && max_norm > 0.f) {
         const float c = max_norm / (sqrtf(*gnorm_sq) + 1e-6f);
         clip = c < 1.f ? c : 1.f;
@@ -508,11 +510,11 @@ extern "C" int pb_zero_reduce_grads(void* const* peer_grads, int world, int rank
 }
 
 // grad: fp32 shard (grad_kind 0, indexed by shard_off), or the rank's full gradient buffer in bf16 (1) or fp32 (2), indexed by
-// full_off.
+// full_off. hyper: null, or device {lr, 1 - beta1^t, sqrt(1 - beta2^t)} that replaces lr and step.
 extern "C" int pb_zero_adamw_gather(void* const* peer_params, int world, int rank, int nseg, const long long* full_off,
                                     const long long* shard_off, const long long* numel, float* master, const void* grad, int grad_kind,
                                     float* m, float* v, float lr, float beta1, float beta2, float eps, float wd, int step,
-                                    const float* gnorm_sq, float max_norm, int ctas, void* stream) {
+                                    const float* gnorm_sq, float max_norm, const float* hyper, int ctas, void* stream) {
     if (world > MAX_RANKS || nseg > MAX_SEGS || grad_kind < 0 || grad_kind > 2) return -1;
     const float bc1 = 1.f - powf(beta1, float(step));
     const float bc2 = sqrtf(1.f - powf(beta2, float(step)));
@@ -522,8 +524,8 @@ extern "C" int pb_zero_adamw_gather(void* const* peer_params, int world, int ran
     const PeerTable pt = make_peers(peer_params, world, rank);
     auto launch = [&](auto kern, auto* g) {
         const LaunchCfg cfg(sg.cta_begin[nseg], 256, 0, ST(stream));
-        if (world == 1) launch_pdl(kern, cfg, pt, sg, master, g, m, v, lr, beta1, beta2, eps, wd, bc1, bc2, gnorm_sq, max_norm);
-        else kern<<<cfg.c.gridDim, 256, 0, ST(stream)>>>(pt, sg, master, g, m, v, lr, beta1, beta2, eps, wd, bc1, bc2, gnorm_sq, max_norm);
+        if (world == 1) launch_pdl(kern, cfg, pt, sg, master, g, m, v, lr, beta1, beta2, eps, wd, bc1, bc2, gnorm_sq, max_norm, hyper);
+        else kern<<<cfg.c.gridDim, 256, 0, ST(stream)>>>(pt, sg, master, g, m, v, lr, beta1, beta2, eps, wd, bc1, bc2, gnorm_sq, max_norm, hyper);
     };
     if (grad_kind == 0) launch(zero_adamw_gather_kernel<float, false>, reinterpret_cast<const float*>(grad));
     else if (grad_kind == 1) launch(zero_adamw_gather_kernel<__nv_bfloat16, true>, reinterpret_cast<const __nv_bfloat16*>(grad));

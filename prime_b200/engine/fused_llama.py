@@ -54,7 +54,7 @@ native.register_cuda_sigs({
     "pb_grad_sumsq": [native.vp, native.i32, native.i32, native.vp, native.vp, native.vp, native.vp, native.vp, native.i32, native.vp],
     "pb_zero_adamw_gather": [native.vp, native.i32, native.i32, native.i32, native.vp, native.vp, native.vp, native.vp,
                              native.vp, native.i32, native.vp, native.vp, native.f32, native.f32, native.f32, native.f32, native.f32,
-                             native.i32, native.vp, native.f32, native.i32, native.vp],
+                             native.i32, native.vp, native.f32, native.vp, native.i32, native.vp],
     "pb_zero_push_params": [native.vp, native.i32, native.i32, native.i32, native.vp, native.vp, native.vp, native.vp,
                             native.i32, native.vp],
     "pb_zero_gather_segments": [native.vp, native.i32, native.i32, native.i32, native.vp, native.vp, native.vp, native.vp, native.vp,
@@ -108,8 +108,37 @@ class LocalComm:
         dst[:n].copy_(src[:n])
 
 
+class _StepGraph:
+    """One recorded ``train_step``: its input buffers, the graph, and references to every buffer the graph touches."""
+
+    def __init__(self, eng: "FusedLlama", B: int, T: int, micro_bs: int, packed: bool, betas, eps, weight_decay, max_norm, report):
+        dev = eng.device
+        self.tokens = torch.empty(B, T, dtype=torch.int64, device=dev)
+        self.labels = torch.empty(B, T, dtype=torch.int64, device=dev)
+        self.seq_start = torch.empty(B * T, dtype=torch.int32, device=dev) if packed else None
+        self.hyper = torch.empty(4, dtype=torch.float32, device=dev)
+        self.graph = torch.cuda.CUDAGraph()
+        main, side = torch.cuda.current_stream(dev), torch.cuda.Stream(device=dev)
+        side.wait_stream(main)
+        before = native.launch_counter()
+        with torch.cuda.stream(side):
+            self.graph.capture_begin(capture_error_mode="thread_local")
+            try:
+                eng._accumulate_micro_batches(self.tokens, self.labels, self.seq_start, micro_bs)
+                eng._update_from_own_grads(0.0, betas, eps, weight_decay, max_norm, hyper=self.hyper)
+                eng._report(report)
+            finally:
+                self.graph.capture_end()
+                eng._accum = False
+        main.wait_stream(side)
+        self.launches = native.launch_counter() - before
+        native.add_launches(-self.launches)              # recorded, not run
+        self.refs = [report, *eng._ws.values(), *eng._seq_start_cache.values(), *K.scratch_buffers()]
+
+
 class FusedLlama:
     """See module docstring. One instance per process / GPU."""
+    _MAX_GRAPHS = 8
 
     def __init__(self, args: ModelArgs, device: torch.device | str = "cuda", comm=None, grad_dtype=torch.bfloat16,
                  ac_ckpt: bool | int = False, ce_chunk_tokens: int = 32768, z_mode: int = K.Z_NONE, z_weight: float = 0.0,
@@ -152,7 +181,8 @@ class FusedLlama:
         allsegs = _SegArrays([s for g in range(len(lay.groups)) for s in lay.group_segments(self.rank, g)])
         self._segs_step = [allsegs] if allsegs.n <= max_segs else self._segs
         self._partials = torch.zeros(4096, dtype=torch.float32, device=dev)
-        self._sumsq_counter = torch.zeros(1, dtype=torch.int32, device=dev)
+        # arrival counters of the kernels whose last CTA finishes a sum (zero between launches): norm, valid labels (2), losses
+        self._counters = torch.zeros(4, dtype=torch.int32, device=dev)
         self._norm_parts = torch.zeros(len(lay.groups), dtype=torch.float32, device=dev)   # sum of squares per group
         self._reduced_groups: set[int] = set()      # groups whose reduce-scatter is already in flight on the comm stream
         self.overlap_reduce = True                  # False: every group is reduced after the backward, on the main stream
@@ -163,6 +193,8 @@ class FusedLlama:
         self.opt_step = 0
         self._accum = False            # gradients hold a partial sum from earlier micro-batches
         self._ws: dict[str, torch.Tensor] = {}
+        self._graphs: dict[tuple, _StepGraph] = {}      # recorded steps by shape and settings (see _graphed_step)
+        self._graph_seen: set[tuple] = set()
         self._rope = K.rope_table(args.max_seq_len * 2, args.head_dim, args.rope_theta, dev)
         self._seq_start_cache: dict[tuple[int, int], torch.Tensor] = {}
         self.comm_stream = torch.cuda.Stream(device=dev) if dev.type == "cuda" else None
@@ -420,6 +452,8 @@ class FusedLlama:
         t = self._ws.get(name)
         n = math.prod(shape)
         if t is None or t.numel() < n or t.dtype != dtype:
+            if t is not None:
+                self._drop_graphs()
             t = torch.empty(n, dtype=dtype, device=self.device)
             self._ws[name] = t
         return t[:n].view(shape)
@@ -470,8 +504,7 @@ class FusedLlama:
         else:
             K.gemm_rope(xn, self.wqkv[i], qkv, self._rope, T, H + KV, hd)     # rotary embedding in the GEMM epilogue
         o = self._saved(i, "o", (M, H * hd))
-        _, lse2 = A.attention_fwd(qkv, seq_start, H, KV, hd, out=o)
-        self._ws[f"L{i}.lse2" if not self._is_ckpt(i) else "Lshared.lse2"] = lse2
+        A.attention_fwd(qkv, seq_start, H, KV, hd, out=o, lse2=self._saved(i, "lse2", (H, M), torch.float32))
         h = self._saved(i, "h", (M, D))
         K.gemm(o, self.w[pre + "attention.wo.weight"], out=h, residual=x)
         hn = self._saved(i, "hn", (M, D))
@@ -526,7 +559,7 @@ class FusedLlama:
             self._block_fwd(i, x, T, seq_start, self._buf("ckpt_out", (M, D)), recompute=True)
         sv = lambda n, shp, dt=torch.bfloat16: self._saved(i, n, shp, dt)  # noqa: E731
         xn, rstd1, qkv, o = sv("xn", (M, D)), sv("rstd1", (M,), torch.float32), sv("qkv", (M, (H + 2 * KV) * hd)), sv("o", (M, H * hd))
-        lse2 = self._ws[f"L{i}.lse2" if not self._is_ckpt(i) else "Lshared.lse2"]
+        lse2 = sv("lse2", (H, M), torch.float32)
         h, hn, rstd2 = sv("h", (M, D)), sv("hn", (M, D)), sv("rstd2", (M,), torch.float32)
         h13, act = sv("h13", (M, 2 * F)), sv("act", (M, F))
         # out = h + act @ w2^T
@@ -566,9 +599,11 @@ class FusedLlama:
     # full micro-step
     # ------------------------------------------------------------------------------------------
     def forward_backward(self, tokens: torch.Tensor, labels: torch.Tensor, seq_start: torch.Tensor | None = None,
-                         loss_scale: float = 1.0, last_microbatch: bool = True) -> dict[str, torch.Tensor]:
+                         loss_scale: float = 1.0, last_microbatch: bool = True, loss_acc: torch.Tensor | None = None,
+                         first_microbatch: bool = True) -> dict[str, torch.Tensor]:
         """One micro-batch: forward, loss, backward; gradients accumulate until ``optimizer_step``.
-        Returns device scalars ``loss`` (mean CE over non-ignored tokens) and ``z_loss``."""
+        Returns device scalars ``loss`` (mean CE over non-ignored tokens) and ``z_loss``; with ``loss_acc`` ([2] fp32) also adds
+        ``loss_scale`` times them there (overwrites it at the first micro-batch)."""
         a = self.args
         B, T = tokens.shape
         M = B * T
@@ -593,8 +628,9 @@ class FusedLlama:
         K.rmsnorm_fwd(xs[L], self.w["norm.weight"], a.norm_eps, out=hn, rstd=rstd)
         dhn = self._buf("head.dhn", (M, D))
         loss_rows = self._buf("head.loss_rows", (M,), torch.float32)
-        z_rows = self._buf("head.z_rows", (M,), torch.float32)
-        inv = K.count_valid(lab)
+        z_rows = self._buf("head.z_rows", (M,), torch.float32) if self.z_mode != K.Z_NONE else None
+        on_gpu = self.device.type == "cuda"
+        inv = K.count_valid(lab, out=self._buf("head.inv", (2,), torch.float32), counter=self._counters[1:3] if on_gpu else None)
         Vp = (V + 7) // 8 * 8
         Mc = min(self.ce_chunk, M)
         logits_buf = self._buf("head.logits", (Mc, Vp))
@@ -604,14 +640,14 @@ class FusedLlama:
             c1 = min(M, c0 + Mc)
             lg = logits_buf[: c1 - c0, :V]
             K.gemm(hn[c0:c1], Wout, out=lg)
-            K.cross_entropy_(lg, lab[c0:c1], inv, loss_rows[c0:c1], z_rows[c0:c1], grad_scale=loss_scale,
+            K.cross_entropy_(lg, lab[c0:c1], inv, loss_rows[c0:c1], z_rows[c0:c1] if z_rows is not None else None, grad_scale=loss_scale,
                              z_mode=self.z_mode, z_weight=self.z_weight)
             K.gemm(lg, Wout, out=dhn[c0:c1], b_mn=True)
             K.gemm(lg, hn[c0:c1], out=gWout, residual=gWout if accum_head else None, a_mn=True, b_mn=True)
             accum_head = True
         out = self._buf("head.scalars", (2,), torch.float32)
-        K.sum_f32(loss_rows, out[0:1], scale_ptr=inv[0:1])
-        K.sum_f32(z_rows, out[1:2], scale_ptr=inv[0:1], scale=self.z_weight)
+        K.loss_sums(loss_rows, z_rows, inv, self.z_weight, out, self._partials if on_gpu else None,
+                    self._counters[3:] if on_gpu else None, acc=loss_acc, acc_scale=loss_scale, acc_first=first_microbatch)
         dx = self._buf("dx_a", (M, D))
         K.rmsnorm_bwd(xs[L], self.w["norm.weight"], rstd, dhn, self.g["norm.weight"], dx=dx, accumulate_dw=self._accum)
         if self._reduce_in_backward:
@@ -677,7 +713,7 @@ class FusedLlama:
             one = (C.c_longlong * 1)
             check(lib.pb_zero_adamw_gather((C.c_void_p * 1)(self.param_shard.data_ptr()), 1, 0, 1, one(0), one(0), one(n), ptr(self.master),
                                            ptr(self.grad_shard), 0, ptr(self.exp_avg), ptr(self.exp_avg_sq), lr, betas[0], betas[1],
-                                           eps, weight_decay, self.opt_step, ptr(self._norm_global), max_norm,
+                                           eps, weight_decay, self.opt_step, ptr(self._norm_global), max_norm, None,
                                            min(self.comm_ctas * 4, 1024), stream_ptr()), "pb_zero_adamw_gather")
             self._root_fresh = False
             self._gbuf_holds = [-1, -1]
@@ -686,7 +722,7 @@ class FusedLlama:
                 continue
             check(lib.pb_zero_adamw_gather(self._peer_params, W, self.rank, sa.n, sa.full, sa.shard, sa.numel, ptr(self.master),
                                            ptr(self.grad_shard), 0, ptr(self.exp_avg), ptr(self.exp_avg_sq), lr, betas[0], betas[1],
-                                           eps, weight_decay, self.opt_step, ptr(self._norm_global), max_norm,
+                                           eps, weight_decay, self.opt_step, ptr(self._norm_global), max_norm, None,
                                            self._opt_ctas(sa), stream_ptr()), "pb_zero_adamw_gather")
         self.comm.barrier()                                   # every rank's replica is complete
         self._accum = False
@@ -704,7 +740,8 @@ class FusedLlama:
     def _direct_update(self) -> bool:
         return self._solo and self._shard_opt is None
 
-    def _update_from_own_grads(self, lr: float, betas, eps: float, weight_decay: float, max_norm: float) -> None:
+    def _update_from_own_grads(self, lr: float, betas, eps: float, weight_decay: float, max_norm: float,
+                               hyper: torch.Tensor | None = None) -> None:
         """The update of a run without peers: the squared norm in one pass over the gradient buffer, then AdamW straight from
         that buffer. Against the reduce into an fp32 shard (14 to 20 launches under the backward) this moves 8 bytes per
         bf16-gradient parameter less and takes no bandwidth from the backward."""
@@ -713,14 +750,15 @@ class FusedLlama:
         norm_out = self._norm_global if len(self._segs_step) == 1 else self._norm_parts
         for i, sa in enumerate(self._segs_step):
             assert sa.n, "a rank without peers owns every row"
-            check(lib.pb_grad_sumsq(ptr(self.grads), int(fp32), sa.n, sa.full, sa.numel, ptr(self._partials), ptr(self._sumsq_counter),
+            check(lib.pb_grad_sumsq(ptr(self.grads), int(fp32), sa.n, sa.full, sa.numel, ptr(self._partials), ptr(self._counters),
                                     ptr(norm_out[i:i + 1]), min(max(sa.total // 16384, sa.n, 1), 148 * 8), stream_ptr()), "pb_grad_sumsq")
         if len(self._segs_step) > 1:
             K.sum_f32(self._norm_parts[:len(self._segs_step)], self._norm_global[0:1])
         for sa in self._segs_step:
             check(lib.pb_zero_adamw_gather(self._peer_params, 1, 0, sa.n, sa.full, sa.shard, sa.numel, ptr(self.master), ptr(self.grads),
                                            2 if fp32 else 1, ptr(self.exp_avg), ptr(self.exp_avg_sq), lr, betas[0], betas[1], eps,
-                                           weight_decay, self.opt_step, ptr(self._norm_global), max_norm, self._opt_ctas(sa), stream_ptr()),
+                                           weight_decay, self.opt_step, ptr(self._norm_global), max_norm, ptr(hyper), self._opt_ctas(sa),
+                                           stream_ptr()),
                   "pb_zero_adamw_gather")
 
     def _reduce_group(self, g: int, overlapped: bool) -> None:
@@ -790,36 +828,106 @@ class FusedLlama:
         B = tokens.shape[0]
         micro_bs = micro_bs or B
         assert B % micro_bs == 0
-        n_micro = B // micro_bs
         if not tokens.is_cuda and self.device.type == "cuda":
             tokens = tokens.to(self.device, non_blocking=True)
             labels = labels.to(self.device, non_blocking=True)
+        if self._graphable(tokens, labels, seq_start, B // micro_bs):
+            report = self._graphed_step(tokens, labels, seq_start, micro_bs, lr, betas, eps, weight_decay, max_norm)
+        else:
+            self._accumulate_micro_batches(tokens, labels, seq_start, micro_bs)
+            norm = self.optimizer_step(lr, betas, eps, weight_decay, max_norm)
+            total = self._buf("step.loss", (2,), torch.float32)
+            if self.device.type != "cuda":
+                return (total[0].item(), norm.item()) if sync_loss else (total[0], norm)
+            report = self._buf("step.report", (4,), torch.float32)
+            self._report(report)
+        if sync_loss:
+            # the step's only device->host read; the device status word rides along, so a peer wait that gave up
+            # (PB_ERR_TIMEOUT_PEER) surfaces as an exception of this step instead of a silently partial update
+            host = report.tolist()
+            if host[3] != 0.0:
+                code = int(host[3])
+                K.status_word(self.device).zero_()
+                raise native.NativeError(f"train_step: device kernel reported error code {code & 0xff} (peer/cta {code >> 8}); "
+                                         "the update of this step is not valid")
+            return host[0], host[2]
+        report = report.clone()
+        return report[0], report[2]
+
+    def _accumulate_micro_batches(self, tokens, labels, seq_start, micro_bs: int) -> None:
+        """Forward and backward of every micro-batch; the averaged losses end in ``step.loss``."""
+        B, T = tokens.shape
+        n_micro = B // micro_bs
         total = self._buf("step.loss", (2,), torch.float32)
-        total.zero_()
         for mb in range(n_micro):
             sl = slice(mb * micro_bs, (mb + 1) * micro_bs)
             ss = None
             if seq_start is not None:
-                T = tokens.shape[1]
-                ss = seq_start[mb * micro_bs * T: (mb + 1) * micro_bs * T] - mb * micro_bs * T
-            out = self.forward_backward(tokens[sl], labels[sl], seq_start=ss, loss_scale=1.0 / n_micro,
-                                        last_microbatch=(mb == n_micro - 1))
-            total[0] += out["loss"] / n_micro
-            total[1] += out["z_loss"] / n_micro
-        norm = self.optimizer_step(lr, betas, eps, weight_decay, max_norm)
-        if sync_loss:
-            # the step's only device->host read; the device status word rides along, so a peer wait that gave up
-            # (PB_ERR_TIMEOUT_PEER) surfaces as an exception of this step instead of a silently partial update
-            st = K.status_word(self.device) if self.device.type == "cuda" else None
-            vals = [total[0], total[1], norm] + ([st[0].to(torch.float32)] if st is not None else [])
-            host = torch.stack(vals).tolist()
-            if st is not None and host[3] != 0.0:
-                code = int(host[3])
-                st.zero_()
-                raise native.NativeError(f"train_step: device kernel reported error code {code & 0xff} (peer/cta {code >> 8}); "
-                                         "the update of this step is not valid")
-            return host[0], host[2]
-        return total[0], norm
+                ss = seq_start[mb * micro_bs * T: (mb + 1) * micro_bs * T]
+                if mb:
+                    ss = ss - mb * micro_bs * T
+            self.forward_backward(tokens[sl], labels[sl], seq_start=ss, loss_scale=1.0 / n_micro, last_microbatch=(mb == n_micro - 1),
+                                  loss_acc=total, first_microbatch=(mb == 0))
+
+    def _report(self, report: torch.Tensor) -> None:
+        check(native.cuda().pb_step_report(ptr(self._ws["step.loss"]), ptr(self._norm_global), ptr(K.status_word(self.device)), ptr(report),
+                                           stream_ptr()), "pb_step_report")
+
+    # ------------------------------------------------------------------------------------------
+    # steps replayed from a CUDA graph
+    # ------------------------------------------------------------------------------------------
+    def _graphable(self, tokens, labels, seq_start, n_micro: int) -> bool:
+        """Small steps without peers are replayed as one graph launch: a launch costs the host about 13 us through the Python
+        wrappers, so a step whose kernels average less than that waits for the host (two-block model, 512 tokens: 69 launches,
+        1.19 ms of host against 0.4 ms of kernels). The line: twice as much host time as the step's operations take at a
+        middling 600 TFLOP/s; above it the queue never runs dry and a graph changes nothing."""
+        if not (self._direct_update and self.wgrad_stream is None and not self._accum and tokens.is_cuda and labels.is_cuda
+                and tokens.dtype == torch.int64 and labels.dtype == torch.int64 and tokens.device == self._counters.device
+                and (seq_start is None or (seq_start.is_cuda and seq_start.dtype == torch.int32))):
+            return False
+        if torch.cuda.is_current_stream_capturing():
+            return False
+        a = self.args
+        launches = (28 * a.n_layers + 10) * n_micro + 4
+        return 6.0 * self.layout.full_numel * tokens.numel() / 600e12 < 2 * launches * 13e-6
+
+    def _graphed_step(self, tokens, labels, seq_start, micro_bs: int, lr: float, betas, eps: float, weight_decay: float,
+                      max_norm: float) -> torch.Tensor:
+        """The step as a graph: recorded at the second call with the same shapes and settings (the first one runs launch by
+        launch and leaves the workspaces allocated), replayed from then on. Inputs and the step's scalars are copied into
+        buffers of the graph, so nothing depends on whose tensors they are. A graph holds every buffer it reads."""
+        self.opt_step += 1
+        B, T = tokens.shape
+        key = (B, T, micro_bs, seq_start is not None, tuple(betas), eps, weight_decay, max_norm, self.z_mode, self.z_weight, self.ce_chunk,
+               self.ac_every)
+        report = self._buf("step.report", (4,), torch.float32)
+        g = self._graphs.get(key)
+        if g is None and key not in self._graph_seen:
+            if len(self._graph_seen) >= 64:
+                self._graph_seen.clear()
+            self._graph_seen.add(key)
+            self._accumulate_micro_batches(tokens, labels, seq_start, micro_bs)
+            self._update_from_own_grads(lr, betas, eps, weight_decay, max_norm)
+            self._accum = False
+            self._report(report)
+            return report
+        if g is None:
+            if len(self._graphs) >= self._MAX_GRAPHS:
+                self._drop_graphs()
+            g = self._graphs[key] = _StepGraph(self, B, T, micro_bs, seq_start is not None, betas, eps, weight_decay, max_norm, report)
+        tokens, labels = tokens.contiguous(), labels.contiguous()
+        seq_start = seq_start.contiguous() if seq_start is not None else None
+        check(native.cuda().pb_stage_step(ptr(tokens), ptr(labels), ptr(seq_start), B * T, ptr(g.tokens), ptr(g.labels), ptr(g.seq_start), lr,
+                                          betas[0], betas[1], self.opt_step, ptr(g.hyper), stream_ptr()), "pb_stage_step")
+        g.graph.replay()
+        native.add_launches(g.launches)
+        return report
+
+    def _drop_graphs(self) -> None:
+        """Graphs point into the workspaces: called before one of those is replaced (the device is idle afterwards)."""
+        if self._graphs:
+            torch.cuda.synchronize(self.device)
+            self._graphs.clear()
 
     # ------------------------------------------------------------------------------------------
     # inference-style forward (logits), used by tests and evaluation

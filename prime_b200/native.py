@@ -38,7 +38,10 @@ _CUDA_SIGS = {
     "pb_swiglu_bwd": [vp, vp, vp, i64, i32, vp],
     "pb_embedding_fwd": [vp, vp, vp, i64, i32, vp],
     "pb_embedding_bwd": [vp, vp, vp, i64, i32, i32, vp],
-    "pb_count_valid": [vp, i64, i32, vp, vp],
+    "pb_count_valid": [vp, i64, i32, vp, vp, vp],
+    "pb_loss_sums": [vp, vp, i32, vp, f32, vp, vp, f32, i32, vp, vp, vp],
+    "pb_stage_step": [vp, vp, vp, i32, vp, vp, vp, f32, f32, f32, i32, vp, vp],
+    "pb_step_report": [vp, vp, vp, vp, vp],
     "pb_cross_entropy": [vp, vp, vp, vp, vp, f32, i64, i32, i64, i32, i32, f32, i32, vp],
     "pb_sum_f32": [vp, i64, vp, vp, f32, vp, i32, vp],
     "pb_sumsq": [vp, i64, i32, vp, vp, i32, vp],
@@ -145,6 +148,12 @@ def check(rc: int, what: str) -> None:
 def launch_counter() -> int:
     """Number of kernels of this package launched since the last reset (this process)."""
     return _launch_count
+
+
+def add_launches(n: int) -> None:
+    """Account for kernels that a replayed graph launched."""
+    global _launch_count
+    _launch_count += n
 
 
 def launch_counter_reset() -> None:

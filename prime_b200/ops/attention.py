@@ -135,7 +135,7 @@ def _small_head_bwd(qkv, o, dout, lse2, seq_start, H, KV, hd, scale, dqkv, rope_
 
 
 def attention_fwd(qkv: torch.Tensor, seq_start: torch.Tensor, H: int, KV: int, hd: int, scale: float | None = None,
-                  out: torch.Tensor | None = None):
+                  out: torch.Tensor | None = None, lse2: torch.Tensor | None = None):
     """Returns (o [M, H*hd] bf16/fp32, lse2 [H, M] fp32 in log2 units of the scaled scores)."""
     M = qkv.shape[0]
     scale = scale if scale is not None else hd ** -0.5
@@ -145,7 +145,8 @@ def attention_fwd(qkv: torch.Tensor, seq_start: torch.Tensor, H: int, KV: int, h
         k = x[:, H * hd: (H + KV) * hd].reshape(M, KV, hd).transpose(0, 1).repeat_interleave(H // KV, dim=0)
         s = (q @ k.transpose(1, 2)) * scale
         s = s.masked_fill(~_dense_mask(seq_start)[None], float("-inf"))
-        lse2 = torch.logsumexp(s, -1) * 1.4426950408889634
+        lse = torch.logsumexp(s, -1) * 1.4426950408889634
+        lse2 = lse if lse2 is None else lse2.copy_(lse)
         o = attention_reference(qkv, seq_start, H, KV, hd, scale).to(qkv.dtype)
         if out is not None:
             out.copy_(o)
@@ -153,10 +154,12 @@ def attention_fwd(qkv: torch.Tensor, seq_start: torch.Tensor, H: int, KV: int, h
         return o, lse2
     assert qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and seq_start.dtype == torch.int32
     if hd not in (64, 128):
-        return _small_head_fwd(qkv, seq_start, H, KV, hd, scale, out)
+        o, lse = _small_head_fwd(qkv, seq_start, H, KV, hd, scale, out)
+        return o, lse if lse2 is None else lse2.copy_(lse)
     if out is None:
         out = torch.empty(M, H * hd, dtype=torch.bfloat16, device=qkv.device)
-    lse2 = torch.empty(H, M, dtype=torch.float32, device=qkv.device)
+    if lse2 is None:
+        lse2 = torch.empty(H, M, dtype=torch.float32, device=qkv.device)
     check(native.cuda().pb_attn_fwd(ptr(qkv), ptr(seq_start), ptr(out), ptr(lse2), M, H, KV, hd, qkv.stride(0),
                                     out.stride(0), scale, ptr(status_word(qkv.device)), stream_ptr()), "pb_attn_fwd")
     return out, lse2

@@ -46,6 +46,11 @@ def _scratch_buf(device, key: str, numel: int, dtype=torch.float32) -> torch.Ten
     return t
 
 
+def scratch_buffers() -> list[torch.Tensor]:
+    """The scratch tensors in use now (a recorded graph keeps them alive: they are replaced when a larger one is needed)."""
+    return [*_scratch.values(), *_SPLITK_WS.values()]
+
+
 # ---------------------------------------------------------------------------------------------
 # GEMM
 # ---------------------------------------------------------------------------------------------
@@ -349,15 +354,34 @@ def embedding_bwd(tokens: torch.Tensor, dout: torch.Tensor, dE: torch.Tensor):
 Z_NONE, Z_MAX, Z_LSE = 0, 1, 2
 
 
-def count_valid(labels: torch.Tensor, ignore_index: int = -100) -> torch.Tensor:
-    """[2] fp32 tensor: (1/count, count) of labels != ignore_index (count clamped to >= 1 for the inverse)."""
-    out = torch.empty(2, dtype=torch.float32, device=labels.device)
+def count_valid(labels: torch.Tensor, ignore_index: int = -100, out: torch.Tensor | None = None,
+                counter: torch.Tensor | None = None) -> torch.Tensor:
+    """[2] fp32 tensor: (1/count, count) of labels != ignore_index (count clamped to >= 1 for the inverse). ``counter``: two
+    zeroed int32 words of the caller's own (zero again afterwards), with which several CTAs share the count."""
+    if out is None:
+        out = torch.empty(2, dtype=torch.float32, device=labels.device)
     if not labels.is_cuda:
         n = int((labels != ignore_index).sum())
         out[0] = 1.0 / max(n, 1)
         out[1] = n
         return out
-    check(native.cuda().pb_count_valid(ptr(labels), labels.numel(), ignore_index, ptr(out), stream_ptr()), "pb_count_valid")
+    check(native.cuda().pb_count_valid(ptr(labels), labels.numel(), ignore_index, ptr(out), ptr(counter), stream_ptr()), "pb_count_valid")
+    return out
+
+
+def loss_sums(loss_rows: torch.Tensor, z_rows: torch.Tensor | None, inv_count: torch.Tensor, z_weight: float, out: torch.Tensor,
+              partial: torch.Tensor | None, counter: torch.Tensor | None, acc: torch.Tensor | None = None, acc_scale: float = 1.0,
+              acc_first: bool = True) -> torch.Tensor:
+    """``out = (mean loss, z_weight * mean z)``; with ``acc`` also ``acc (+)= acc_scale * out``. ``partial`` (>= 296 fp32) and
+    ``counter`` (one zeroed int32 word) are scratch of the caller's own."""
+    if not loss_rows.is_cuda:
+        out[0] = loss_rows.sum() * inv_count[0]
+        out[1] = z_rows.sum() * inv_count[0] * z_weight if z_rows is not None else 0.0
+        if acc is not None:
+            acc.copy_(out * acc_scale if acc_first else acc + out * acc_scale)
+        return out
+    check(native.cuda().pb_loss_sums(ptr(loss_rows), ptr(z_rows), loss_rows.numel(), ptr(inv_count), z_weight, ptr(out), ptr(acc),
+                                     acc_scale, int(acc_first), ptr(partial), ptr(counter), stream_ptr()), "pb_loss_sums")
     return out
 
 

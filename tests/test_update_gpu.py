@@ -59,7 +59,7 @@ def test_adamw_reads_shard_or_own_gradients(segs, kind):
     params = torch.zeros(n_full, dtype=torch.bfloat16, device="cuda")
     sq = torch.tensor([16.0], device="cuda")
     check(native.cuda().pb_zero_adamw_gather((C.c_void_p * 1)(params.data_ptr()), 1, 0, len(segs), full, shard, numel, ptr(p), ptr(gsrc), kind,
-                                             ptr(m), ptr(v), 1e-2, 0.9, 0.95, 1e-8, 0.1, 3, ptr(sq), 1.0, 148, stream_ptr()),
+                                             ptr(m), ptr(v), 1e-2, 0.9, 0.95, 1e-8, 0.1, 3, ptr(sq), 1.0, None, 148, stream_ptr()),
           "pb_zero_adamw_gather")
     for a, b, n in segs:
         g = (gsrc[b: b + n] if kind == 0 else gsrc[a: a + n]).float().cpu()
@@ -68,3 +68,61 @@ def test_adamw_reads_shard_or_own_gradients(segs, kind):
         for got, want in ((p, rp), (m, rm), (v, rv)):
             assert torch.allclose(got[b: b + n].cpu(), want, rtol=2e-5, atol=2e-6)
         assert torch.equal(params[a: a + n], p[b: b + n].bfloat16())
+
+
+@pytest.mark.parametrize("n", [1, 1000, 65536 + 3])
+def test_label_count_and_loss_sums(n):
+    torch.manual_seed(2)
+    labels = torch.randint(0, 50, (n,), device="cuda")
+    labels[::7] = -100
+    cnt = torch.zeros(4, dtype=torch.int32, device="cuda")
+    rows, z = torch.rand(n, device="cuda"), torch.rand(n, device="cuda")
+    partial, acc = torch.zeros(512, device="cuda"), torch.tensor([1.0, 2.0], device="cuda")
+    k = int((labels != -100).sum())
+    for _ in range(2):             # the counters are zero again after a launch
+        inv = K.count_valid(labels, counter=cnt[1:3])
+        assert inv.tolist() == pytest.approx([1.0 / max(k, 1), k], rel=1e-6)
+        out = torch.zeros(2, device="cuda")
+        K.loss_sums(rows, z, inv, 0.5, out, partial, cnt[3:], acc=acc, acc_scale=0.25, acc_first=False)
+    want = [rows.double().sum().item() / max(k, 1), 0.5 * z.double().sum().item() / max(k, 1)]
+    assert out.tolist() == pytest.approx(want, rel=1e-5)
+    assert acc.tolist() == pytest.approx([1.0 + 0.5 * want[0], 2.0 + 0.5 * want[1]], rel=1e-5)
+    K.loss_sums(rows, None, inv, 0.5, out, partial, cnt[3:])
+    assert out.tolist() == pytest.approx([want[0], 0.0], rel=1e-5)
+    assert not cnt.any()
+
+
+@pytest.mark.parametrize("hd,micro,packed,fp32", [(64, 4, False, True), (64, 2, True, True), (32, 2, True, False)])
+def test_graphed_steps_match_steps_launched_one_by_one(monkeypatch, hd, micro, packed, fp32):
+    """Same inputs, new ones each step, one shape in between that makes the workspaces grow and drops the recorded graphs."""
+    from prime_b200.engine.fused_llama import FusedLlama
+    from prime_b200.models.llama import ModelArgs
+    args = ModelArgs(dim=256, n_layers=2, n_heads=256 // hd, ffn_hidden=512, vocab_size=1024, max_seq_len=256, init_mode="normal")
+    dt = torch.float32 if fp32 else torch.bfloat16
+    a, b = (FusedLlama(args, device="cuda", ce_chunk_tokens=512, grad_dtype=dt) for _ in range(2))
+    for e in (a, b):
+        e.init_weights(seed=3)
+    monkeypatch.setattr(b, "_graphable", lambda *x: False)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    replayed = 0
+    for i, (B, T) in enumerate([(4, 200)] * 4 + [(8, 256)] + [(4, 200)] * 3):
+        ids = torch.randint(0, 1024, (B, T + 1), device="cuda", generator=g)
+        ss = None
+        if packed:
+            cut = 37 + 20 * i
+            ss = (torch.arange(B * T, device="cuda", dtype=torch.int32) // T) * T
+            ss += torch.where(torch.arange(B * T, device="cuda") % T >= cut, cut, 0).int()
+        res = [e.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3 * (i + 1), micro_bs=micro, seq_start=ss) for e in (a, b)]
+        replayed += bool(a._graphs)
+        # the kernels are the same; only the embedding gradient's atomic adds may come in another order (bf16: 2^-8 each)
+        assert res[0] == pytest.approx(res[1], rel=2e-3)
+    assert replayed >= 5 and not b._graphs
+    assert a.opt_step == b.opt_step == 8
+    tol = 1e-4 if fp32 else 5e-3
+    assert ((a.master - b.master).norm() / b.master.norm()).item() < tol
+    assert ((a.exp_avg - b.exp_avg).norm() / b.exp_avg.norm()).item() < (1e-3 if fp32 else 3e-2)
+    loss, norm = a.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3, micro_bs=micro, seq_start=ss, sync_loss=False)
+    keep = loss.item()
+    a.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3, micro_bs=micro, seq_start=ss, sync_loss=False)
+    assert loss.item() == keep and norm.item() > 0
+    K.check_status()
