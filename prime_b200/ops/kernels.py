@@ -83,9 +83,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, resi
         assert residual.dtype == out.dtype and residual.shape == out.shape and residual.stride(-1) == 1
     ldr = residual.stride(0) if residual is not None else 0
     # bn: 0 = choose; 128 / 256 = single-CTA tile width; 512 = the CTA-pair (cta_group::2) 256x256 kernel
-    use_pair = bn == 512 or (bn == 0 and _GEMM_PAIR and M >= 512 and N >= 256)
+    slices = _splitk_slices(M, N, K, a.device) if bn == 0 and _GEMM_PAIR else 1
+    use_pair = bn == 512 or slices > 1 or (bn == 0 and _GEMM_PAIR and M >= 512 and N >= 256)
     if use_pair:
-        slices = _splitk_slices(M, N, K, a.device) if bn == 0 else 1
         if slices > 1:
             # few output tiles, long K (weight gradients): K slices as extra work items, fp32 partials, one reduce
             ws = _splitk_ws(slices * M * N, a.device)
@@ -128,8 +128,11 @@ def _splitk_ws(numel: int, device) -> torch.Tensor:
 
 def _splitk_slices(M: int, N: int, K: int, device) -> int:
     """K slices for the CTA-pair GEMM: 1 unless the product has too few 256x256 tiles to fill the GPU and a long
-    K. Minimises waves x k-blocks per slice (0.42 us per k-block) plus the fp32 partials' round trip."""
-    if N % 4 or K < 4096:
+    K. Minimises waves x k-blocks per slice (0.42 us per k-block) plus the fp32 partials' round trip and the reduce
+    launch (5 us). Products of 256 rows or columns are included: the single-CTA kernel that they would otherwise run
+    walks the whole K in a handful of CTAs ([256 x 768] over K = 8192: 58 us in 12 CTAs). A slice keeps at least four k-blocks, below
+    which its pipeline never fills."""
+    if N % 4 or K < 2048 or M < 256 or N < 256:
         return 1
     pairs = _N_PAIRS.get(device)
     if pairs is None:
@@ -139,7 +142,7 @@ def _splitk_slices(M: int, N: int, K: int, device) -> int:
         return 1
     kb = (K + 63) // 64
     best, best_t = 1, -(-tiles // pairs) * kb * 0.42
-    for s_ in range(2, 17):
+    for s_ in range(2, min(32, kb // 4) + 1):
         if s_ * M * N * 4 > (256 << 20):
             break
         t = -(-tiles * s_ // pairs) * -(-kb // s_) * 0.42 + s_ * M * N * 8 / 5e6 + 5.0
