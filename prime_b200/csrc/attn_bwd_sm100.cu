@@ -20,10 +20,11 @@ namespace pb {
 
 struct AttnBwdParams {
     int M, H, KV, n_tiles;
+    int hd;                // columns of a head, <= HD (narrower heads are zero-filled by the tensor maps)
     const int* seq_start;
     const float* lse2;     // [H, M]
     const float* D;        // [H, M]
-    float* dq_acc;         // [M, H*HD] fp32, zero-initialised by the caller
+    float* dq_acc;         // [M, H*hd] fp32, zero-initialised by the caller
     __nv_bfloat16* dqkv;   // [M, (H+2KV)*HD]; the backward kernel writes the k and v column blocks
     long long dqkv_stride;
     float scale, scale_log2;
@@ -166,8 +167,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                     mbar_expect_tx(bar_kv, 2 * Cfg::TILE_BYTES);
 #pragma unroll
                     for (int b = 0; b < NB; ++b) {
-                        tma_load_2d(sK + b * 16384, &tmQKV, bar_kv, (p.H + item.g) * HD + 64 * b, kv0);
-                        tma_load_2d(sV + b * 16384, &tmQKV, bar_kv, (p.H + p.KV + item.g) * HD + 64 * b, kv0);
+                        tma_load_3d(sK + b * 16384, &tmQKV, bar_kv, 64 * b, p.H + item.g, kv0);
+                        tma_load_3d(sV + b * 16384, &tmQKV, bar_kv, 64 * b, p.H + p.KV + item.g, kv0);
                     }
                 }
                 int hq = item.g * G, qi = 0;
@@ -183,10 +184,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                         mbar_expect_tx(bar_qfull + 8 * st, 2 * Cfg::TILE_BYTES);   // Q and dO land on one barrier
 #pragma unroll
                         for (int b = 0; b < NB; ++b)
-                            tma_load_2d(sQ + st * Cfg::TILE_BYTES + b * 16384, &tmQKV, bar_qfull + 8 * st, hq * HD + 64 * b, q0);
+                            tma_load_3d(sQ + st * Cfg::TILE_BYTES + b * 16384, &tmQKV, bar_qfull + 8 * st, 64 * b, hq, q0);
 #pragma unroll
                         for (int b = 0; b < NB; ++b)
-                            tma_load_2d(sDO + st * Cfg::TILE_BYTES + b * 16384, &tmDO, bar_qfull + 8 * st, hq * HD + 64 * b, q0);
+                            tma_load_3d(sDO + st * Cfg::TILE_BYTES + b * 16384, &tmDO, bar_qfull + 8 * st, 64 * b, hq, q0);
                     }
                     __syncwarp();
                     if (++qi == n_q) { qi = 0; ++hq; }
@@ -350,8 +351,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (lane == 0) {
-                        tma_reduce_add_2d(&tmDQ, my_dq, hq * HD + c0, dq_y);
-                        tma_reduce_add_2d(&tmDQ, my_dq + 4096, hq * HD + c0 + 32, dq_y);
+                        if (c0 < p.hd) tma_reduce_add_3d(&tmDQ, my_dq, c0, hq, dq_y);
+                        if (c0 + 32 < p.hd) tma_reduce_add_3d(&tmDQ, my_dq + 4096, c0 + 32, hq, dq_y);
                         tma_store_commit();
                     }
                 }
@@ -498,8 +499,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
             }
             tc_fence_after();
             const int row = kv0 + r;
-            __nv_bfloat16* dk_row = p.dqkv + (long long)row * p.dqkv_stride + (p.H + g) * HD;
-            __nv_bfloat16* dv_row = p.dqkv + (long long)row * p.dqkv_stride + (p.H + p.KV + g) * HD;
+            __nv_bfloat16* dk_row = p.dqkv + (long long)row * p.dqkv_stride + (p.H + g) * p.hd;
+            __nv_bfloat16* dv_row = p.dqkv + (long long)row * p.dqkv_stride + (p.H + p.KV + g) * p.hd;
 #pragma unroll 1
             for (int cidx = half * (HD / 2); cidx < (half + 1) * (HD / 2); cidx += 32) {
                 uint32_t a[32], b[32];
@@ -509,6 +510,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                 if (row < p.M) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {
+                        if (cidx + i >= p.hd) break;
                         uint4 u, w;
                         u.x = pack_bf16x2(__uint_as_float(a[i]) * p.scale, __uint_as_float(a[i + 1]) * p.scale);
                         u.y = pack_bf16x2(__uint_as_float(a[i + 2]) * p.scale, __uint_as_float(a[i + 3]) * p.scale);
@@ -535,13 +537,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
     }
 }
 
-// D[h, m] = sum_d dO[m, h*HD + d] * O[m, h*HD + d]. HD/8 consecutive lanes share one (m, h) row and
-// load 16 bytes each; every thread keeps four rows in flight.
-template <int HD>
+// D[h, m] = sum_d dO[m, h*hd + d] * O[m, h*hd + d]. LPR consecutive lanes (hd / 8 rounded up to a power of two) share one
+// (m, h) row and load 16 bytes each; every thread keeps four rows in flight.
+template <int LPR>
 __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
-                                                            float* __restrict__ D, long long M, int H, long long o_stride,
+                                                            float* __restrict__ D, long long M, int H, int hd, long long o_stride,
                                                             long long do_stride) {
-    constexpr int LPR = HD / 8;                       // lanes per row
     constexpr int ROWS_PER_BLOCK = 256 / LPR;
     pdl_sync();
     const int sub = threadIdx.x % LPR;
@@ -552,11 +553,11 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const long long it = base + u * stride;
-            if (it < total) {
+            if (it < total && sub * 8 < hd) {
                 const long long m = it / H;
                 const int h = int(it - m * H);
-                a[u] = *reinterpret_cast<const uint4*>(o + m * o_stride + h * HD + sub * 8);
-                b[u] = *reinterpret_cast<const uint4*>(dout + m * do_stride + h * HD + sub * 8);
+                a[u] = *reinterpret_cast<const uint4*>(o + m * o_stride + h * hd + sub * 8);
+                b[u] = *reinterpret_cast<const uint4*>(dout + m * do_stride + h * hd + sub * 8);
             } else {
                 a[u] = make_uint4(0, 0, 0, 0);
                 b[u] = make_uint4(0, 0, 0, 0);
@@ -647,10 +648,8 @@ __global__ void attn_bwd_span_kernel(const int* __restrict__ seq_start, int n_ti
 }
 
 int sm_count();
-int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld,
-                      uint32_t box_inner, uint32_t box_outer);
-int make_tmap_f32_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld,
-                     uint32_t box_inner, uint32_t box_outer);
+int make_tmap_heads(CUtensorMap* out, const void* ptr, int elem_bytes, uint64_t hd, uint64_t n_heads, uint64_t outer, uint64_t ld,
+                    uint32_t box_inner, uint32_t box_outer);
 
 template <int HD>
 static int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tdq, const AttnBwdParams& p,
@@ -679,37 +678,36 @@ extern "C" int pb_attn_bwd(const void* qkv, const void* o, const void* dout, con
                            long long qkv_stride, long long o_stride, long long do_stride, long long dqkv_stride, float scale,
                            int* tile_scratch, int* status, void* stream) {
     using namespace pb;
-    if (HD != 64 && HD != 128) return -1;
+    if (HD <= 0 || HD > 128 || HD % 8) return -1;
     if (H % KV) return -1;
     if ((qkv_stride % 8) || (o_stride % 8) || (do_stride % 8) || (dqkv_stride % 8)) return -2;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     CUtensorMap tq, tdo, tdq;
-    int rc = make_tmap_bf16_2d(&tq, qkv, uint64_t(H + 2 * KV) * HD, M, qkv_stride, 64, 128);
+    int rc = make_tmap_heads(&tq, qkv, 2, HD, uint64_t(H + 2 * KV), M, qkv_stride, 64, 128);
     if (rc) return rc;
-    rc = make_tmap_bf16_2d(&tdo, dout, uint64_t(H) * HD, M, do_stride, 64, 128);
+    rc = make_tmap_heads(&tdo, dout, 2, HD, H, M, do_stride, 64, 128);
     if (rc) return rc;
-    rc = make_tmap_f32_2d(&tdq, dq_acc, uint64_t(H) * HD, M, uint64_t(H) * HD, 32, 32);
+    rc = make_tmap_heads(&tdq, dq_acc, 4, HD, H, M, uint64_t(H) * HD, 32, 32);
     if (rc) return rc;
     if (cudaMemsetAsync(dq_acc, 0, size_t(M) * H * HD * sizeof(float), st) != cudaSuccess) return -40;
     if (o) {   // o == null: the caller already filled D
         const long long rows = (long long)M * H;
-        const int rows_per_block = 256 / (HD / 8);
+        const int lpr = HD <= 16 ? 2 : HD <= 32 ? 4 : HD <= 64 ? 8 : 16;
+        const int rows_per_block = 256 / lpr;
         long long blocks = (rows + 4LL * rows_per_block - 1) / (4LL * rows_per_block);
         if (blocks < 1) blocks = 1;
-        if (HD == 64)
-            launch_pdl(attn_bwd_prep_kernel<64>, LaunchCfg(unsigned(blocks), 256, 0, st), (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, D, M, H,
-                                                                         o_stride, do_stride);
-        else
-            launch_pdl(attn_bwd_prep_kernel<128>, LaunchCfg(unsigned(blocks), 256, 0, st), (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, D, M, H,
-                                                                          o_stride, do_stride);
+        auto kern = lpr == 2 ? attn_bwd_prep_kernel<2> : lpr == 4 ? attn_bwd_prep_kernel<4> : lpr == 8 ? attn_bwd_prep_kernel<8>
+                                                                                               : attn_bwd_prep_kernel<16>;
+        launch_pdl(kern, LaunchCfg(unsigned(blocks), 256, 0, st), (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, D, M, H, HD, o_stride,
+                   do_stride);
     }
     AttnBwdParams p;
-    p.M = M; p.H = H; p.KV = KV; p.n_tiles = (M + 127) / 128; p.seq_start = seq_start; p.lse2 = lse2; p.D = D;
+    p.M = M; p.H = H; p.KV = KV; p.hd = HD; p.n_tiles = (M + 127) / 128; p.seq_start = seq_start; p.lse2 = lse2; p.D = D;
     p.dq_acc = dq_acc; p.dqkv = reinterpret_cast<__nv_bfloat16*>(dqkv); p.dqkv_stride = dqkv_stride;
     p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
     if (tile_scratch == nullptr) return -3;
     p.nq = tile_scratch; p.counter = tile_scratch + p.n_tiles; p.n_items = p.n_tiles * KV;
-    rc = HD == 64 ? launch_attn_bwd<64>(tq, tdo, tdq, p, st) : launch_attn_bwd<128>(tq, tdo, tdq, p, st);
+    rc = HD <= 64 ? launch_attn_bwd<64>(tq, tdo, tdq, p, st) : launch_attn_bwd<128>(tq, tdo, tdq, p, st);
     if (rc) return rc;
     const long long total = (long long)M * (H + KV) * (HD / 8);
     long long blocks = (total + 255) / 256;

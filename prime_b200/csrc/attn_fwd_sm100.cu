@@ -1,7 +1,8 @@
 // Causal / document-masked GQA flash attention forward for sm_100a on tcgen05 + TMEM + TMA.
 //
 // Input is the fused, already rotated projection buffer qkv[M, (H + 2*KV) * HD]:
-// q head h at column h*HD, k head g at (H + g)*HD, v head g at (H + KV + g)*HD.
+// q head h at column h*hd, k head g at (H + g)*hd, v head g at (H + KV + g)*hd. The kernel is built for HD = 64 or 128 columns
+// per head; a narrower head (hd a multiple of 8) is zero-filled to HD by the tensor map, and only its hd columns are written.
 // The M rows are a packed token stream; seq_start[m] is the first row query m may attend to
 // (start of its batch row or, with sequence packing, of its document), and m itself is the
 // last (causal). This replaces repeat_kv + FlexAttention/SDPA of the reference
@@ -23,6 +24,7 @@ namespace pb {
 
 struct AttnFwdParams {
     int M, H, KV;
+    int hd;             // columns of a head, <= HD
     const int* seq_start;
     __nv_bfloat16* O;
     long long o_stride;
@@ -119,7 +121,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
             if (lane == 0) {
                 mbar_expect_tx(bar_q, Cfg::TILE_BYTES);
 #pragma unroll
-                for (int b = 0; b < NB; ++b) tma_load_2d(sQ + b * 16384, &tm, bar_q, head * HD + 64 * b, q0);
+                for (int b = 0; b < NB; ++b) tma_load_3d(sQ + b * 16384, &tm, bar_q, 64 * b, head, q0);
             }
             bool ok = true;
             for (int j = 0; j < n_kv && ok; ++j) {
@@ -133,11 +135,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
                     mbar_expect_tx(bar_kfull + 8 * st, Cfg::TILE_BYTES);
 #pragma unroll
                     for (int b = 0; b < NB; ++b)
-                        tma_load_2d(sK + st * Cfg::TILE_BYTES + b * 16384, &tm, bar_kfull + 8 * st, (p.H + kvh) * HD + 64 * b, kv0);
+                        tma_load_3d(sK + st * Cfg::TILE_BYTES + b * 16384, &tm, bar_kfull + 8 * st, 64 * b, p.H + kvh, kv0);
                     mbar_expect_tx(bar_vfull + 8 * st, Cfg::TILE_BYTES);
 #pragma unroll
                     for (int b = 0; b < NB; ++b)
-                        tma_load_2d(sV + st * Cfg::TILE_BYTES + b * 16384, &tm, bar_vfull + 8 * st, (p.H + p.KV + kvh) * HD + 64 * b, kv0);
+                        tma_load_3d(sV + st * Cfg::TILE_BYTES + b * 16384, &tm, bar_vfull + 8 * st, 64 * b, p.H + p.KV + kvh, kv0);
                 }
                 __syncwarp();
             }
@@ -321,7 +323,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
         if (ok) {
             tc_fence_after();
             const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-            __nv_bfloat16* dst = p.O + (long long)row * p.o_stride + head * HD;
+            __nv_bfloat16* dst = p.O + (long long)row * p.o_stride + head * p.hd;
 #pragma unroll
             for (int cidx = 0; cidx < HD; cidx += 32) {
                 uint32_t o[32];
@@ -330,6 +332,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
                 if (row < p.M) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {
+                        if (cidx + i >= p.hd) break;
                         uint4 u;
                         u.x = pack_bf16x2(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
                         u.y = pack_bf16x2(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
@@ -352,8 +355,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
     }
 }
 
-int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld,
-                      uint32_t box_inner, uint32_t box_outer);
+int make_tmap_heads(CUtensorMap* out, const void* ptr, int elem_bytes, uint64_t hd, uint64_t n_heads, uint64_t outer, uint64_t ld,
+                    uint32_t box_inner, uint32_t box_outer);
 
 template <int HD>
 static int launch_attn_fwd(const CUtensorMap& tm, const AttnFwdParams& p, cudaStream_t st) {
@@ -374,15 +377,15 @@ static int launch_attn_fwd(const CUtensorMap& tm, const AttnFwdParams& p, cudaSt
 extern "C" int pb_attn_fwd(const void* qkv, const int* seq_start, void* o, float* lse2, int M, int H, int KV, int HD,
                            long long qkv_stride, long long o_stride, float scale, int* status, void* stream) {
     using namespace pb;
-    if (HD != 64 && HD != 128) return -1;
+    if (HD <= 0 || HD > 128 || HD % 8) return -1;
     if (H % KV) return -1;
     if ((qkv_stride % 8) || (o_stride % 8) || (reinterpret_cast<uintptr_t>(qkv) & 15) || (reinterpret_cast<uintptr_t>(o) & 15)) return -2;
     CUtensorMap tm;
-    int rc = make_tmap_bf16_2d(&tm, qkv, uint64_t(H + 2 * KV) * HD, M, qkv_stride, 64, 128);
+    int rc = make_tmap_heads(&tm, qkv, 2, HD, uint64_t(H + 2 * KV), M, qkv_stride, 64, 128);
     if (rc) return rc;
     AttnFwdParams p;
-    p.M = M; p.H = H; p.KV = KV; p.seq_start = seq_start; p.O = reinterpret_cast<__nv_bfloat16*>(o); p.o_stride = o_stride;
+    p.M = M; p.H = H; p.KV = KV; p.hd = HD; p.seq_start = seq_start; p.O = reinterpret_cast<__nv_bfloat16*>(o); p.o_stride = o_stride;
     p.lse2 = lse2; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    return HD == 64 ? launch_attn_fwd<64>(tm, p, st) : launch_attn_fwd<128>(tm, p, st);
+    return HD <= 64 ? launch_attn_fwd<64>(tm, p, st) : launch_attn_fwd<128>(tm, p, st);
 }

@@ -230,18 +230,20 @@ int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_
     return r == CUDA_SUCCESS ? 0 : -(1000 + int(r));
 }
 
-// 2-D fp32 tensor map (used as the destination of bulk reduce-adds)
-int make_tmap_f32_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld,
-                     uint32_t box_inner, uint32_t box_outer) {
+// Heads of `hd` columns side by side in rows of `outer`: dims {hd, n_heads, outer}, box {box_inner, 1, box_outer}. A box wider
+// than the head reads zeros past its last column (and a store or reduce clips them), so a kernel built for 64 or 128 columns
+// takes any narrower head without a padded copy. elem_bytes: 2 = bf16, 4 = fp32.
+int make_tmap_heads(CUtensorMap* out, const void* ptr, int elem_bytes, uint64_t hd, uint64_t n_heads, uint64_t outer, uint64_t ld,
+                    uint32_t box_inner, uint32_t box_outer) {
     EncodeTiledFn enc = get_encode_fn();
     if (!enc) return -10;
-    cuuint64_t dims[2] = {inner, outer};
-    cuuint64_t strides[1] = {ld * 4};
-    cuuint32_t box[2] = {box_inner, box_outer};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    cuuint64_t dims[3] = {hd, n_heads, outer};
+    cuuint64_t strides[2] = {hd * elem_bytes, ld * elem_bytes};
+    cuuint32_t box[3] = {box_inner, 1, box_outer};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(out, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(ptr), dims,
+                     strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : -(1000 + int(r));
 }
 

@@ -61,43 +61,22 @@ def attention_reference(qkv: torch.Tensor, seq_start: torch.Tensor, H: int, KV: 
     return (p @ v).transpose(0, 1).reshape(M, H * hd)
 
 
-_warned_small_head = False
+_warned_dense = False
 
 
-def _padded_hd(hd: int) -> int:
-    """Kernel head size that a head of ``hd`` columns is zero-padded to (0: none fits)."""
-    return 64 if hd < 64 else 128 if hd < 128 else 0
+def _kernel_head(hd: int) -> bool:
+    """The tcgen05 kernels take heads of up to 128 columns in 16-byte steps; below 64 (or between 64 and 128) their tensor maps
+    fill the missing columns with zeros, which changes neither the scores nor the real output columns."""
+    return hd <= 128 and hd % 8 == 0
 
 
-def _pad_heads(x: torch.Tensor, n_heads: int, hd: int, to: int) -> torch.Tensor:
-    """[M, n_heads * hd] -> [M, n_heads * to], every head zero-padded on the right."""
-    M = x.shape[0]
-    out = x.new_zeros(M, n_heads, to)
-    out[:, :, :hd] = x.reshape(M, n_heads, hd)
-    return out.view(M, n_heads * to)
-
-
-def _cut_heads(x: torch.Tensor, n_heads: int, hd: int, padded: int) -> torch.Tensor:
-    return x.view(x.shape[0], n_heads, padded)[:, :, :hd].reshape(x.shape[0], n_heads * hd)
-
-
-def _small_head_fwd(qkv, seq_start, H, KV, hd, scale, out):
-    """Head sizes other than 64 / 128 (the debug presets: 16 and 32). Heads that fit are zero-padded to the next kernel
-    head size, which changes neither the scores nor the real output columns, so these models run the same tcgen05
-    kernels; larger heads run the dense fp32 statement on the device."""
-    to = _padded_hd(hd)
-    if to and hd % 8 == 0:
-        o_p, lse2 = attention_fwd(_pad_heads(qkv, H + 2 * KV, hd, to), seq_start, H, KV, to, scale)
-        o = _cut_heads(o_p, H, hd, to)
-        if out is not None:
-            out.copy_(o)
-            o = out
-        return o, lse2
-    global _warned_small_head
-    if not _warned_small_head:
+def _dense_fwd(qkv, seq_start, H, KV, hd, scale, out):
+    """Heads that have no tcgen05 kernel (above 128 columns, or not a multiple of 8): the dense fp32 statement on the device."""
+    global _warned_dense
+    if not _warned_dense:
         import warnings
-        warnings.warn(f"head_dim={hd} has no tcgen05 attention kernel (64 and 128 do); using dense attention")
-        _warned_small_head = True
+        warnings.warn(f"head_dim={hd} has no tcgen05 attention kernel (multiples of 8 up to 128 do); using dense attention")
+        _warned_dense = True
     M = qkv.shape[0]
     x = qkv.float()
     q = x[:, : H * hd].reshape(M, H, hd).transpose(0, 1)
@@ -111,17 +90,7 @@ def _small_head_fwd(qkv, seq_start, H, KV, hd, scale, out):
     return o, lse2
 
 
-def _small_head_bwd(qkv, o, dout, lse2, seq_start, H, KV, hd, scale, dqkv, rope_table, seq_len, row_dots):
-    to = _padded_hd(hd)
-    if to and hd % 8 == 0:
-        g_p = attention_bwd(_pad_heads(qkv, H + 2 * KV, hd, to), _pad_heads(o, H, hd, to), _pad_heads(dout, H, hd, to), lse2,
-                            seq_start, H, KV, to, scale, row_dots=row_dots)
-        g = _cut_heads(g_p, H + 2 * KV, hd, to).contiguous()
-        if rope_table is not None:      # the kernel's own inverse rotation pairs columns of the padded head: done here instead
-            from .kernels import rope_
-            g = rope_(g, rope_table, seq_len, H + KV, hd, backward=True)
-        dqkv.copy_(g)
-        return dqkv
+def _dense_bwd(qkv, dout, seq_start, H, KV, hd, scale, dqkv, rope_table, seq_len):
     with torch.enable_grad():
         x = qkv.detach().float().requires_grad_(True)
         ref = attention_reference(x, seq_start, H, KV, hd, scale)
@@ -153,8 +122,8 @@ def attention_fwd(qkv: torch.Tensor, seq_start: torch.Tensor, H: int, KV: int, h
             o = out
         return o, lse2
     assert qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and seq_start.dtype == torch.int32
-    if hd not in (64, 128):
-        o, lse = _small_head_fwd(qkv, seq_start, H, KV, hd, scale, out)
+    if not _kernel_head(hd):
+        o, lse = _dense_fwd(qkv, seq_start, H, KV, hd, scale, out)
         return o, lse if lse2 is None else lse2.copy_(lse)
     if out is None:
         out = torch.empty(M, H * hd, dtype=torch.bfloat16, device=qkv.device)
@@ -192,8 +161,8 @@ def attention_bwd(qkv: torch.Tensor, o: torch.Tensor, dout: torch.Tensor, lse2: 
         dqkv.copy_(g.to(dqkv.dtype))
         return dqkv
     assert dout.stride(1) == 1 and o.stride(1) == 1 and dqkv.stride(1) == 1
-    if hd not in (64, 128):
-        return _small_head_bwd(qkv, o, dout, lse2, seq_start, H, KV, hd, scale, dqkv, rope_table, seq_len, row_dots)
+    if not _kernel_head(hd):
+        return _dense_bwd(qkv, dout, seq_start, H, KV, hd, scale, dqkv, rope_table, seq_len)
     dq_acc = _scratch_buf(qkv.device, "attn_dq", M * H * hd)
     D = row_dots if row_dots is not None else _scratch_buf(qkv.device, "attn_D", M * H)
     tiles = _scratch_buf(qkv.device, "attn_tiles", (M + 127) // 128 + 1, torch.int32)

@@ -199,7 +199,8 @@ def gemm_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, table: torch.
     row (position = row index modulo ``seq_len``) before the store. Falls back to GEMM + rope_."""
     M, K = x.shape
     N = w.shape[0]
-    if x.is_cuda and _pair_ok(M, N) and head_dim % 64 == 0 and out.stride(-1) == 1 and table.shape[0] >= seq_len:
+    if (x.is_cuda and _pair_ok(M, N) and (head_dim % 64 == 0 or head_dim in (8, 16, 32)) and n_rot_heads * head_dim % 64 == 0
+            and out.stride(-1) == 1 and table.shape[0] >= seq_len):
         _gemm_epi(x, w, out, M, N, K, False, 2, seq_len, n_rot_heads * head_dim, head_dim, table, "rope")
         return out
     gemm(x, w, out=out)

@@ -1,7 +1,8 @@
-"""Sizes at the edges of the GEMM dispatch: few rows, short K."""
+"""Sizes at the edges of the GEMM and attention dispatch: few rows, short K, narrow heads."""
 import pytest
 import torch
 
+from prime_b200.ops import attention as A
 from prime_b200.ops import kernels as ops
 
 pytestmark = pytest.mark.gpu
@@ -26,3 +27,39 @@ def test_split_k_of_narrow_products(M, N, K, res):
         ops.gemm(a, b, out=out, residual=r, a_mn=True, b_mn=True)
         ops.check_status()
         assert _rel(out, ref + (r.float() if res else 0)) < (1e-2 if dt == torch.bfloat16 else 1e-3)
+
+
+# heads of 8 to 120 columns through the 64- and 128-column kernels; M no multiple of the 128-row tile
+@pytest.mark.parametrize("hd", [8, 16, 32, 40, 72, 96, 120])
+def test_narrow_heads(hd):
+    torch.manual_seed(0)
+    B, T, H, KV = 2, 203, 4, 2
+    qkv = torch.randn(B * T, (H + 2 * KV) * hd, device="cuda", dtype=torch.bfloat16)
+    ss = A.seq_start_from_seqlens([[100, 103], [203]], T, "cuda")
+    o, lse2 = A.attention_fwd(qkv, ss, H, KV, hd)
+    x = qkv.float().requires_grad_(True)
+    ref = A.attention_reference(x, ss, H, KV, hd)
+    assert _rel(o, ref.detach()) < 2e-2
+    dout = torch.randn(B * T, H * hd, device="cuda", dtype=torch.bfloat16)
+    table = ops.rope_table(T, hd, 10000.0, "cuda")
+    g = A.attention_bwd(qkv, o, dout, lse2, ss, H, KV, hd, rope_table=table, seq_len=T)
+    ops.check_status()
+    (gref,) = torch.autograd.grad(ref, x, dout.float())
+    gref = ops.rope_(gref.cpu(), table.cpu(), T, H + KV, hd, backward=True).cuda()
+    # bf16 P and dS (2^-9 each) against fp32: as for the full-width heads
+    assert _rel(g, gref) < 3e-2
+
+
+@pytest.mark.parametrize("hd", [16, 32])
+def test_rope_epilogue_narrow_heads(hd):
+    torch.manual_seed(0)
+    M, K, T, H, KV = 777, 256, 200, 256 // hd, 128 // hd
+    N = (H + 2 * KV) * hd
+    x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()
+    table = ops.rope_table(T, hd, 10000.0, "cuda")
+    out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    ops.gemm_rope(x, w, out, table, T, H + KV, hd)
+    ref = ops.rope_((x.float() @ w.float().t()).cpu(), table.cpu(), T, H + KV, hd).cuda()
+    ops.check_status()
+    assert _rel(out, ref) < 1e-2
