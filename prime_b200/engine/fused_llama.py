@@ -120,6 +120,7 @@ class _StepGraph:
         self.graph = torch.cuda.CUDAGraph()
         main, side = torch.cuda.current_stream(dev), torch.cuda.Stream(device=dev)
         side.wait_stream(main)
+        K.take_scratch(side)                             # of earlier users of this handle: the graph gets its own
         before = native.launch_counter()
         with torch.cuda.stream(side):
             self.graph.capture_begin(capture_error_mode="thread_local")
@@ -133,7 +134,7 @@ class _StepGraph:
         main.wait_stream(side)
         self.launches = native.launch_counter() - before
         native.add_launches(-self.launches)              # recorded, not run
-        self.refs = [report, *eng._ws.values(), *eng._seq_start_cache.values(), *K.scratch_buffers()]
+        self.refs = [report, *eng._ws.values(), *eng._seq_start_cache.values(), *K.take_scratch(side)]
 
 
 class FusedLlama:
@@ -731,9 +732,14 @@ class FusedLlama:
     @property
     def grad_shard(self) -> torch.Tensor:
         """This rank's reduced fp32 gradients, one value per owned parameter element. A run without peers that updates with the
-        AdamW kernel never asks for it (4 bytes per parameter that stay free)."""
+        AdamW kernel never asks for it (4 bytes per parameter that stay free); there it is filled from the gradient buffer on
+        each access."""
         if self._grad_shard is None:
             self._grad_shard = torch.zeros(self.layout.shard_numel[self.rank], dtype=torch.float32, device=self.device)
+        if self._direct_update:
+            for sa in self._segs_step:
+                for f, s, n in zip(sa.full[:sa.n], sa.shard[:sa.n], sa.numel[:sa.n]):
+                    self._grad_shard[s: s + n].copy_(self.grads[f: f + n])
         return self._grad_shard
 
     @property

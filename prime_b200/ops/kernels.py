@@ -17,7 +17,7 @@ import os as _os
 # PRIME_B200_GEMM=single forces the single-CTA kernel (A/B measurements); default uses the CTA-pair kernel when it fits
 _GEMM_PAIR = _os.environ.get("PRIME_B200_GEMM", "pair") != "single"
 _status: dict[int, torch.Tensor] = {}
-_scratch: dict[tuple[int, str], torch.Tensor] = {}
+_scratch: dict[tuple[int, int, str], torch.Tensor] = {}       # by device, stream and use
 
 
 def status_word(device: torch.device) -> torch.Tensor:
@@ -38,17 +38,23 @@ def check_status(device: torch.device | None = None) -> None:
 
 
 def _scratch_buf(device, key: str, numel: int, dtype=torch.float32) -> torch.Tensor:
-    k = (device.index or 0, key)
+    """Scratch of one use on the current stream: kernels of other streams (weight gradients beside the backward, another
+    thread's model) run at the same time and have their own. At most 64 are kept, the oldest go back to the allocator."""
+    k = (device.index or 0, torch.cuda.current_stream(device).cuda_stream, key)
     t = _scratch.get(k)
     if t is None or t.numel() < numel or t.dtype != dtype:
+        for old in list(_scratch)[:max(0, len(_scratch) - 63)]:
+            _scratch.pop(old, None)
         t = torch.empty(numel, dtype=dtype, device=device)
         _scratch[k] = t
     return t
 
 
-def scratch_buffers() -> list[torch.Tensor]:
-    """The scratch tensors in use now (a recorded graph keeps them alive: they are replaced when a larger one is needed)."""
-    return [*_scratch.values(), *_SPLITK_WS.values()]
+def take_scratch(stream: torch.cuda.Stream) -> list[torch.Tensor]:
+    """Hand over the scratch of ``stream``, which then starts anew: a recorded graph owns what was allocated while it was recorded,
+    since its replays may run beside other work on whichever stream has that handle later."""
+    keys = [k for k in list(_scratch) if k[1] == stream.cuda_stream]
+    return [t for t in (_scratch.pop(k, None) for k in keys) if t is not None]
 
 
 # ---------------------------------------------------------------------------------------------
@@ -88,7 +94,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, resi
     if use_pair:
         if slices > 1:
             # few output tiles, long K (weight gradients): K slices as extra work items, fp32 partials, one reduce
-            ws = _splitk_ws(slices * M * N, a.device)
+            ws = _scratch_buf(a.device, "splitk", slices * M * N)
             rc = native.cuda().pb_gemm_bf16_pair_splitk(ptr(a), ptr(b), ptr(ws), M, N, K, a.stride(0), b.stride(0), int(a_mn),
                                                         int(b_mn), slices, max_ctas, ptr(status_word(a.device)), stream_ptr())
             check(rc, f"pb_gemm_bf16_pair_splitk(M={M},N={N},K={K},slices={slices})")
@@ -114,16 +120,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, resi
     return out
 
 
-_SPLITK_WS: dict = {}
 _N_PAIRS: dict = {}
-
-
-def _splitk_ws(numel: int, device) -> torch.Tensor:
-    t = _SPLITK_WS.get(device)
-    if t is None or t.numel() < numel:
-        t = torch.empty(numel, dtype=torch.float32, device=device)
-        _SPLITK_WS[device] = t
-    return t
 
 
 def _splitk_slices(M: int, N: int, K: int, device) -> int:

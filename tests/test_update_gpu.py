@@ -126,3 +126,30 @@ def test_graphed_steps_match_steps_launched_one_by_one(monkeypatch, hd, micro, p
     a.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3, micro_bs=micro, seq_start=ss, sync_loss=False)
     assert loss.item() == keep and norm.item() > 0
     K.check_status()
+
+
+def test_grad_shard_holds_the_gradients_of_a_step_without_peers():
+    from prime_b200.engine.fused_llama import FusedLlama
+    from prime_b200.models.llama import ModelArgs
+    eng = FusedLlama(ModelArgs(dim=256, n_layers=2, n_heads=4, ffn_hidden=512, vocab_size=1024, max_seq_len=256, init_mode="normal"),
+                     device="cuda", ce_chunk_tokens=512)
+    eng.init_weights(seed=3)
+    ids = torch.randint(0, 1024, (2, 129), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    for _ in range(3):
+        loss, norm = eng.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3)
+        # the norm is the root of the shard's sum of squares: fp32 sums, far below 1e-4
+        assert eng.grad_shard.double().norm().item() == pytest.approx(norm, rel=1e-4)
+    for name, g in eng.g.items():
+        assert torch.equal(eng.shard_view(eng.grad_shard, name), g.float())
+
+
+def test_scratch_is_one_per_stream():
+    a = torch.randn(4096, 256, device="cuda").bfloat16()
+    K.gemm(a, a, a_mn=True, b_mn=True)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        K.gemm(a, a, a_mn=True, b_mn=True)
+    torch.cuda.synchronize()
+    ws = [t.data_ptr() for k, t in K._scratch.items() if k[2] == "splitk"]
+    assert len(ws) >= 2 and len(set(ws)) == len(ws)
+    assert K.take_scratch(side) and not any(k[1] == side.cuda_stream for k in K._scratch)
