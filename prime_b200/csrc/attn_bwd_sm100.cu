@@ -698,7 +698,7 @@ extern "C" int pb_attn_bwd(const void* qkv, const void* o, const void* dout, con
         if (blocks < 1) blocks = 1;
         auto kern = lpr == 2 ? attn_bwd_prep_kernel<2> : lpr == 4 ? attn_bwd_prep_kernel<4> : lpr == 8 ? attn_bwd_prep_kernel<8>
                                                                                                : attn_bwd_prep_kernel<16>;
-        launch_pdl(kern, LaunchCfg(unsigned(blocks), 256, 0, st), (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, D, M, H, HD, o_stride,
+        launch_pdl(kern, LaunchCfg(unsigned(blocks), 256, 0, st).traffic(4.0 * rows * HD), (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, D, M, H, HD, o_stride,
                    do_stride);
     }
     AttnBwdParams p;
@@ -712,7 +712,7 @@ extern "C" int pb_attn_bwd(const void* qkv, const void* o, const void* dout, con
     const long long total = (long long)M * (H + KV) * (HD / 8);
     long long blocks = (total + 255) / 256;
     if (blocks > 148 * 8) blocks = 148 * 8;
-    launch_pdl(attn_bwd_finish_kernel, LaunchCfg(unsigned(blocks), 256, 0, st), dq_acc, (__nv_bfloat16*)dqkv, rope_table, M, T, H, KV, HD, dqkv_stride,
+    launch_pdl(attn_bwd_finish_kernel, LaunchCfg(unsigned(blocks), 256, 0, st).traffic(6.0 * M * H * HD), dq_acc, (__nv_bfloat16*)dqkv, rope_table, M, T, H, KV, HD, dqkv_stride,
                                                               rope_table != nullptr);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }

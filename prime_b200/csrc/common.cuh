@@ -155,7 +155,11 @@ struct ItemRing {
 // predecessor has completed and its writes are visible, and only then lets the successor start, so at most one kernel waits at
 // a time and everything before the predecessor is complete as well. Rules: no global memory access before pdl_sync(),
 // every thread calls it, and kernels that talk to other GPUs are launched the ordinary way.
-// (pdl_sync() does nothing in an ordinary launch.) Measured: forward pass of the 150M model over 3 x 777 tokens, 87 launches,
+// (pdl_sync() does nothing in an ordinary launch.)
+// CTAs of an early launch go to the first SMs that have room and pile up there, while the grids of the streaming kernels are
+// made for an even share of every SM: the AdamW pass of the 10B blocks (148 CTAs, 58 GB) took 18 ms instead of 11.4. Such a
+// kernel says how many bytes it moves (LaunchCfg::traffic) and is launched early only below 32 MB, which take about as long as
+// the 5 us that an early launch saves. Measured: forward pass of the 150M model over 3 x 777 tokens, 87 launches,
 // 2.10 -> 1.91 ms; 70M step of 32 x 1024 tokens, 388 launches, 13.5 -> 13.1 ms; nothing on steps of 100 ms and more.
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_sync() {
@@ -165,9 +169,11 @@ __device__ __forceinline__ void pdl_sync() {
 
 struct LaunchCfg {
     cudaLaunchConfig_t c{};
+    bool early = true;
     LaunchCfg(dim3 grid, dim3 block, size_t smem, cudaStream_t st) {
         c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = st;
     }
+    LaunchCfg& traffic(double bytes) { early = bytes < 32e6; return *this; }
 };
 template <typename... P, typename... A>
 static inline cudaError_t launch_pdl(void (*kern)(P...), LaunchCfg cfg, A&&... args) {
@@ -175,7 +181,7 @@ static inline cudaError_t launch_pdl(void (*kern)(P...), LaunchCfg cfg, A&&... a
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.c.attrs = at;
-    cfg.c.numAttrs = 1;
+    cfg.c.numAttrs = cfg.early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg.c, kern, static_cast<P>(args)...);
 }
 

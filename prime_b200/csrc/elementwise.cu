@@ -497,7 +497,7 @@ using namespace pb;
 
 extern "C" int pb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int M, int N, float eps, void* stream) {
     if (N % 8) return -1;
-    launch_pdl(rmsnorm_fwd_kernel, LaunchCfg(grid_for(M, 8), 256, 0, ST(stream)), (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+    launch_pdl(rmsnorm_fwd_kernel, LaunchCfg(grid_for(M, 8), 256, 0, ST(stream)).traffic(4.0 * M * N), (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
                                                                 (__nv_bfloat16*)y, rstd, M, N, eps);
     return CHECK_LAUNCH();
 }
@@ -513,7 +513,7 @@ extern "C" int pb_rmsnorm_bwd(const void* x, const void* w, const float* rstd, c
     auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w; auto DY = (const __nv_bfloat16*)dy;
     auto DR = (const __nv_bfloat16*)dres; auto DX = (__nv_bfloat16*)dx;
     // rows wider than 1024 are shared by two or four warps (at most four 256-column chunks per warp)
-#define RB(NCH, WPR) case NCH: launch_pdl(rmsnorm_bwd_kernel<NCH, WPR>, LaunchCfg(ctas, 256, 0, ST(stream)), X, W, rstd, DY, DR, DX, dw_partial, M); break;
+#define RB(NCH, WPR) case NCH: launch_pdl(rmsnorm_bwd_kernel<NCH, WPR>, LaunchCfg(ctas, 256, 0, ST(stream)).traffic(8.0 * M * N), X, W, rstd, DY, DR, DX, dw_partial, M); break;
     switch (N / 256) {
         RB(1, 1) RB(2, 1) RB(3, 1) RB(4, 1) RB(6, 2) RB(8, 2) RB(12, 4) RB(16, 4)
         default: return -1;
@@ -527,31 +527,31 @@ extern "C" int pb_rmsnorm_bwd(const void* x, const void* w, const float* rstd, c
 extern "C" int pb_rope(void* qkv, const float* table, long long M, int T, int n_rot_heads, int hd, int row_stride,
                        int backward, void* stream) {
     if (hd % 8 || row_stride % 8) return -1;
-    launch_pdl(rope_kernel, LaunchCfg(grid_for(M * n_rot_heads * (hd / 8), 256), 256, 0, ST(stream)), 
+    launch_pdl(rope_kernel, LaunchCfg(grid_for(M * n_rot_heads * (hd / 8), 256), 256, 0, ST(stream)).traffic(4.0 * M * n_rot_heads * hd), 
         (__nv_bfloat16*)qkv, table, M, T, n_rot_heads, hd, row_stride, backward ? -1.f : 1.f);
     return CHECK_LAUNCH();
 }
 
 extern "C" int pb_swiglu_fwd(const void* h13, void* act, long long M, int F, void* stream) {
     if (F % 8) return -1;
-    launch_pdl(swiglu_fwd_kernel, LaunchCfg(grid_for(M * (F / 8), 256), 256, 0, ST(stream)), (const __nv_bfloat16*)h13, (__nv_bfloat16*)act, M, F);
+    launch_pdl(swiglu_fwd_kernel, LaunchCfg(grid_for(M * (F / 8), 256), 256, 0, ST(stream)).traffic(6.0 * M * F), (const __nv_bfloat16*)h13, (__nv_bfloat16*)act, M, F);
     return CHECK_LAUNCH();
 }
 extern "C" int pb_swiglu_bwd(const void* h13, const void* dact, void* dh13, long long M, int F, void* stream) {
     if (F % 8) return -1;
-    launch_pdl(swiglu_bwd_kernel, LaunchCfg(grid_for(M * (F / 8), 256), 256, 0, ST(stream)), (const __nv_bfloat16*)h13, (const __nv_bfloat16*)dact,
+    launch_pdl(swiglu_bwd_kernel, LaunchCfg(grid_for(M * (F / 8), 256), 256, 0, ST(stream)).traffic(10.0 * M * F), (const __nv_bfloat16*)h13, (const __nv_bfloat16*)dact,
                                                                           (__nv_bfloat16*)dh13, M, F);
     return CHECK_LAUNCH();
 }
 
 extern "C" int pb_embedding_fwd(const long long* tok, const void* E, void* out, long long M, int D, void* stream) {
     if (D % 8) return -1;
-    launch_pdl(embedding_fwd_kernel, LaunchCfg(grid_for(M * (D / 8), 256), 256, 0, ST(stream)), tok, (const __nv_bfloat16*)E, (__nv_bfloat16*)out, M, D);
+    launch_pdl(embedding_fwd_kernel, LaunchCfg(grid_for(M * (D / 8), 256), 256, 0, ST(stream)).traffic(4.0 * M * D), tok, (const __nv_bfloat16*)E, (__nv_bfloat16*)out, M, D);
     return CHECK_LAUNCH();
 }
 extern "C" int pb_embedding_bwd(const long long* tok, const void* dout, void* dE, long long M, int D, int grad_fp32, void* stream) {
     if (D % 8) return -1;
-    launch_pdl(embedding_bwd_kernel, LaunchCfg(grid_for(M * (D / 8), 256), 256, 0, ST(stream)), tok, (const __nv_bfloat16*)dout, dE, M, D, grad_fp32);
+    launch_pdl(embedding_bwd_kernel, LaunchCfg(grid_for(M * (D / 8), 256), 256, 0, ST(stream)).traffic(6.0 * M * D), tok, (const __nv_bfloat16*)dout, dE, M, D, grad_fp32);
     return CHECK_LAUNCH();
 }
 
@@ -592,7 +592,7 @@ extern "C" int pb_cross_entropy(void* logits, const long long* labels, float* lo
     if (ld % 8) return -1;
     // 256 threads per row: more resident CTAs per SM overlap one row's exponentials with another's loads (260 us
     // against 296 us with 512 threads for 8192 x 32000)
-    launch_pdl(cross_entropy_kernel, LaunchCfg((unsigned)rows, 256, 0, ST(stream)), (__nv_bfloat16*)logits, labels, loss_rows, z_rows, inv_count,
+    launch_pdl(cross_entropy_kernel, LaunchCfg((unsigned)rows, 256, 0, ST(stream)).traffic(4.0 * rows * V), (__nv_bfloat16*)logits, labels, loss_rows, z_rows, inv_count,
                                                                  grad_scale, V, ld, ignore_index, z_mode, z_weight, write_grad);
     return CHECK_LAUNCH();
 }
@@ -609,8 +609,8 @@ extern "C" int pb_sum_f32(const float* x, long long n, float* scratch, const flo
 // out (+)= sum(x^2) ; scratch >= 1024 floats
 extern "C" int pb_sumsq(const void* x, long long n, int is_fp32, float* scratch, float* out, int accumulate, void* stream) {
     const int nb = grid_for(n, 256, 1024);
-    if (is_fp32) launch_pdl(sumsq_kernel<float>, LaunchCfg(nb, 256, 0, ST(stream)), (const float*)x, n, scratch);
-    else launch_pdl(sumsq_kernel<__nv_bfloat16>, LaunchCfg(nb, 256, 0, ST(stream)), (const __nv_bfloat16*)x, n, scratch);
+    if (is_fp32) launch_pdl(sumsq_kernel<float>, LaunchCfg(nb, 256, 0, ST(stream)).traffic(4.0 * n), (const float*)x, n, scratch);
+    else launch_pdl(sumsq_kernel<__nv_bfloat16>, LaunchCfg(nb, 256, 0, ST(stream)).traffic(2.0 * n), (const __nv_bfloat16*)x, n, scratch);
     launch_pdl(sum_stage2_kernel, LaunchCfg(1, 32, 0, ST(stream)), scratch, nb, nullptr, 1.f, out, accumulate);
     return CHECK_LAUNCH();
 }
@@ -623,23 +623,23 @@ extern "C" int pb_adamw(float* p, const void* g, int g_fp32, float* m, float* v,
     const float bc2 = sqrtf(1.f - powf(beta2, float(step)));
     const int nb = grid_for(n, 256, 148 * 16);
     if (g_fp32)
-        launch_pdl(adamw_kernel<float>, LaunchCfg(nb, 256, 0, ST(stream)), p, (const float*)g, m, v, (__nv_bfloat16*)p_bf16, n, lr, beta1, beta2, eps,
+        launch_pdl(adamw_kernel<float>, LaunchCfg(nb, 256, 0, ST(stream)).traffic(28.0 * n), p, (const float*)g, m, v, (__nv_bfloat16*)p_bf16, n, lr, beta1, beta2, eps,
                                                          wd, bc1, bc2, gnorm, max_norm, gscale);
     else
-        launch_pdl(adamw_kernel<__nv_bfloat16>, LaunchCfg(nb, 256, 0, ST(stream)), p, (const __nv_bfloat16*)g, m, v, (__nv_bfloat16*)p_bf16, n, lr,
+        launch_pdl(adamw_kernel<__nv_bfloat16>, LaunchCfg(nb, 256, 0, ST(stream)).traffic(28.0 * n), p, (const __nv_bfloat16*)g, m, v, (__nv_bfloat16*)p_bf16, n, lr,
                                                                  beta1, beta2, eps, wd, bc1, bc2, gnorm, max_norm, gscale);
     return CHECK_LAUNCH();
 }
 
 extern "C" int pb_cast_f32_bf16(const float* src, void* dst, long long n, void* stream) {
     if (n <= 0) return 0;
-    launch_pdl(cast_f32_to_bf16_kernel, LaunchCfg(grid_for(n, 256, 148 * 16), 256, 0, ST(stream)), src, (__nv_bfloat16*)dst, n);
+    launch_pdl(cast_f32_to_bf16_kernel, LaunchCfg(grid_for(n, 256, 148 * 16), 256, 0, ST(stream)).traffic(6.0 * n), src, (__nv_bfloat16*)dst, n);
     return CHECK_LAUNCH();
 }
 
 extern "C" int pb_add_bf16(const void* a, const void* b, void* out, long long n, void* stream) {
     if (n % 8) return -1;
-    launch_pdl(add_bf16_kernel, LaunchCfg(grid_for(n / 8, 256), 256, 0, ST(stream)), (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)out, n / 8);
+    launch_pdl(add_bf16_kernel, LaunchCfg(grid_for(n / 8, 256), 256, 0, ST(stream)).traffic(6.0 * n), (const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)out, n / 8);
     return CHECK_LAUNCH();
 }
 
@@ -683,7 +683,7 @@ extern "C" int pb_splitk_reduce(const float* ws, int slices, long long M, int N,
                                 long long ld_out, int out_fp32, void* stream) {
     if (N % 4 || ld_out % 4 || (res && ld_res % 4)) return -1;
     const unsigned grid = grid_for(M * (N / 4), 256);
-    if (out_fp32) launch_pdl(splitk_reduce_kernel<true>, LaunchCfg(grid, 256, 0, ST(stream)), ws, slices, M, N, res, ld_res, out, ld_out);
-    else launch_pdl(splitk_reduce_kernel<false>, LaunchCfg(grid, 256, 0, ST(stream)), ws, slices, M, N, res, ld_res, out, ld_out);
+    if (out_fp32) launch_pdl(splitk_reduce_kernel<true>, LaunchCfg(grid, 256, 0, ST(stream)).traffic(4.0 * slices * M * N), ws, slices, M, N, res, ld_res, out, ld_out);
+    else launch_pdl(splitk_reduce_kernel<false>, LaunchCfg(grid, 256, 0, ST(stream)).traffic(4.0 * slices * M * N), ws, slices, M, N, res, ld_res, out, ld_out);
     return CHECK_LAUNCH();
 }

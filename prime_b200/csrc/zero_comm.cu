@@ -523,7 +523,9 @@ extern "C" int pb_zero_adamw_gather(void* const* peer_params, int world, int ran
     if (sg.cta_begin[nseg] <= 0) return 0;
     const PeerTable pt = make_peers(peer_params, world, rank);
     auto launch = [&](auto kern, auto* g) {
-        const LaunchCfg cfg(sg.cta_begin[nseg], 256, 0, ST(stream));
+        double n = 0;
+        for (int i = 0; i < nseg; ++i) n += double(numel[i]);
+        const LaunchCfg cfg = LaunchCfg(sg.cta_begin[nseg], 256, 0, ST(stream)).traffic(28.0 * n);
         if (world == 1) launch_pdl(kern, cfg, pt, sg, master, g, m, v, lr, beta1, beta2, eps, wd, bc1, bc2, gnorm_sq, max_norm, hyper);
         else kern<<<cfg.c.gridDim, 256, 0, ST(stream)>>>(pt, sg, master, g, m, v, lr, beta1, beta2, eps, wd, bc1, bc2, gnorm_sq, max_norm, hyper);
     };
@@ -542,8 +544,11 @@ extern "C" int pb_grad_sumsq(const void* grads, int grad_fp32, int nseg, const l
     const SegTable sg = make_segs(nseg, full_off, full_off, numel, ctas);
     ctas = sg.cta_begin[nseg];
     if (ctas <= 0) return -1;
-    if (grad_fp32) launch_pdl(grad_sumsq_kernel<float>, LaunchCfg(ctas, 256, 0, ST(stream)), reinterpret_cast<const float*>(grads), sg, scratch, counter, out);
-    else launch_pdl(grad_sumsq_kernel<__nv_bfloat16>, LaunchCfg(ctas, 256, 0, ST(stream)), reinterpret_cast<const __nv_bfloat16*>(grads), sg, scratch, counter, out);
+    double bytes = 0;
+    for (int i = 0; i < nseg; ++i) bytes += double(numel[i]) * (grad_fp32 ? 4 : 2);
+    const LaunchCfg cfg = LaunchCfg(ctas, 256, 0, ST(stream)).traffic(bytes);
+    if (grad_fp32) launch_pdl(grad_sumsq_kernel<float>, cfg, reinterpret_cast<const float*>(grads), sg, scratch, counter, out);
+    else launch_pdl(grad_sumsq_kernel<__nv_bfloat16>, cfg, reinterpret_cast<const __nv_bfloat16*>(grads), sg, scratch, counter, out);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }
 
