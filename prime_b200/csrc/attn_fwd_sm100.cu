@@ -11,8 +11,8 @@
 //
 // One CTA = one 128-row query tile of one head, 256 threads in two warpgroups: warp 0 TMA producer, warp 1 MMA
 // issuer (owns TMEM), warps 2-3 only hold the first warpgroup together, warps 4-7 softmax (one thread per query
-// row: row max / sum are thread-local). At head size 64, where two CTAs share an SM, the first warpgroup gives
-// registers up (setmaxnreg) so that a softmax thread can hold its 128-wide score row without spilling.
+// row: row max / sum are thread-local). Two CTAs share an SM, so that one's exponentials run under the other's MMAs; the
+// first warpgroup gives registers up (setmaxnreg) so that a softmax thread can hold its 128-wide score row without spilling.
 //   S = Q K^T            -> TMEM [128 x 128] fp32
 //   P = exp2(S*c - m*c)  -> bf16 pairs in TMEM (tcgen05.st), read by the PV MMA as its A operand
 //   O  += P V            -> TMEM [128 x HD] fp32, accumulated by the MMA across KV tiles; rows are
@@ -36,20 +36,27 @@ struct AttnFwdParams {
 template <int HD>
 struct AttnFwdCfg {
     static constexpr int TILE_BYTES = 128 * HD * 2;          // one Q / K / V tile
-    static constexpr int KV_STAGES = 2;
-    // two CTAs of the HD=64 variant must fit one SM, so there is no alignment slack: the kernel
+    // Two CTAs per SM at either head size: half the SM's shared memory, tensor memory (256 columns) and registers each.
+    // HD=64: two K/V stages, and P has columns of its own, so the tensor core computes S of the next tile during the
+    // exponentials of this one. HD=128: one K/V stage, and P takes the place of S, whose row the softmax thread already
+    // holds; the next S waits for the PV MMA of this tile, and the other CTA fills the tensor core meanwhile. (With one CTA
+    // per SM and 512 columns the same overlap as HD=64 left the MMAs idle half of the time:
+    // 8 x 2048 tokens, 16 heads 281 -> 226 us; 1 x 8192, 32 / 8 heads 767 -> 709 us.)
+    static constexpr int KV_STAGES = (HD == 64) ? 2 : 1;
+    static constexpr bool P_ALIASES_S = (HD != 64);
+    // two CTAs must fit one SM, so there is no alignment slack: the kernel
     // checks that the dynamic shared window is 1024-byte aligned and reports an error otherwise
     static constexpr int SMEM_BYTES = TILE_BYTES * (1 + 2 * KV_STAGES) + 128;
-    // TMEM columns: S (fp32) 0..127, O (fp32) 128..128+HD, P (bf16 pairs, A operand of the PV MMA) next 64
-    static constexpr int T_P = 128 + HD;
-    static constexpr int TMEM_COLS = (HD == 64) ? 256 : 512;
+    // TMEM columns: S (fp32) 0..127, O (fp32) 128..128+HD, P (bf16 pairs, A operand of the PV MMA) 64 columns
+    static constexpr int T_P = P_ALIASES_S ? 0 : 128 + HD;
+    static constexpr int TMEM_COLS = 256;
 };
 
 __device__ __forceinline__ void fwd_reg_dealloc_40() { asm volatile("setmaxnreg.dec.sync.aligned.u32 40;"); }
 __device__ __forceinline__ void fwd_reg_alloc_216() { asm volatile("setmaxnreg.inc.sync.aligned.u32 216;"); }
 
 template <int HD>
-__global__ void __launch_bounds__(256, (HD == 64 ? 2 : 1))
+__global__ void __launch_bounds__(256, 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
     using Cfg = AttnFwdCfg<HD>;
     constexpr int NB = HD / 64;   // 64-column swizzle blocks per tile
@@ -61,18 +68,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
     }
     uint8_t* gen = smem_raw;
     const uint32_t sQ = base;
-    const uint32_t sK = sQ + Cfg::TILE_BYTES;                           // [2]
-    const uint32_t sV = sK + Cfg::KV_STAGES * Cfg::TILE_BYTES;           // [2]
+    const uint32_t sK = sQ + Cfg::TILE_BYTES;                           // [KV_STAGES]
+    const uint32_t sV = sK + Cfg::KV_STAGES * Cfg::TILE_BYTES;           // [KV_STAGES]
     uint64_t* bars = reinterpret_cast<uint64_t*>(gen + Cfg::TILE_BYTES * (1 + 2 * Cfg::KV_STAGES));
     const uint32_t bar_q = smem_u32(bars);
     const uint32_t bar_kfull = bar_q + 8;        // [2]
     const uint32_t bar_vfull = bar_kfull + 16;   // [2]
-    const uint32_t bar_kvempty = bar_vfull + 16; // [2]
-    const uint32_t bar_sfull = bar_kvempty + 16;
+    const uint32_t bar_kempty = bar_vfull + 16;  // [2] S = Q K^T of the tile has retired
+    const uint32_t bar_vempty = bar_kempty + 16; // [2] O += P V of the tile has retired
+    const uint32_t bar_sfull = bar_vempty + 16;
     const uint32_t bar_pfull = bar_sfull + 8;
     const uint32_t bar_ofull = bar_pfull + 8;
     const uint32_t bar_sfree = bar_ofull + 8;    // softmax warps hold S_j in registers: S TMEM may be overwritten
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -86,7 +94,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
         for (int s = 0; s < 2; ++s) {
             mbar_init(bar_kfull + 8 * s, 1);
             mbar_init(bar_vfull + 8 * s, 1);
-            mbar_init(bar_kvempty + 8 * s, 1);
+            mbar_init(bar_kempty + 8 * s, 1);
+            mbar_init(bar_vempty + 8 * s, 1);
         }
         mbar_init(bar_sfull, 1);
         mbar_init(bar_pfull, 4);
@@ -113,9 +122,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
     const int kv_hi = q_tile;                      // inclusive
     const int n_kv = kv_hi - kv_lo + 1;
 
-    // head size 64: 2 CTAs x (128 x 40 + 128 x 216) registers = the SM's 64 K
+    // 2 CTAs x (128 x 40 + 128 x 216) registers = the SM's 64 K
     if (warp < 4) {
-        if (HD == 64) fwd_reg_dealloc_40();
+        fwd_reg_dealloc_40();
         if (warp == 0) {
             // ------------------------------ TMA producer ------------------------------
             if (lane == 0) {
@@ -125,17 +134,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
             }
             bool ok = true;
             for (int j = 0; j < n_kv && ok; ++j) {
-                const int st = j & 1;
-                const uint32_t ph = (j >> 1) & 1;
-                ok = mbar_wait(bar_kvempty + 8 * st, ph ^ 1, abort_flag, p.status, PB_ERR_TIMEOUT_EMPTY);
+                const int st = j % Cfg::KV_STAGES;
+                const uint32_t ph = (j / Cfg::KV_STAGES) & 1;
+                const int kv0 = (kv_lo + j) * 128;
+                ok = mbar_wait(bar_kempty + 8 * st, ph ^ 1, abort_flag, p.status, PB_ERR_TIMEOUT_EMPTY);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 if (lane == 0) {
-                    const int kv0 = (kv_lo + j) * 128;
                     mbar_expect_tx(bar_kfull + 8 * st, Cfg::TILE_BYTES);
 #pragma unroll
                     for (int b = 0; b < NB; ++b)
                         tma_load_3d(sK + st * Cfg::TILE_BYTES + b * 16384, &tm, bar_kfull + 8 * st, 64 * b, p.H + kvh, kv0);
+                }
+                ok = mbar_wait(bar_vempty + 8 * st, ph ^ 1, abort_flag, p.status, PB_ERR_TIMEOUT_EMPTY);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                if (lane == 0) {
                     mbar_expect_tx(bar_vfull + 8 * st, Cfg::TILE_BYTES);
 #pragma unroll
                     for (int b = 0; b < NB; ++b)
@@ -156,6 +170,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
                     umma_f16_ss(tS, umma_smem_desc(sQ + off, 16, 1024), umma_smem_desc(kb + off, 16, 1024), idesc_s, k ? 1u : 0u);
                 }
                 umma_commit(bar_sfull);
+                umma_commit(bar_kempty + 8 * st);
             };
             bool ok = mbar_wait(bar_q, 0, abort_flag, p.status, PB_ERR_TIMEOUT_FULL);
             ok = __all_sync(0xffffffffu, ok);
@@ -169,9 +184,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
                 __syncwarp();
             }
             for (int j = 0; j < n_kv && ok; ++j) {
-                const int st = j & 1;
-                const uint32_t ph = (j >> 1) & 1;
-                if (j + 1 < n_kv) {
+                const int st = j % Cfg::KV_STAGES;
+                const uint32_t ph = (j / Cfg::KV_STAGES) & 1;
+                if (!Cfg::P_ALIASES_S && j + 1 < n_kv) {
                     // S_{j+1} is issued as soon as the softmax warps have pulled S_j into registers, so the
                     // tensor core computes it while they do the exponentials of tile j
                     const int st1 = (j + 1) & 1;
@@ -202,13 +217,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p) {
                         umma_f16_ts(tO, tP + k * 8, db, idesc_o, (j | k) ? 1u : 0u);   // O accumulates over all kv tiles
                     }
                     umma_commit(bar_ofull);
-                    umma_commit(bar_kvempty + 8 * st);
+                    umma_commit(bar_vempty + 8 * st);
                 }
                 __syncwarp();
+                if (Cfg::P_ALIASES_S && j + 1 < n_kv) {
+                    // the next K has been under way since S_j retired; S_{j+1} overwrites P_j, so PV_j has to be done
+                    ok = mbar_wait(bar_kfull + 8 * ((j + 1) % Cfg::KV_STAGES), ((j + 1) / Cfg::KV_STAGES) & 1, abort_flag, p.status, PB_ERR_TIMEOUT_FULL);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    ok = mbar_wait(bar_ofull, j & 1, abort_flag, p.status, PB_ERR_TIMEOUT_TMEM_FULL);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (lane == 0) issue_s((j + 1) % Cfg::KV_STAGES);
+                    __syncwarp();
+                }
             }
         }
     } else {
-        if (HD == 64) fwd_reg_alloc_216();
+        fwd_reg_alloc_216();
         // ------------------------------ softmax warps ------------------------------
         // One thread per query row. The whole 128-wide score row is pulled from TMEM in one go and
         // stays in registers; O lives in TMEM (the PV MMA accumulates into it) and is rescaled only
