@@ -63,3 +63,23 @@ def test_rope_epilogue_narrow_heads(hd):
     ref = ops.rope_((x.float() @ w.float().t()).cpu(), table.cpu(), T, H + KV, hd).cuda()
     ops.check_status()
     assert _rel(out, ref) < 1e-2
+
+
+# vocabularies at the edges of the three block widths, with and without a ragged tail, down to a row shorter than one vector
+@pytest.mark.parametrize("V", [5, 1024, 4099, 49152, 49160, 98304, 98315, 128256])
+@pytest.mark.parametrize("z_mode", [ops.Z_NONE, ops.Z_MAX, ops.Z_LSE])
+def test_cross_entropy_widths(V, z_mode):
+    torch.manual_seed(0)
+    rows, ld = 37, (V + 7) // 8 * 8
+    x = (torch.randn(rows, ld, device="cuda") * 3).bfloat16()[:, :V]
+    x[3, V - 1] = x[3, 0] = 30.0                       # a tie of the maximum: the first index counts
+    labels = torch.randint(0, V, (rows,), device="cuda")
+    labels[::5], labels[1], labels[2] = -100, 0, V - 1
+    inv = ops.count_valid(labels)
+    loss, z = torch.empty(rows, device="cuda"), torch.empty(rows, device="cuda")
+    ref, rloss, rz = x.cpu().clone(), torch.empty(rows), torch.empty(rows)
+    ops.cross_entropy_(x, labels, inv, loss, z, grad_scale=0.5, z_mode=z_mode, z_weight=1e-2)
+    ops.cross_entropy_(ref, labels.cpu(), inv.cpu(), rloss, rz, grad_scale=0.5, z_mode=z_mode, z_weight=1e-2)
+    # fp32 sums of up to 2^17 exponentials, each within a few 2^-23
+    assert torch.allclose(loss.cpu(), rloss, rtol=2e-5, atol=2e-5) and torch.allclose(z.cpu(), rz, rtol=2e-5, atol=2e-5)
+    assert _rel(x.cpu(), ref) < 4e-3                   # both sides round to bf16 (2^-9)
