@@ -21,12 +21,11 @@ struct GemmParams {
     int tiles_m, group_m;
     int tn_rot;      // tile columns are visited starting at this one (all-gather GEMM: the n-block fetched first)
     // split-K: work item w = slice * num_tiles + tile; slice s covers k-blocks [s * kb_per_split, ...) and
-    // stores its fp32 partial tile at C + s * split_stride elements (plain direct-store epilogue only)
+    // stores its fp32 partial tile in plane s of the output tensor map (staged fp32 epilogue)
     int num_items, kb_per_split;
-    long long split_stride;
     // fused epilogues of the CTA-pair kernel (GEMM_EPI_*); 0 = plain store
     int epi, epi_i0, epi_i1, epi_i2;
-    int staged;      // plain / RoPE epilogue: 1 = stage the bf16 tile in shared memory and store it with TMA
+    int staged;      // plain / RoPE epilogue: the tile is staged in shared memory and leaves by TMA: 1 = bf16, 2 = fp32, 3 = fp32 added to C
     void* aux;
     long long ldaux;
     void* aux2;
@@ -128,6 +127,7 @@ __device__ __forceinline__ void gemm_store_chunk(const GemmParams& p, const uint
     }
 }
 
+int make_tmap_f32_out(CUtensorMap* out, const void* ptr, uint64_t cols, uint64_t rows, uint64_t ld, uint64_t slices, uint64_t slice_stride);
 int make_tmap_bf16_2d(CUtensorMap* out, const void* ptr, uint64_t inner, uint64_t outer, uint64_t ld, uint32_t box_inner,
                       uint32_t box_outer);
 int sm_count();

@@ -247,6 +247,19 @@ int make_tmap_heads(CUtensorMap* out, const void* ptr, int elem_bytes, uint64_t 
     return r == CUDA_SUCCESS ? 0 : -(1000 + int(r));
 }
 
+// fp32 output [slices][rows][cols] of the staged GEMM epilogue: box of 32 columns x 128 rows (128-byte rows, swizzled)
+int make_tmap_f32_out(CUtensorMap* out, const void* ptr, uint64_t cols, uint64_t rows, uint64_t ld, uint64_t slices, uint64_t slice_stride) {
+    EncodeTiledFn enc = get_encode_fn();
+    if (!enc) return -10;
+    cuuint64_t dims[3] = {cols, rows, slices};
+    cuuint64_t strides[2] = {ld * 4, slice_stride * 4};
+    cuuint32_t box[3] = {32, 128, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : -(1000 + int(r));
+}
+
 int sm_count() {
     static int n = 0;
     if (!n) {

@@ -83,3 +83,29 @@ def test_cross_entropy_widths(V, z_mode):
     # fp32 sums of up to 2^17 exponentials, each within a few 2^-23
     assert torch.allclose(loss.cpu(), rloss, rtol=2e-5, atol=2e-5) and torch.allclose(z.cpu(), rz, rtol=2e-5, atol=2e-5)
     assert _rel(x.cpu(), ref) < 4e-3                   # both sides round to bf16 (2^-9)
+
+
+# fp32 outputs: tiles cut in both directions, a pitch wider than the row, accumulation into C, another addend (direct stores)
+@pytest.mark.parametrize("M,N,K", [(512, 256, 64), (513, 260, 520), (777, 1028, 128), (1000, 4096 + 36, 256)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_fp32_output(M, N, K, a_mn, b_mn):
+    torch.manual_seed(0)
+
+    def operand(rows, mn):
+        r8, k8 = (rows + 7) // 8 * 8, (K + 7) // 8 * 8
+        return torch.randn(K, r8, device="cuda").bfloat16()[:, :rows] if mn else torch.randn(rows, k8, device="cuda").bfloat16()[:, :K]
+    a, b = operand(M, a_mn), operand(N, b_mn)
+    ref = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    wide = torch.full((M + 1, N + 12), 7.0, device="cuda")
+    out = wide[:M, :N]
+    ops.gemm(a, b, out=out, a_mn=a_mn, b_mn=b_mn)
+    tol = 2.0 ** -22 * K ** 0.5                        # fp32 accumulation of K products
+    assert _rel(out.double(), ref) < tol
+    assert (wide[M] == 7).all() and (wide[:, N:] == 7).all()
+    ops.gemm(a, b, out=out, residual=out, a_mn=a_mn, b_mn=b_mn)
+    assert _rel(out.double(), 2 * ref) < tol
+    res = torch.randn(M, N, device="cuda")
+    ops.gemm(a, b, out=out, residual=res, a_mn=a_mn, b_mn=b_mn)
+    ops.check_status()
+    assert _rel(out.double(), ref + res.double()) < tol
+    assert (wide[M] == 7).all() and (wide[:, N:] == 7).all()
