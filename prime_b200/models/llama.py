@@ -178,9 +178,8 @@ class Attention(nn.Module):
         nn.init.trunc_normal_(self.wo.weight, mean=0.0, std=init_std)
 
     def forward(self, x2d, rope_table, seq_len, seq_start):
-        qkv = torch.cat([F_.linear(x2d, self.wq.weight), F_.linear(x2d, self.wk.weight), F_.linear(x2d, self.wv.weight)], -1)
-        qkv = F_.rope(qkv, rope_table, seq_len, self.n_heads + self.n_kv_heads, self.head_dim)
-        o = F_.attention(qkv, seq_start, self.n_heads, self.n_kv_heads, self.head_dim)
+        o = F_.self_attention(x2d, self.wq.weight, self.wk.weight, self.wv.weight, rope_table, seq_start, seq_len, self.n_heads,
+                              self.n_kv_heads, self.head_dim)
         return F_.linear(o, self.wo.weight)
 
 
@@ -192,7 +191,7 @@ class FeedForward(nn.Module):
         self.w3 = nn.Linear(dim, hidden_dim, bias=False)
 
     def forward(self, x):
-        return F_.linear(F_.swiglu(torch.cat([F_.linear(x, self.w1.weight), F_.linear(x, self.w3.weight)], -1)), self.w2.weight)
+        return F_.linear(F_.swiglu_linear(x, self.w1.weight, self.w3.weight), self.w2.weight)
 
     def init_weights(self, init_std: float):
         nn.init.trunc_normal_(self.w1.weight, mean=0.0, std=0.02)

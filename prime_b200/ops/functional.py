@@ -59,7 +59,7 @@ class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         xb, wb, rstd = ctx.saved_tensors
-        dw = torch.zeros(wb.numel(), dtype=torch.float32, device=xb.device)
+        dw = torch.empty(wb.numel(), dtype=torch.float32, device=xb.device)     # overwritten (accumulate_dw=False)
         dx = K.rmsnorm_bwd(xb, wb, rstd, _bf16(dy).contiguous(), dw, accumulate_dw=False)
         return dx, dw.to(ctx.w_dtype), None
 
@@ -143,3 +143,87 @@ def attention(qkv: torch.Tensor, seq_start: torch.Tensor, H: int, KV: int, hd: i
     if qkv.is_cuda:
         return _Attention.apply(qkv, seq_start, H, KV, hd)
     return A.attention_reference(qkv, seq_start, H, KV, hd).to(qkv.dtype)
+
+
+# ------------------------------------------------------------------------------------------ fused blocks
+def _stack_bf16(*ws: torch.Tensor) -> torch.Tensor:
+    """Weights of equal width below one another in one bf16 matrix."""
+    out = torch.empty(sum(w.shape[0] for w in ws), ws[0].shape[1], dtype=torch.bfloat16, device=ws[0].device)
+    r = 0
+    for w in ws:
+        out[r: r + w.shape[0]].copy_(w)
+        r += w.shape[0]
+    return out
+
+
+def _stacked_wgrads(ctx, dy: torch.Tensor, xb: torch.Tensor, first: int, rows) -> list[torch.Tensor | None]:
+    """One weight gradient per stacked weight, each from its columns of ``dy`` in place and into a tensor of its own."""
+    out, r = [], 0
+    for i, n in enumerate(rows):
+        dw = None
+        if ctx.needs_input_grad[first + i]:
+            dw = K.gemm(dy[:, r: r + n], xb, a_mn=True, b_mn=True, out_dtype=torch.float32).to(ctx.w_dtypes[i])
+        out.append(dw)
+        r += n
+    return out
+
+
+class _SelfAttention(torch.autograd.Function):
+    """q, k and v projections in one GEMM whose epilogue rotates q and k, then attention. As separate linear, cat, rope and
+    attention nodes a block took 14 more launches and 5 more copies of activation size."""
+
+    @staticmethod
+    def forward(ctx, x, wq, wk, wv, table, seq_start, seq_len, H, KV, hd):
+        xb, wb = _bf16(x).contiguous(), _stack_bf16(wq, wk, wv)
+        qkv = torch.empty(xb.shape[0], wb.shape[0], dtype=torch.bfloat16, device=xb.device)
+        K.gemm_rope(xb, wb, qkv, table, seq_len, H + KV, hd)
+        o, lse2 = A.attention_fwd(qkv, seq_start, H, KV, hd)
+        ctx.save_for_backward(xb, wb, qkv, o, lse2, table, seq_start)
+        ctx.meta = (seq_len, H, KV, hd)
+        ctx.w_dtypes = (wq.dtype, wk.dtype, wv.dtype)
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        xb, wb, qkv, o, lse2, table, seq_start = ctx.saved_tensors
+        seq_len, H, KV, hd = ctx.meta
+        dqkv = A.attention_bwd(qkv, o, _bf16(do).contiguous(), lse2, seq_start, H, KV, hd, rope_table=table, seq_len=seq_len)
+        dx = K.gemm(dqkv, wb, b_mn=True) if ctx.needs_input_grad[0] else None
+        return dx, *_stacked_wgrads(ctx, dqkv, xb, 1, (H * hd, KV * hd, KV * hd)), None, None, None, None, None, None
+
+
+def self_attention(x, wq, wk, wv, table, seq_start, seq_len: int, H: int, KV: int, hd: int) -> torch.Tensor:
+    """``attention(rope(x @ [wq; wk; wv].T))`` for 2-D ``x``: what ``linear``, ``rope`` and ``attention`` compute one by one."""
+    if x.is_cuda:
+        return _SelfAttention.apply(x, wq, wk, wv, table, seq_start, seq_len, H, KV, hd)
+    qkv = torch.cat([linear(x, wq), linear(x, wk), linear(x, wv)], -1)
+    return attention(rope(qkv, table, seq_len, H + KV, hd), seq_start, H, KV, hd)
+
+
+class _SwiGLULinear(torch.autograd.Function):
+    """gate and up projections in one GEMM whose epilogue takes the SwiGLU."""
+
+    @staticmethod
+    def forward(ctx, x, w1, w3):
+        xb, wb = _bf16(x).contiguous(), _stack_bf16(w1, w3)
+        h13 = torch.empty(xb.shape[0], wb.shape[0], dtype=torch.bfloat16, device=xb.device)
+        act = torch.empty(xb.shape[0], w1.shape[0], dtype=torch.bfloat16, device=xb.device)
+        K.gemm_swiglu(xb, wb, h13, act)
+        ctx.save_for_backward(xb, wb, h13)
+        ctx.w_dtypes = (w1.dtype, w3.dtype)
+        return act
+
+    @staticmethod
+    def backward(ctx, d):
+        xb, wb, h13 = ctx.saved_tensors
+        dh13 = K.swiglu_bwd(h13, _bf16(d).contiguous())
+        dx = K.gemm(dh13, wb, b_mn=True) if ctx.needs_input_grad[0] else None
+        F_ = wb.shape[0] // 2
+        return dx, *_stacked_wgrads(ctx, dh13, xb, 1, (F_, F_))
+
+
+def swiglu_linear(x, w1, w3) -> torch.Tensor:
+    """``swiglu(x @ [w1; w3].T)`` for 2-D ``x``."""
+    if x.is_cuda:
+        return _SwiGLULinear.apply(x, w1, w3)
+    return swiglu(torch.cat([linear(x, w1), linear(x, w3)], -1))

@@ -7,6 +7,8 @@ use and what the GPU numerics tests compare against.
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from .. import native
@@ -120,9 +122,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, resi
     return out
 
 
-_N_PAIRS: dict = {}
-
-
+@functools.lru_cache(maxsize=1024)
 def _splitk_slices(M: int, N: int, K: int, device) -> int:
     """K slices for the CTA-pair GEMM: 1 unless the product has too few 256x256 tiles to fill the GPU and a long
     K. Minimises waves x k-blocks per slice (0.42 us per k-block) plus the fp32 partials' round trip and the reduce
@@ -131,9 +131,7 @@ def _splitk_slices(M: int, N: int, K: int, device) -> int:
     which its pipeline never fills."""
     if N % 4 or K < 2048 or M < 256 or N < 256:
         return 1
-    pairs = _N_PAIRS.get(device)
-    if pairs is None:
-        pairs = _N_PAIRS[device] = torch.cuda.get_device_properties(device).multi_processor_count // 2
+    pairs = torch.cuda.get_device_properties(device).multi_processor_count // 2
     tiles = ((M + 255) // 256) * ((N + 255) // 256)
     if tiles * 4 > pairs * 3:
         return 1

@@ -109,3 +109,28 @@ def test_fp32_output(M, N, K, a_mn, b_mn):
     ops.check_status()
     assert _rel(out.double(), ref + res.double()) < tol
     assert (wide[M] == 7).all() and (wide[:, N:] == 7).all()
+
+
+@pytest.mark.parametrize("M,H,KV,hd,Fd", [(96, 4, 2, 64, 512), (700, 4, 4, 32, 704), (1030, 2, 1, 128, 520)])
+def test_fused_projections_match_the_separate_ops(M, H, KV, hd, Fd):
+    from prime_b200.ops import functional as F_
+    torch.manual_seed(0)
+    D = 256
+    x0 = torch.randn(M, D, device="cuda").bfloat16()
+    ws = [(torch.randn(n, D, device="cuda") * D ** -0.5).requires_grad_() for n in (H * hd, KV * hd, KV * hd, Fd, Fd)]
+    ws[2].requires_grad_(False)                        # a frozen weight gets no gradient
+    table, ss = ops.rope_table(M, hd, 10000.0, "cuda"), A.seq_start_from_batch(1, M, "cuda")
+    go, ga = torch.randn(M, H * hd, device="cuda").bfloat16(), torch.randn(M, Fd, device="cuda").bfloat16()
+
+    def grads(attn, act, x):
+        for keep in (True, False):                     # a second backward finds the saved tensors as they were
+            g = torch.autograd.grad([attn, act], [x, ws[0], ws[1], ws[3], ws[4]], [go, ga], retain_graph=keep)
+        return [attn.detach(), act.detach(), *g]
+    x = x0.clone().requires_grad_()
+    got = grads(F_.self_attention(x, *ws[:3], table, ss, M, H, KV, hd), F_.swiglu_linear(x, *ws[3:]), x)
+    x = x0.clone().requires_grad_()
+    qkv = F_.rope(torch.cat([F_.linear(x, w) for w in ws[:3]], -1), table, M, H + KV, hd)
+    want = grads(F_.attention(qkv, ss, H, KV, hd), F_.swiglu(torch.cat([F_.linear(x, w) for w in ws[3:]], -1)), x)
+    ops.check_status()
+    for g, w in zip(got, want):
+        assert g.dtype == w.dtype and g.shape == w.shape and _rel(g, w) < 2e-2      # a few more bf16 roundings on the separate side
