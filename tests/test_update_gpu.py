@@ -114,13 +114,15 @@ def test_graphed_steps_match_steps_launched_one_by_one(monkeypatch, hd, micro, p
             ss += torch.where(torch.arange(B * T, device="cuda") % T >= cut, cut, 0).int()
         res = [e.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3 * (i + 1), micro_bs=micro, seq_start=ss) for e in (a, b)]
         replayed += bool(a._graphs)
-        # the kernels are the same; only the embedding gradient's atomic adds may come in another order (bf16: 2^-8 each)
+        # the kernels are the same; only the embedding gradient's atomic adds may come in another order (bf16: 2^-8 each).
+        # Adam turns such a difference of a tiny gradient into one of the update's full size, so every step starts from one state
         assert res[0] == pytest.approx(res[1], rel=2e-3)
+        assert ((a.master - b.master).norm() / b.master.norm()).item() < (1e-4 if fp32 else 5e-3)
+        assert ((a.exp_avg - b.exp_avg).norm() / b.exp_avg.norm()).item() < (1e-3 if fp32 else 3e-2)
+        for name in ("master", "exp_avg", "exp_avg_sq", "params"):
+            getattr(b, name).copy_(getattr(a, name))
     assert replayed >= 5 and not b._graphs
     assert a.opt_step == b.opt_step == 8
-    tol = 1e-4 if fp32 else 5e-3
-    assert ((a.master - b.master).norm() / b.master.norm()).item() < tol
-    assert ((a.exp_avg - b.exp_avg).norm() / b.exp_avg.norm()).item() < (1e-3 if fp32 else 3e-2)
     loss, norm = a.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3, micro_bs=micro, seq_start=ss, sync_loss=False)
     keep = loss.item()
     a.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3, micro_bs=micro, seq_start=ss, sync_loss=False)
