@@ -12,6 +12,7 @@
 //   AdamW        src/zeroband/optimizers.py:25-30 (torch.optim.AdamW semantics)
 #include "common.cuh"
 #include "rmsnorm_bwd.cuh"
+#include <algorithm>
 
 namespace pb {
 
@@ -559,14 +560,15 @@ extern "C" int pb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd
     return CHECK_LAUNCH();
 }
 
-// number of CTAs (= rows of the fp32 partial buffer [ctas, N]) the backward uses
+// number of CTAs (= rows of the fp32 partial buffer [ctas, N]) the backward uses at most
 extern "C" int pb_rmsnorm_bwd_ctas() { return 148 * 2; }
 
 extern "C" int pb_rmsnorm_bwd(const void* x, const void* w, const float* rstd, const void* dy, const void* dres,
                               void* dx, float* dw_partial, void* dw, int dw_fp32, int dw_accumulate, int M, int N,
                               void* stream) {
     if (N % 256 || N > 4096) return -1;
-    const int ctas = pb_rmsnorm_bwd_ctas();
+    const int rows_per_cta = N <= 1024 ? 8 : N <= 2048 ? 4 : 2;      // of one iteration; a CTA without rows would only add a zero partial
+    const int ctas = std::max(1, std::min(pb_rmsnorm_bwd_ctas(), (M + rows_per_cta - 1) / rows_per_cta));
     auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w; auto DY = (const __nv_bfloat16*)dy;
     auto DR = (const __nv_bfloat16*)dres; auto DX = (__nv_bfloat16*)dx;
     // rows wider than 1024 are shared by two or four warps (at most four 256-column chunks per warp)
@@ -577,7 +579,7 @@ extern "C" int pb_rmsnorm_bwd(const void* x, const void* w, const float* rstd, c
     }
 #undef RB
     if (cudaGetLastError() != cudaSuccess) return -30;
-    launch_pdl(colsum_partials_kernel, LaunchCfg((N + 31) / 32, 256, 0, ST(stream)), dw_partial, dw, ctas, N, dw_fp32, dw_accumulate);
+    launch_pdl(colsum_partials_kernel, LaunchCfg((N + 31) / 32, 32 * COLSUM_GROUPS, 0, ST(stream)), dw_partial, dw, ctas, N, dw_fp32, dw_accumulate);
     return CHECK_LAUNCH();
 }
 

@@ -134,3 +134,19 @@ def test_fused_projections_match_the_separate_ops(M, H, KV, hd, Fd):
     ops.check_status()
     for g, w in zip(got, want):
         assert g.dtype == w.dtype and g.shape == w.shape and _rel(g, w) < 2e-2      # a few more bf16 roundings on the separate side
+
+
+# fewer rows than one CTA iteration, one more than it, and around the number of CTAs, for one, two and four warps per row
+@pytest.mark.parametrize("M", [1, 7, 9, 593, 2371])
+@pytest.mark.parametrize("N", [256, 1024, 1536, 4096])
+def test_rmsnorm_bwd_row_counts(M, N):
+    torch.manual_seed(0)
+    x, dy = (torch.randn(M, N, device="cuda").bfloat16() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(N, device="cuda")).bfloat16()
+    _, rstd = ops.rmsnorm_fwd(x, w, 1e-5)
+    dw, rdw = torch.full((N,), 3.0, device="cuda"), torch.full((N,), 3.0)
+    for acc in (False, True):
+        dx = ops.rmsnorm_bwd(x, w, rstd, dy, dw, accumulate_dw=acc)
+        rdx = ops.rmsnorm_bwd(x.cpu(), w.cpu(), rstd.cpu(), dy.cpu(), rdw, accumulate_dw=acc)
+    assert _rel(dx.cpu(), rdx) < 4e-3                  # bf16 results of the same fp32 math
+    assert _rel(dw.cpu(), rdw) < 1e-5                  # fp32 sums of M terms in two orders
