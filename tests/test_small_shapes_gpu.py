@@ -86,7 +86,7 @@ def test_cross_entropy_widths(V, z_mode):
 
 
 # fp32 outputs: tiles cut in both directions, a pitch wider than the row, accumulation into C, another addend (direct stores)
-@pytest.mark.parametrize("M,N,K", [(512, 256, 64), (513, 260, 520), (777, 1028, 128), (1000, 4096 + 36, 256)])
+@pytest.mark.parametrize("M,N,K", [(512, 256, 64), (513, 260, 520), (600, 1027, 64), (777, 1028, 128), (1000, 4096 + 36, 256)])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
 def test_fp32_output(M, N, K, a_mn, b_mn):
     torch.manual_seed(0)
@@ -96,7 +96,7 @@ def test_fp32_output(M, N, K, a_mn, b_mn):
         return torch.randn(K, r8, device="cuda").bfloat16()[:, :rows] if mn else torch.randn(rows, k8, device="cuda").bfloat16()[:, :K]
     a, b = operand(M, a_mn), operand(N, b_mn)
     ref = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
-    wide = torch.full((M + 1, N + 12), 7.0, device="cuda")
+    wide = torch.full((M + 1, (N + 3) // 4 * 4 + 12), 7.0, device="cuda")
     out = wide[:M, :N]
     ops.gemm(a, b, out=out, a_mn=a_mn, b_mn=b_mn)
     tol = 2.0 ** -22 * K ** 0.5                        # fp32 accumulation of K products
@@ -104,7 +104,7 @@ def test_fp32_output(M, N, K, a_mn, b_mn):
     assert (wide[M] == 7).all() and (wide[:, N:] == 7).all()
     ops.gemm(a, b, out=out, residual=out, a_mn=a_mn, b_mn=b_mn)
     assert _rel(out.double(), 2 * ref) < tol
-    res = torch.randn(M, N, device="cuda")
+    res = torch.randn(M, wide.shape[1], device="cuda")[:, :N]
     ops.gemm(a, b, out=out, residual=res, a_mn=a_mn, b_mn=b_mn)
     ops.check_status()
     assert _rel(out.double(), ref + res.double()) < tol
