@@ -128,9 +128,14 @@ def ptr(t: torch.Tensor | None):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
+def raw_stream(device_index: int | None = None) -> int:
+    """Handle of the current stream of a device (the current one by default), without the ``torch.cuda.Stream`` object around it,
+    whose making takes longer than the rest of a launch's arguments."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device_index is None else device_index)
+
+
 def stream_ptr(stream: torch.cuda.Stream | None = None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    return C.c_void_p(raw_stream() if stream is None else stream.cuda_stream)
 
 
 # kernels launched per successful native call (1 unless listed); used for launch accounting

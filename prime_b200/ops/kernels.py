@@ -42,7 +42,7 @@ def check_status(device: torch.device | None = None) -> None:
 def _scratch_buf(device, key: str, numel: int, dtype=torch.float32) -> torch.Tensor:
     """Scratch of one use on the current stream: kernels of other streams (weight gradients beside the backward, another
     thread's model) run at the same time and have their own. At most 64 are kept, the oldest go back to the allocator."""
-    k = (device.index or 0, torch.cuda.current_stream(device).cuda_stream, key)
+    k = (device.index or 0, native.raw_stream(device.index), key)
     t = _scratch.get(k)
     if t is None or t.numel() < numel or t.dtype != dtype:
         for old in list(_scratch)[:max(0, len(_scratch) - 63)]:
