@@ -148,12 +148,7 @@ def attention(qkv: torch.Tensor, seq_start: torch.Tensor, H: int, KV: int, hd: i
 # ------------------------------------------------------------------------------------------ fused blocks
 def _stack_bf16(*ws: torch.Tensor) -> torch.Tensor:
     """Weights of equal width below one another in one bf16 matrix."""
-    out = torch.empty(sum(w.shape[0] for w in ws), ws[0].shape[1], dtype=torch.bfloat16, device=ws[0].device)
-    r = 0
-    for w in ws:
-        out[r: r + w.shape[0]].copy_(w)
-        r += w.shape[0]
-    return out
+    return torch.cat(ws, out=torch.empty(sum(w.shape[0] for w in ws), ws[0].shape[1], dtype=torch.bfloat16, device=ws[0].device))
 
 
 def _stacked_wgrads(ctx, dy: torch.Tensor, xb: torch.Tensor, first: int, rows) -> list[torch.Tensor | None]:
