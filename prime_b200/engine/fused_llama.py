@@ -172,7 +172,9 @@ class FusedLlama:
         self.master = torch.zeros(n_shard, dtype=torch.float32, device=dev)
         self.exp_avg = torch.zeros(n_shard, dtype=torch.float32, device=dev)
         self.exp_avg_sq = torch.zeros(n_shard, dtype=torch.float32, device=dev)
-        self._grad_shard = None        # fp32 reduced gradients; allocated on first use (see grad_shard)
+        # fp32 reduced gradients. A run that reduces has them from the start: the first use is inside the reduce, which the
+        # communication stream runs behind an event that an allocation (and its fill) at that point would come after.
+        self._grad_shard = None if self._solo else torch.zeros(n_shard, dtype=torch.float32, device=dev)
         self._peer_params = self.comm.peer_ptrs(self.params) if not self.reshard else None
         self._peer_grads = self.comm.peer_ptrs(self.grads)
         self._segs = [_SegArrays(lay.group_segments(self.rank, g)) for g in range(len(lay.groups))]
@@ -732,8 +734,8 @@ class FusedLlama:
     @property
     def grad_shard(self) -> torch.Tensor:
         """This rank's reduced fp32 gradients, one value per owned parameter element. A run without peers that updates with the
-        AdamW kernel never asks for it (4 bytes per parameter that stay free); there it is filled from the gradient buffer on
-        each access."""
+        AdamW kernel never asks for it (4 bytes per parameter that stay free); there it is allocated by the first access and
+        filled from the gradient buffer on each one. ``set_shard_optimizer`` is such an access, before any reduce."""
         if self._grad_shard is None:
             self._grad_shard = torch.zeros(self.layout.shard_numel[self.rank], dtype=torch.float32, device=self.device)
         if self._direct_update:

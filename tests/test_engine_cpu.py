@@ -218,3 +218,10 @@ def test_soap_runs_as_a_shard_optimizer_of_the_fused_engine(tmp_path):
     assert eng2.opt_step == eng.opt_step
     q0 = eng2._shard_params[0]
     assert backend2.shard_optimizer.state[q0]["step"] == 5
+
+
+def test_a_run_that_reduces_has_its_gradient_shard_from_the_start():
+    """Allocated later, its zero fill would be queued behind the event that lets the communication stream start the reduce."""
+    _, eng = _mk(_tiny())
+    assert not eng._solo and eng._grad_shard is not None
+    assert eng._grad_shard.numel() == eng.layout.shard_numel[0] and not eng._grad_shard.any()

@@ -155,3 +155,23 @@ def test_scratch_is_one_per_stream():
     ws = [t.data_ptr() for k, t in K._scratch.items() if k[2] == "splitk"]
     assert len(ws) >= 2 and len(set(ws)) == len(ws)
     assert K.take_scratch(side) and not any(k[1] == side.cuda_stream for k in K._scratch)
+
+
+@pytest.mark.parametrize("overlap", [True, False])
+def test_first_reduced_step_keeps_every_gradient(overlap):
+    """The reduce path with one rank: the shard holds the gradient buffer after the first step, whichever stream reduced it."""
+    from prime_b200.engine.fused_llama import FusedLlama, LocalComm
+    from prime_b200.models.llama import ModelArgs
+
+    class OneRank(LocalComm):       # not the plain LocalComm, whose runs update from their own gradients
+        pass
+    eng = FusedLlama(ModelArgs(dim=256, n_layers=2, n_heads=4, ffn_hidden=512, vocab_size=1024, max_seq_len=256, init_mode="normal"),
+                     device="cuda", comm=OneRank(), ce_chunk_tokens=512)
+    eng.overlap_reduce = overlap
+    eng.init_weights(seed=3)
+    ids = torch.randint(0, 1024, (2, 129), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    _, norm = eng.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3)
+    for name, g in eng.g.items():
+        assert torch.equal(eng.shard_view(eng.grad_shard, name), g.float()), name
+    # the norm is the root of the shard's sum of squares: fp32 sums, far below 1e-4
+    assert eng.grad_shard.double().norm().item() == pytest.approx(norm, rel=1e-4)
