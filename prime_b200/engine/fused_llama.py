@@ -739,6 +739,7 @@ class FusedLlama:
         if self._grad_shard is None:
             self._grad_shard = torch.zeros(self.layout.shard_numel[self.rank], dtype=torch.float32, device=self.device)
         if self._direct_update:
+            self._wait_all_wgrads()
             for sa in self._segs_step:
                 for f, s, n in zip(sa.full[:sa.n], sa.shard[:sa.n], sa.numel[:sa.n]):
                     self._grad_shard[s: s + n].copy_(self.grads[f: f + n])
@@ -754,6 +755,7 @@ class FusedLlama:
         that buffer. Against the reduce into an fp32 shard (14 to 20 launches under the backward) this moves 8 bytes per
         bf16-gradient parameter less and takes no bandwidth from the backward."""
         lib = native.cuda()
+        self._wait_all_wgrads()        # the last weight gradients (block 0) may still be under way on their own stream
         fp32 = self.grad_dtype == torch.float32
         norm_out = self._norm_global if len(self._segs_step) == 1 else self._norm_parts
         for i, sa in enumerate(self._segs_step):

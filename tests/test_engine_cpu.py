@@ -225,3 +225,30 @@ def test_a_run_that_reduces_has_its_gradient_shard_from_the_start():
     _, eng = _mk(_tiny())
     assert not eng._solo and eng._grad_shard is not None
     assert eng._grad_shard.numel() == eng.layout.shard_numel[0] and not eng._grad_shard.any()
+
+
+def test_update_without_peers_waits_for_the_weight_gradient_stream(monkeypatch):
+    """The host's order of calls, on stand-ins for the streams and the kernel library: the update and a reader of the gradient shard
+    join the stream of the weight gradients before they touch a gradient."""
+    from prime_b200 import native
+    from prime_b200.engine import fused_llama
+    _, eng = _mk(_tiny())
+    order = []
+
+    class Stream:
+        def wait_stream(self, s):
+            order.append("join" if s is eng.wgrad_stream else "other")
+
+    class Lib:
+        def __getattr__(self, name):
+            return lambda *a: order.append(name) or 0
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: Stream())
+    monkeypatch.setattr(native, "cuda", Lib)
+    monkeypatch.setattr(fused_llama, "stream_ptr", lambda *a: None)
+    eng._solo, eng.wgrad_stream = True, object()
+    eng._readers = {1: "event"}
+    eng._update_from_own_grads(1e-3, (0.9, 0.95), 1e-8, 0.1, 1.0)
+    assert order == ["join", "pb_grad_sumsq", "pb_zero_adamw_gather"]
+    order.clear()
+    eng._readers = {1: "event"}
+    assert eng.grad_shard is not None and order == ["join"]

@@ -15,6 +15,10 @@ pytestmark = pytest.mark.gpu
 SEGS = [[(0, 0, 4096)], [(0, 0, 70001)], [(1, 1, 5000), (6008, 5008, 3)], [(64, 0, 1 << 20), ((1 << 20) + 128, 1 << 20, 999)]]
 
 
+def _rel(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm()).item()
+
+
 def _arrays(segs):
     arr = C.c_longlong * len(segs)
     return arr(*[s[0] for s in segs]), arr(*[s[1] for s in segs]), arr(*[s[2] for s in segs])
@@ -175,3 +179,31 @@ def test_first_reduced_step_keeps_every_gradient(overlap):
         assert torch.equal(eng.shard_view(eng.grad_shard, name), g.float()), name
     # the norm is the root of the shard's sum of squares: fp32 sums, far below 1e-4
     assert eng.grad_shard.double().norm().item() == pytest.approx(norm, rel=1e-4)
+
+
+def test_update_sees_the_gradients_of_the_weight_gradient_stream(monkeypatch):
+    from prime_b200.engine.fused_llama import FusedLlama
+    from prime_b200.models.llama import ModelArgs
+    args = ModelArgs(dim=1024, n_layers=2, n_heads=16, ffn_hidden=4096, vocab_size=1024, max_seq_len=512, init_mode="normal")
+    runs = []
+    for on in ("0", "1"):
+        monkeypatch.setenv("PRIME_B200_WGRAD_STREAM", on)
+        eng = FusedLlama(args, device="cuda", grad_dtype=torch.float32)
+        assert (eng.wgrad_stream is not None) == (on == "1")
+        eng.init_weights(seed=3)
+        ids = torch.randint(0, 1024, (16, 513), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+        loss, norm = eng.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3)
+        # first moment of the first step: 0.1 * clipped gradient, in fp32 products
+        want = 0.1 * min(1.0, 1.0 / (norm + 1e-6)) * eng.grads
+        for p in eng.layout.params:
+            s = slice(p.offset, p.offset + p.numel)
+            assert _rel(eng.shard_view(eng.exp_avg, p.name).flatten(), want[s]) < 1e-5, p.name
+        assert eng.grad_shard.double().norm().item() == pytest.approx(norm, rel=1e-4)
+        runs.append((loss, norm, eng))
+    (l0, n0, a), (l1, n1, b) = runs
+    # The kernels are the same. dQ is summed by atomic adds, whose order moves its rounding to bf16 by one unit (2^-8) at most: that
+    # reaches every gradient below the upper block's attention, once per block
+    assert l0 == pytest.approx(l1, rel=1e-6) and n0 == pytest.approx(n1, rel=2 * 2.0 ** -8)
+    for name, g in a.g.items():
+        assert _rel(b.g[name], g) < 2 * 2.0 ** -8, name
+    K.check_status()
