@@ -795,7 +795,11 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
 
 extern "C" int pb_splitk_reduce(const float* ws, int slices, long long M, int N, const void* res, long long ld_res, void* out,
                                 long long ld_out, int out_fp32, void* stream) {
-    if (N % 4 || ld_out % 4 || (res && ld_res % 4)) return -1;
+    // whole vectors of four elements: 16 bytes of fp32, 8 of bf16
+    const uintptr_t vec = out_fp32 ? 16 : 8;
+    if (N % 4 || ld_out % 4 || (res && ld_res % 4) || (reinterpret_cast<uintptr_t>(ws) % 16) || (reinterpret_cast<uintptr_t>(out) % vec) ||
+        (reinterpret_cast<uintptr_t>(res) % vec))
+        return -1;
     const unsigned grid = grid_for(M * (N / 4), 256);
     if (out_fp32) launch_pdl(splitk_reduce_kernel<true>, LaunchCfg(grid, 256, 0, ST(stream)).traffic(4.0 * slices * M * N), ws, slices, M, N, res, ld_res, out, ld_out);
     else launch_pdl(splitk_reduce_kernel<false>, LaunchCfg(grid, 256, 0, ST(stream)).traffic(4.0 * slices * M * N), ws, slices, M, N, res, ld_res, out, ld_out);

@@ -91,7 +91,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, resi
         assert residual.dtype == out.dtype and residual.shape == out.shape and residual.stride(-1) == 1
     ldr = residual.stride(0) if residual is not None else 0
     # bn: 0 = choose; 128 / 256 = single-CTA tile width; 512 = the CTA-pair (cta_group::2) 256x256 kernel
-    slices = _splitk_slices(M, N, K, a.device) if bn == 0 and _GEMM_PAIR else 1
+    slices = _splitk_slices(M, N, K, a.device) if bn == 0 and _GEMM_PAIR and _splitk_fits(out, residual) else 1
     use_pair = bn == 512 or slices > 1 or (bn == 0 and _GEMM_PAIR and M >= 512 and N >= 256)
     if use_pair:
         if slices > 1:
@@ -120,6 +120,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, resi
         int(out.dtype == torch.float32), bn if bn in (128, 256) else 0, max_ctas, ptr(status_word(a.device)), stream_ptr())
     check(rc, f"pb_gemm_bf16(M={M},N={N},K={K},a_mn={a_mn},b_mn={b_mn})")
     return out
+
+
+def _splitk_fits(out: torch.Tensor, residual: torch.Tensor | None) -> bool:
+    """The reduce of the split-K partials moves vectors of four elements. Outputs and addends that these do not fit go to the other
+    kernels, which say what they think of them before anything is launched."""
+    return all(t is None or (t.stride(0) % 4 == 0 and t.data_ptr() % (4 * t.element_size()) == 0) for t in (out, residual))
 
 
 @functools.lru_cache(maxsize=1024)

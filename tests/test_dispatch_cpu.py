@@ -1,0 +1,45 @@
+"""Which route a call takes, and what the C entries refuse, as far as that needs no GPU."""
+import ctypes as C
+
+import pytest
+import torch
+
+from prime_b200 import native
+from prime_b200.ops import kernels as K
+
+
+def _lib():
+    try:
+        return native.cuda()
+    except native.NativeError:
+        pytest.skip("CUDA library not built")
+
+
+# a made-up address must not reach a device, even if the check that this tests is lost
+no_device = pytest.mark.skipif(torch.cuda.is_available(), reason="the addresses are made up")
+
+
+@no_device
+@pytest.mark.parametrize("fp32", [True, False])
+def test_splitk_reduce_refuses_what_its_vectors_do_not_fit(fp32):
+    """Outputs and addends off the 16 (fp32) or 8 (bf16) bytes of four elements: refused before any launch (the addresses are made up)."""
+    lib, size, base = _lib(), 4 if fp32 else 2, 1 << 40
+
+    def call(ws=base, res=0, out=base, ld_out=1028, ld_res=1028, N=1024):
+        return lib.pb_splitk_reduce(C.c_void_p(ws), 2, 256, N, C.c_void_p(res or None), ld_res, C.c_void_p(out), ld_out, int(fp32), None)
+    for k in (1, 2, 3):
+        assert call(out=base + k * size) == -1
+        assert call(res=base + k * size) == -1
+        assert call(ws=base + 4 * k) == -1
+        assert call(ld_out=1028 + k) == -1
+        assert call(res=base, ld_res=1028 + k) == -1
+        assert call(N=1024 + k) == -1
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_splitk_is_chosen_for_whole_vectors_only(dtype):
+    wide = torch.zeros(256, 1032, dtype=dtype)
+    good = wide[:, 4:1028]
+    assert K._splitk_fits(good, None) and K._splitk_fits(good, good)
+    for bad in (wide[:, 1:1025], wide[:, 2:1026], torch.zeros(256, 1030, dtype=dtype)[:, :1024]):
+        assert not K._splitk_fits(bad, None) and not K._splitk_fits(good, bad)

@@ -150,3 +150,18 @@ def test_rmsnorm_bwd_row_counts(M, N):
         rdx = ops.rmsnorm_bwd(x.cpu(), w.cpu(), rstd.cpu(), dy.cpu(), rdw, accumulate_dw=acc)
     assert _rel(dx.cpu(), rdx) < 4e-3                  # bf16 results of the same fp32 math
     assert _rel(dw.cpu(), rdw) < 1e-5                  # fp32 sums of M terms in two orders
+
+
+# a product that is split over K, into and with a matrix that starts inside a 16-byte unit: refused like by the other kernels
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_split_k_into_an_unaligned_output_is_refused(dt):
+    from prime_b200.native import NativeError
+    a = torch.randn(2304, 256, device="cuda").bfloat16()
+    wide = torch.full((256, 1032), 7.0, device="cuda", dtype=dt)
+    b = torch.randn(2304, 1024, device="cuda").bfloat16()
+    assert ops._splitk_slices(256, 1024, 2304, a.device) > 1
+    with pytest.raises(NativeError):
+        ops.gemm(a, b, out=wide[:, 1:1025], a_mn=True, b_mn=True)
+    with pytest.raises(NativeError):
+        ops.gemm(a, b, out=wide[:, :1024], residual=wide[:, 1:1025], a_mn=True, b_mn=True)
+    assert (wide == 7).all()
