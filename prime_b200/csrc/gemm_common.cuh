@@ -26,6 +26,7 @@ struct GemmParams {
     // fused epilogues of the CTA-pair kernel (GEMM_EPI_*); 0 = plain store
     int epi, epi_i0, epi_i1, epi_i2;
     int staged;      // plain / RoPE epilogue: the tile is staged in shared memory and leaves by TMA: 1 = bf16, 2 = fp32, 3 = fp32 added to C
+    int n_tma;       // bf16 columns that leave by TMA: N cut to whole 16-byte units; the threads store the rest of a row themselves
     void* aux;
     long long ldaux;
     void* aux2;

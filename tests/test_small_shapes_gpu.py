@@ -165,3 +165,37 @@ def test_split_k_into_an_unaligned_output_is_refused(dt):
     with pytest.raises(NativeError):
         ops.gemm(a, b, out=wide[:, :1024], residual=wide[:, 1:1025], a_mn=True, b_mn=True)
     assert (wide == 7).all()
+
+
+# bf16 rows that end inside a 16-byte unit, in a wider matrix: what lies behind them stays (plain, added and rotated outputs)
+@pytest.mark.parametrize("M,N,K", [(512, 257, 64), (513, 263, 520), (700, 319, 64), (600, 1027, 128), (1000, 4092, 256)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_bf16_output_in_a_wider_matrix(M, N, K, a_mn, b_mn):
+    torch.manual_seed(0)
+
+    def operand(rows, mn):
+        r8, k8 = (rows + 7) // 8 * 8, (K + 7) // 8 * 8
+        return torch.randn(K, r8, device="cuda").bfloat16()[:, :rows] if mn else torch.randn(rows, k8, device="cuda").bfloat16()[:, :K]
+    a, b = operand(M, a_mn), operand(N, b_mn)
+    ref = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    wide = torch.full((M + 1, (N + 7) // 8 * 8 + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+    out = wide[:M, :N]
+    res = torch.randn(M, wide.shape[1], device="cuda").bfloat16()[:, :N]
+    for r in (None, res):
+        ops.gemm(a, b, out=out, residual=r, a_mn=a_mn, b_mn=b_mn)
+        want = ref if r is None else ref + r.double()
+        assert _rel(out, want) < 3e-3                  # one rounding to bf16 (2^-9)
+        assert _rel(out[:, N - 8:], want[:, N - 8:]) < 4e-3
+        assert (wide[M] == 7).all() and (wide[:, N:] == 7).all()
+    before = out.double()
+    ops.gemm(a, b, out=out, residual=out, a_mn=a_mn, b_mn=b_mn)
+    ops.check_status()
+    assert _rel(out, ref + before) < 3e-3
+    assert (wide[M] == 7).all() and (wide[:, N:] == 7).all()
+    if not a_mn and not b_mn:
+        table, hd = ops.rope_table(M, 64, 10000.0, "cuda"), 64
+        ops.gemm_rope(a, b, out, table, M, 4, hd)
+        want = ops.rope_(ref.float().cpu(), table.cpu(), M, 4, hd).cuda()
+        ops.check_status()
+        assert _rel(out, want) < 4e-3
+        assert (wide[M] == 7).all() and (wide[:, N:] == 7).all()
