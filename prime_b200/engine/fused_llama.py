@@ -876,7 +876,7 @@ class FusedLlama:
             sl = slice(mb * micro_bs, (mb + 1) * micro_bs)
             ss = None
             if seq_start is not None:
-                ss = seq_start[mb * micro_bs * T: (mb + 1) * micro_bs * T]
+                ss = seq_start[mb * micro_bs * T: (mb + 1) * micro_bs * T].contiguous()       # the kernels take dense row maps
                 if mb:
                     ss = ss - mb * micro_bs * T
             self.forward_backward(tokens[sl], labels[sl], seq_start=ss, loss_scale=1.0 / n_micro, last_microbatch=(mb == n_micro - 1),

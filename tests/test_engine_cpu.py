@@ -252,3 +252,19 @@ def test_update_without_peers_waits_for_the_weight_gradient_stream(monkeypatch):
     order.clear()
     eng._readers = {1: "event"}
     assert eng.grad_shard is not None and order == ["join"]
+
+
+@pytest.mark.parametrize("micro", [1, 2, 4])
+def test_row_maps_reach_the_kernels_dense(monkeypatch, micro):
+    """Every second element of a longer tensor, or one value for all rows: a micro-batch gets its own dense part, the first one too."""
+    _, eng = _mk(_tiny())
+    B, T = 4, 16
+    starts = torch.arange(B).repeat_interleave(T).int() * T
+    tokens = torch.zeros(B, T, dtype=torch.int64)
+    for given in (torch.stack([starts, starts + 1], 1)[:, 0], torch.zeros(1, dtype=torch.int32).expand(B * T), starts):
+        seen = []
+        monkeypatch.setattr(eng, "forward_backward", lambda *a, seq_start, **k: seen.append(seq_start))
+        eng._accumulate_micro_batches(tokens, tokens, given, micro)
+        assert len(seen) == B // micro and all(s.is_contiguous() and s.dtype == torch.int32 for s in seen)
+        for mb, s in enumerate(seen):
+            assert torch.equal(s, given[mb * micro * T: (mb + 1) * micro * T] - mb * micro * T)
