@@ -689,7 +689,9 @@ extern "C" int pb_attn_bwd(const void* qkv, const void* o, const void* dout, con
     using namespace pb;
     if (HD <= 0 || HD > 128 || HD % 8) return -1;
     if (H % KV) return -1;
-    if ((qkv_stride % 8) || (o_stride % 8) || (do_stride % 8) || (dqkv_stride % 8)) return -2;
+    if ((qkv_stride % 8) || (o_stride % 8) || (do_stride % 8) || (dqkv_stride % 8) ||
+        ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dqkv)) & 15))
+        return -2;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     CUtensorMap tq, tdo, tdq;
     int rc = make_tmap_heads(&tq, qkv, 2, HD, uint64_t(H + 2 * KV), M, qkv_stride, 64, 128);

@@ -70,6 +70,22 @@ def _kernel_head(hd: int) -> bool:
     return hd <= 128 and hd % 8 == 0
 
 
+def _rows_fit(t: torch.Tensor) -> bool:
+    """bf16 rows of whole 16-byte units on 16-byte boundaries: what the tensor maps and vector accesses of the kernels take."""
+    return t.dtype == torch.bfloat16 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+
+
+def _fitting_input(t: torch.Tensor, hd: int) -> torch.Tensor:
+    """Operands of heads other than 64 and 128 columns may lie anywhere: those that the kernels cannot read in place are copied.
+    (For 64 and 128 the kernels refuse them.)"""
+    return t if hd in (64, 128) or _rows_fit(t) else t.clone(memory_format=torch.contiguous_format)
+
+
+def _fitting_output(t: torch.Tensor, hd: int) -> torch.Tensor:
+    """``t``, or a tensor to be copied to it: likewise, for results of any layout and type."""
+    return t if hd in (64, 128) or _rows_fit(t) else torch.empty(t.shape, dtype=torch.bfloat16, device=t.device)
+
+
 def _dense_fwd(qkv, seq_start, H, KV, hd, scale, out):
     """Heads that have no tcgen05 kernel (above 128 columns, or not a multiple of 8): the dense fp32 statement on the device."""
     global _warned_dense
@@ -129,9 +145,10 @@ def attention_fwd(qkv: torch.Tensor, seq_start: torch.Tensor, H: int, KV: int, h
         out = torch.empty(M, H * hd, dtype=torch.bfloat16, device=qkv.device)
     if lse2 is None:
         lse2 = torch.empty(H, M, dtype=torch.float32, device=qkv.device)
-    check(native.cuda().pb_attn_fwd(ptr(qkv), ptr(seq_start), ptr(out), ptr(lse2), M, H, KV, hd, qkv.stride(0),
-                                    out.stride(0), scale, ptr(status_word(qkv.device)), stream_ptr()), "pb_attn_fwd")
-    return out, lse2
+    qkv, o = _fitting_input(qkv, hd), _fitting_output(out, hd)
+    check(native.cuda().pb_attn_fwd(ptr(qkv), ptr(seq_start), ptr(o), ptr(lse2), M, H, KV, hd, qkv.stride(0),
+                                    o.stride(0), scale, ptr(status_word(qkv.device)), stream_ptr()), "pb_attn_fwd")
+    return out if o is out else out.copy_(o), lse2
 
 
 def row_dots_buffer(device, M: int, H: int) -> torch.Tensor:
@@ -167,8 +184,9 @@ def attention_bwd(qkv: torch.Tensor, o: torch.Tensor, dout: torch.Tensor, lse2: 
     D = row_dots if row_dots is not None else _scratch_buf(qkv.device, "attn_D", M * H)
     tiles = _scratch_buf(qkv.device, "attn_tiles", (M + 127) // 128 + 1, torch.int32)
     assert rope_table is None or seq_len > 0
-    check(native.cuda().pb_attn_bwd(ptr(qkv), ptr(o) if row_dots is None else None, ptr(dout), ptr(lse2), ptr(seq_start), ptr(dqkv), ptr(dq_acc), ptr(D),
+    qkv, o, dout, g = _fitting_input(qkv, hd), _fitting_input(o, hd), _fitting_input(dout, hd), _fitting_output(dqkv, hd)
+    check(native.cuda().pb_attn_bwd(ptr(qkv), ptr(o) if row_dots is None else None, ptr(dout), ptr(lse2), ptr(seq_start), ptr(g), ptr(dq_acc), ptr(D),
                                     ptr(rope_table), max(int(seq_len), 1), M, H, KV, hd, qkv.stride(0),
-                                    o.stride(0), dout.stride(0), dqkv.stride(0), scale, ptr(tiles), ptr(status_word(qkv.device)),
+                                    o.stride(0), dout.stride(0), g.stride(0), scale, ptr(tiles), ptr(status_word(qkv.device)),
                                     stream_ptr()), "pb_attn_bwd")
-    return dqkv
+    return dqkv if g is dqkv else dqkv.copy_(g)

@@ -43,3 +43,31 @@ def test_splitk_is_chosen_for_whole_vectors_only(dtype):
     assert K._splitk_fits(good, None) and K._splitk_fits(good, good)
     for bad in (wide[:, 1:1025], wide[:, 2:1026], torch.zeros(256, 1030, dtype=dtype)[:, :1024]):
         assert not K._splitk_fits(bad, None) and not K._splitk_fits(good, bad)
+
+
+@no_device
+def test_attention_backward_refuses_rows_off_16_bytes():
+    """o and dqkv are read and written in 16-byte vectors that no tensor map checks."""
+    lib = _lib()
+    from prime_b200.ops import attention  # noqa: F401  (declares the C signatures)
+    base = 1 << 40
+
+    def call(**off):
+        a = [C.c_void_p(base + off.get(k, 0)) for k in ("qkv", "o", "dout", "lse2", "ss", "dqkv", "dq", "D")]
+        return lib.pb_attn_bwd(*a, None, 1, 256, 4, 2, 64, 512, 256, 256, 512, 0.125, None, None, None)
+    for k in ("qkv", "o", "dout", "dqkv"):
+        for bytes_off in (2, 4, 8):
+            assert call(**{k: bytes_off}) == -2
+
+
+def test_narrow_heads_are_copied_only_where_the_kernels_cannot_reach_them():
+    from prime_b200.ops import attention as A
+    wide = torch.zeros(16, 272, dtype=torch.bfloat16)
+    fits = wide[:, 8:264]
+    for bad in (wide[:, 1:257], torch.zeros(16, 260, dtype=torch.bfloat16)[:, :256], torch.zeros(256, 16, dtype=torch.bfloat16).t()):
+        for hd in (8, 32, 96):
+            assert A._fitting_input(fits, hd) is fits and A._fitting_output(fits, hd) is fits
+            assert A._rows_fit(A._fitting_input(bad, hd)) and A._rows_fit(A._fitting_output(bad, hd))
+        for hd in (64, 128):
+            assert A._fitting_input(bad, hd) is bad and A._fitting_output(bad, hd) is bad
+    assert A._fitting_output(torch.zeros(16, 256), 32).dtype == torch.bfloat16

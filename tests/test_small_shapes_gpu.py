@@ -199,3 +199,27 @@ def test_bf16_output_in_a_wider_matrix(M, N, K, a_mn, b_mn):
         ops.check_status()
         assert _rel(out, want) < 4e-3
         assert (wide[M] == 7).all() and (wide[:, N:] == 7).all()
+
+
+def test_narrow_heads_in_any_layout():
+    """Rows of odd pitch, rows off the 16-byte boundary and fp32 results give what dense tensors give."""
+    torch.manual_seed(0)
+    M, H, KV, hd = 203, 4, 2, 32
+    W, Wo = (H + 2 * KV) * hd, H * hd
+
+    def odd(t, pad=1):                                 # the same values one column into a matrix of odd pitch
+        wide = torch.zeros(t.shape[0], t.shape[1] + 2 * pad + 1, device="cuda", dtype=t.dtype)
+        wide[:, pad: pad + t.shape[1]] = t
+        return wide[:, pad: pad + t.shape[1]]
+    qkv, dout = torch.randn(M, W, device="cuda").bfloat16(), torch.randn(M, Wo, device="cuda").bfloat16()
+    ss, table = A.seq_start_from_batch(1, M, "cuda"), ops.rope_table(M, hd, 10000.0, "cuda")
+    o, lse2 = A.attention_fwd(qkv, ss, H, KV, hd)
+    g = A.attention_bwd(qkv, o, dout, lse2, ss, H, KV, hd, rope_table=table, seq_len=M)
+    for dt in (torch.bfloat16, torch.float32):
+        out, dqkv = odd(torch.zeros(M, Wo, device="cuda", dtype=dt)), odd(torch.zeros(M, W, device="cuda", dtype=dt))
+        o2, lse2b = A.attention_fwd(odd(qkv), ss, H, KV, hd, out=out)
+        assert o2 is out and torch.equal(out.float(), o.float()) and torch.equal(lse2b, lse2)
+        g2 = A.attention_bwd(odd(qkv), odd(o), odd(dout), lse2, ss, H, KV, hd, dqkv=dqkv, rope_table=table, seq_len=M)
+        ops.check_status()
+        # dQ is summed by atomic adds: their order moves its rounding to bf16 by one unit at most
+        assert g2 is dqkv and _rel(dqkv, g) < 2.0 ** -8
