@@ -8,6 +8,7 @@ use and what the GPU numerics tests compare against.
 from __future__ import annotations
 
 import functools
+import threading
 
 import torch
 
@@ -19,7 +20,7 @@ import os as _os
 # PRIME_B200_GEMM=single forces the single-CTA kernel (A/B measurements); default uses the CTA-pair kernel when it fits
 _GEMM_PAIR = _os.environ.get("PRIME_B200_GEMM", "pair") != "single"
 _status: dict[int, torch.Tensor] = {}
-_scratch: dict[tuple[int, int, str], torch.Tensor] = {}       # by device, stream and use
+_scratch: dict[tuple[int, int, str, int], torch.Tensor] = {}       # by device, stream, use and thread; the last used comes last
 
 
 def status_word(device: torch.device) -> torch.Tensor:
@@ -40,22 +41,24 @@ def check_status(device: torch.device | None = None) -> None:
 
 
 def _scratch_buf(device, key: str, numel: int, dtype=torch.float32) -> torch.Tensor:
-    """Scratch of one use on the current stream: kernels of other streams (weight gradients beside the backward, another
-    thread's model) run at the same time and have their own. At most 64 are kept, the oldest go back to the allocator."""
-    k = (device.index or 0, native.raw_stream(device.index), key)
-    t = _scratch.get(k)
+    """Scratch of one use on the current stream by the current thread. Kernels of other streams (weight gradients beside the
+    backward) run at the same time; another thread may launch between the kernel that fills the scratch and the one that reads
+    it, on the same stream too, since a native call lets other threads run. Each has its own. At most 64 are kept, those
+    unused for longest go back to the allocator (which hands them out again in the order of their stream)."""
+    k = (device.index or 0, native.raw_stream(device.index), key, threading.get_ident())
+    t = _scratch.pop(k, None)
     if t is None or t.numel() < numel or t.dtype != dtype:
         for old in list(_scratch)[:max(0, len(_scratch) - 63)]:
             _scratch.pop(old, None)
         t = torch.empty(numel, dtype=dtype, device=device)
-        _scratch[k] = t
+    _scratch[k] = t
     return t
 
 
 def take_scratch(stream: torch.cuda.Stream) -> list[torch.Tensor]:
-    """Hand over the scratch of ``stream``, which then starts anew: a recorded graph owns what was allocated while it was recorded,
-    since its replays may run beside other work on whichever stream has that handle later."""
-    keys = [k for k in list(_scratch) if k[1] == stream.cuda_stream]
+    """Hand over this thread's scratch of ``stream``, which then starts anew: a recorded graph owns what was allocated while it was
+    recorded, since its replays may run beside other work on whichever stream has that handle later."""
+    keys = [k for k in list(_scratch) if k[1] == stream.cuda_stream and k[3] == threading.get_ident()]
     return [t for t in (_scratch.pop(k, None) for k in keys) if t is not None]
 
 

@@ -71,3 +71,21 @@ def test_narrow_heads_are_copied_only_where_the_kernels_cannot_reach_them():
         for hd in (64, 128):
             assert A._fitting_input(bad, hd) is bad and A._fitting_output(bad, hd) is bad
     assert A._fitting_output(torch.zeros(16, 256), 32).dtype == torch.bfloat16
+
+
+def test_scratch_belongs_to_one_thread_and_is_bounded(monkeypatch):
+    import threading
+    monkeypatch.setattr(native, "raw_stream", lambda index=None: 7)
+    monkeypatch.setattr(K, "_scratch", {})
+    dev = torch.device("cpu")
+    mine, theirs = K._scratch_buf(dev, "splitk", 100), []
+    t = threading.Thread(target=lambda: theirs.append(K._scratch_buf(dev, "splitk", 100)))
+    t.start()
+    t.join()
+    assert mine.data_ptr() != theirs[0].data_ptr()                    # one stream, one use, two threads
+    assert K._scratch_buf(dev, "splitk", 80).data_ptr() == mine.data_ptr()
+    for i in range(200):                                              # what stays in use outlives what does not
+        K._scratch_buf(dev, f"use{i}", 1)
+        assert K._scratch_buf(dev, "splitk", 100).data_ptr() == mine.data_ptr() and len(K._scratch) <= 64
+    got = K.take_scratch(type("S", (), {"cuda_stream": 7})())
+    assert any(g.data_ptr() == mine.data_ptr() for g in got) and not any(k[3] == threading.get_ident() for k in K._scratch)

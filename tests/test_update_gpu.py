@@ -207,3 +207,28 @@ def test_update_sees_the_gradients_of_the_weight_gradient_stream(monkeypatch):
     for name, g in a.g.items():
         assert _rel(b.g[name], g) < 2 * 2.0 ** -8, name
     K.check_status()
+
+
+def test_threads_on_one_stream_do_not_share_partials():
+    """Products whose partials one launch writes and the next one sums, from two threads on the default stream."""
+    import threading
+    torch.manual_seed(4)
+    ops_ = [torch.randn(8192, n, device="cuda").bfloat16() for n in (256, 512)]
+    want = [x.float().t() @ x.float() for x in ops_]
+    torch.cuda.synchronize()
+    start, good = threading.Barrier(2), []
+
+    def work(i):
+        torch.cuda.set_device(0)
+        start.wait()
+        outs = [K.gemm(ops_[i], ops_[i], a_mn=True, b_mn=True, out_dtype=torch.float32) for _ in range(200)]
+        torch.cuda.synchronize()
+        good.extend(1 for o in outs if _rel(o, want[i]) < 1e-3)       # fp32 sums of the same products in another order
+    assert all(K._splitk_slices(x.shape[1], x.shape[1], 8192, x.device) > 1 for x in ops_)
+    ts = [threading.Thread(target=work, args=(i,)) for i in (0, 1)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert len(good) == 400
+    K.check_status()
