@@ -140,6 +140,11 @@ class _StepGraph:
 class FusedLlama:
     """See module docstring. One instance per process / GPU."""
     _MAX_GRAPHS = 8
+    # Recording costs 7-30 ms and a replay saves 0.5 ms (two-block model of 512 tokens: launch by launch 914 us, replayed 374 us,
+    # recorded and replayed 7-24 ms; the debug model's step 1913, 1388 us and 17-30 ms). With room left a shape is recorded
+    # at its second call. With none left it takes the place of the least recently used only after this many calls, so that a
+    # program with more shapes than graphs pays for a recording once in a few hundred steps.
+    _RUNS_TO_EVICT = 32
 
     def __init__(self, args: ModelArgs, device: torch.device | str = "cuda", comm=None, grad_dtype=torch.bfloat16,
                  ac_ckpt: bool | int = False, ce_chunk_tokens: int = 32768, z_mode: int = K.Z_NONE, z_weight: float = 0.0,
@@ -196,8 +201,8 @@ class FusedLlama:
         self.opt_step = 0
         self._accum = False            # gradients hold a partial sum from earlier micro-batches
         self._ws: dict[str, torch.Tensor] = {}
-        self._graphs: dict[tuple, _StepGraph] = {}      # recorded steps by shape and settings (see _graphed_step)
-        self._graph_seen: set[tuple] = set()
+        self._graphs: dict[tuple, _StepGraph] = {}      # recorded steps by shape and settings, the last used last (see _graphed_step)
+        self._graph_runs: dict[tuple, int] = {}         # calls of a shape without a graph since it last had one
         self._rope = K.rope_table(args.max_seq_len * 2, args.head_dim, args.rope_theta, dev)
         self._seq_start_cache: dict[tuple[int, int], torch.Tensor] = {}
         self.comm_stream = torch.cuda.Stream(device=dev) if dev.type == "cuda" else None
@@ -907,27 +912,32 @@ class FusedLlama:
     def _graphed_step(self, tokens, labels, seq_start, micro_bs: int, lr: float, betas, eps: float, weight_decay: float,
                       max_norm: float) -> torch.Tensor:
         """The step as a graph: recorded at the second call with the same shapes and settings (the first one runs launch by
-        launch and leaves the workspaces allocated), replayed from then on. Inputs and the step's scalars are copied into
-        buffers of the graph, so nothing depends on whose tensors they are. A graph holds every buffer it reads."""
+        launch and leaves the workspaces allocated; see _RUNS_TO_EVICT for a full table), replayed from then on. Inputs and the
+        step's scalars are copied into buffers of the graph, so nothing depends on whose tensors they are. A graph holds every
+        buffer it reads."""
         self.opt_step += 1
         B, T = tokens.shape
         key = (B, T, micro_bs, seq_start is not None, tuple(betas), eps, weight_decay, max_norm, self.z_mode, self.z_weight, self.ce_chunk,
                self.ac_every)
         report = self._buf("step.report", (4,), torch.float32)
-        g = self._graphs.get(key)
-        if g is None and key not in self._graph_seen:
-            if len(self._graph_seen) >= 64:
-                self._graph_seen.clear()
-            self._graph_seen.add(key)
-            self._accumulate_micro_batches(tokens, labels, seq_start, micro_bs)
-            self._update_from_own_grads(lr, betas, eps, weight_decay, max_norm)
-            self._accum = False
-            self._report(report)
-            return report
+        g = self._graphs.pop(key, None)
         if g is None:
-            if len(self._graphs) >= self._MAX_GRAPHS:
-                self._drop_graphs()
-            g = self._graphs[key] = _StepGraph(self, B, T, micro_bs, seq_start is not None, betas, eps, weight_decay, max_norm, report)
+            runs = self._graph_runs.pop(key, 0)
+            full = len(self._graphs) >= self._MAX_GRAPHS
+            if runs < (self._RUNS_TO_EVICT if full else 1):
+                self._accumulate_micro_batches(tokens, labels, seq_start, micro_bs)
+                self._update_from_own_grads(lr, betas, eps, weight_decay, max_norm)
+                self._accum = False
+                self._report(report)
+                for old in list(self._graph_runs)[:max(0, len(self._graph_runs) - 63)]:
+                    del self._graph_runs[old]
+                self._graph_runs[key] = runs + 1
+                return report
+            if full:
+                torch.cuda.synchronize(self.device)          # the graph that goes may still be running
+                del self._graphs[next(iter(self._graphs))]
+            g = _StepGraph(self, B, T, micro_bs, seq_start is not None, betas, eps, weight_decay, max_norm, report)
+        self._graphs[key] = g
         tokens, labels = tokens.contiguous(), labels.contiguous()
         seq_start = seq_start.contiguous() if seq_start is not None else None
         check(native.cuda().pb_stage_step(ptr(tokens), ptr(labels), ptr(seq_start), B * T, ptr(g.tokens), ptr(g.labels), ptr(g.seq_start), lr,
@@ -937,7 +947,9 @@ class FusedLlama:
         return report
 
     def _drop_graphs(self) -> None:
-        """Graphs point into the workspaces: called before one of those is replaced (the device is idle afterwards)."""
+        """Graphs point into the workspaces: called before one of those is replaced (the device is idle afterwards). Every shape
+        starts anew, so that steps whose sizes keep growing are not recorded between one growth and the next."""
+        self._graph_runs.clear()
         if self._graphs:
             torch.cuda.synchronize(self.device)
             self._graphs.clear()

@@ -268,3 +268,77 @@ def test_row_maps_reach_the_kernels_dense(monkeypatch, micro):
         assert len(seen) == B // micro and all(s.is_contiguous() and s.dtype == torch.int32 for s in seen)
         for mb, s in enumerate(seen):
             assert torch.equal(s, given[mb * micro * T: (mb + 1) * micro * T] - mb * micro * T)
+
+
+@pytest.fixture()
+def graph_engine(monkeypatch):
+    """An engine whose steps and graphs are stand-ins that write down what is recorded, replayed and launched."""
+    from prime_b200 import native
+    from prime_b200.engine import fused_llama
+    _, eng = _mk(_tiny())
+    log = []
+
+    class Graph:
+        launches = 0
+
+        def __init__(self, eng, B, T, *a):
+            self.tokens = self.labels = self.hyper = torch.zeros(1)
+            self.seq_start, self.graph, self.shape = None, self, (B, T)
+            log.append(("record", B, T))
+
+        def replay(self):
+            log.append(("replay", *self.shape))
+
+    def run(tokens, *a):
+        log.append(("run", *tokens.shape))
+        eng._buf("work", tokens.shape)
+    monkeypatch.setattr(fused_llama, "_StepGraph", Graph)
+    monkeypatch.setattr(fused_llama, "stream_ptr", lambda *a: None)
+    monkeypatch.setattr(native, "cuda", lambda: type("Lib", (), {"pb_stage_step": staticmethod(lambda *a: 0)}))
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: None)
+    monkeypatch.setattr(eng, "_accumulate_micro_batches", run)
+    monkeypatch.setattr(eng, "_update_from_own_grads", lambda *a, **k: None)
+    monkeypatch.setattr(eng, "_report", lambda *a: None)
+
+    def step(B, T):
+        n = len(log)
+        x = torch.zeros(B, T, dtype=torch.int64)
+        eng._graphed_step(x, x, None, B, 1e-3, (0.9, 0.95), 1e-8, 0.1, 1.0)
+        return [e[0] for e in log[n:]]
+    return eng, step, log
+
+
+def test_more_shapes_than_graphs_are_not_recorded_over_and_over(graph_engine):
+    eng, step, log = graph_engine
+    eng._buf("work", (64, 64))
+    rounds, shapes = 100, [(2, 8 + i) for i in range(eng._MAX_GRAPHS + 1)]
+    for _ in range(rounds):
+        for s in shapes:
+            step(*s)
+    # one recording for each of the first eight, then one per _RUNS_TO_EVICT rounds
+    assert sum(e[0] == "record" for e in log) <= eng._MAX_GRAPHS + rounds / eng._RUNS_TO_EVICT
+    assert sum(e[0] == "replay" for e in log) >= (rounds - 2) * eng._MAX_GRAPHS - eng._MAX_GRAPHS
+    assert len(eng._graphs) == eng._MAX_GRAPHS
+
+
+def test_the_least_recently_used_graph_gives_way(graph_engine):
+    eng, step, log = graph_engine
+    eng._buf("work", (64, 64))
+    shapes = [(2, 8 + i) for i in range(eng._MAX_GRAPHS)]
+    for s in shapes:
+        assert step(*s) == ["run"] and step(*s) == ["record", "replay"]
+    assert step(*shapes[0]) == ["replay"]               # now shapes[1] was used longest ago
+    for _ in range(eng._RUNS_TO_EVICT):
+        assert step(3, 8) == ["run"]
+    assert step(3, 8) == ["record", "replay"]
+    assert step(*shapes[0]) == ["replay"] and step(*shapes[2]) == ["replay"] and step(*shapes[1]) == ["run"]
+
+
+def test_growing_steps_are_not_recorded_in_between(graph_engine):
+    """A short shape that alternates with ever longer ones: each growth of a workspace drops what was recorded before it."""
+    eng, step, log = graph_engine
+    for i in range(20):
+        step(2, 8)
+        step(2, 16 + i)
+    assert not any(e[0] == "record" for e in log)
+    assert step(2, 8) == ["run"] and step(2, 8) == ["record", "replay"]      # once it has stopped
