@@ -382,10 +382,10 @@ class FusedLlama:
         gradient shard. The engine still does forward / backward, the reduce-scatter, the global-norm clip and the bf16
         all-gather; the optimizer sees exactly what FSDP2 would hand a sharded optimizer (each rank's rows of every
         parameter), which is how a fully-sharded Shampoo / SOAP preconditions: per rank, on its own block of rows."""
-        params = []
+        params, grads = [], self.grad_shard        # read once: without peers each access copies the whole gradient buffer
         for name, shard in self.named_master_shards():
             q = torch.nn.Parameter(shard, requires_grad=True)
-            q.grad = self.shard_view(self.grad_shard, name)
+            q.grad = self.shard_view(grads, name)
             params.append(q)
         self._shard_params = params
         self._shard_opt = factory([q for q in params if q.numel() > 0])

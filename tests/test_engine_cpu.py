@@ -342,3 +342,13 @@ def test_growing_steps_are_not_recorded_in_between(graph_engine):
         step(2, 16 + i)
     assert not any(e[0] == "record" for e in log)
     assert step(2, 8) == ["run"] and step(2, 8) == ["record", "replay"]      # once it has stopped
+
+
+def test_shard_optimizer_reads_the_gradient_shard_once(monkeypatch):
+    _, eng = _mk(_tiny())
+    reads, shard = [], FusedLlama.grad_shard
+    monkeypatch.setattr(FusedLlama, "grad_shard", property(lambda self: reads.append(1) or shard.fget(self)))
+    eng.set_shard_optimizer(lambda ps: torch.optim.SGD(ps, lr=0.1))
+    assert len(reads) == 1
+    for (name, _), q in zip(eng.named_master_shards(), eng._shard_params):
+        assert q.grad.data_ptr() == eng.shard_view(eng._grad_shard, name).data_ptr()
