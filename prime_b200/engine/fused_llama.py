@@ -382,7 +382,7 @@ class FusedLlama:
         gradient shard. The engine still does forward / backward, the reduce-scatter, the global-norm clip and the bf16
         all-gather; the optimizer sees exactly what FSDP2 would hand a sharded optimizer (each rank's rows of every
         parameter), which is how a fully-sharded Shampoo / SOAP preconditions: per rank, on its own block of rows."""
-        params, grads = [], self.grad_shard        # read once: without peers each access copies the whole gradient buffer
+        params, grads = [], self.grad_shard        # read once: the first access may copy the whole gradient buffer
         for name, shard in self.named_master_shards():
             q = torch.nn.Parameter(shard, requires_grad=True)
             q.grad = self.shard_view(grads, name)
@@ -696,6 +696,8 @@ class FusedLlama:
         W = self.world
         if self._direct_update:
             self._update_from_own_grads(lr, betas, eps, weight_decay, max_norm)
+            if self._grad_shard is not None:
+                self._fill_grad_shard()
             self._accum = False
             return self._norm_global[0].sqrt()
         # Reduce-scatter by pull, one launch per parameter group. Groups whose gradients were final during the backward are
@@ -738,17 +740,21 @@ class FusedLlama:
 
     @property
     def grad_shard(self) -> torch.Tensor:
-        """This rank's reduced fp32 gradients, one value per owned parameter element. A run without peers that updates with the
-        AdamW kernel never asks for it (4 bytes per parameter that stay free); there it is allocated by the first access and
-        filled from the gradient buffer on each one. ``set_shard_optimizer`` is such an access, before any reduce."""
+        """This rank's reduced fp32 gradients of the last step, one value per owned parameter element. A run without peers that
+        updates with the AdamW kernel has no use for them (4 bytes per parameter that stay free): there the first access
+        allocates the tensor and copies the gradient buffer to it, and from then on every step does.
+        ``set_shard_optimizer`` is such an access, before any reduce."""
         if self._grad_shard is None:
             self._grad_shard = torch.zeros(self.layout.shard_numel[self.rank], dtype=torch.float32, device=self.device)
-        if self._direct_update:
-            self._wait_all_wgrads()
-            for sa in self._segs_step:
-                for f, s, n in zip(sa.full[:sa.n], sa.shard[:sa.n], sa.numel[:sa.n]):
-                    self._grad_shard[s: s + n].copy_(self.grads[f: f + n])
+            if self._direct_update:
+                self._fill_grad_shard()
         return self._grad_shard
+
+    def _fill_grad_shard(self) -> None:
+        self._wait_all_wgrads()
+        for sa in self._segs_step:
+            for f, s, n in zip(sa.full[:sa.n], sa.shard[:sa.n], sa.numel[:sa.n]):
+                self._grad_shard[s: s + n].copy_(self.grads[f: f + n])
 
     @property
     def _direct_update(self) -> bool:
@@ -851,6 +857,8 @@ class FusedLlama:
             labels = labels.to(self.device, non_blocking=True)
         if self._graphable(tokens, labels, seq_start, B // micro_bs):
             report = self._graphed_step(tokens, labels, seq_start, micro_bs, lr, betas, eps, weight_decay, max_norm)
+            if self._grad_shard is not None:
+                self._fill_grad_shard()
         else:
             self._accumulate_micro_batches(tokens, labels, seq_start, micro_bs)
             norm = self.optimizer_step(lr, betas, eps, weight_decay, max_norm)

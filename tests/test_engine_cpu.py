@@ -250,7 +250,7 @@ def test_update_without_peers_waits_for_the_weight_gradient_stream(monkeypatch):
     eng._update_from_own_grads(1e-3, (0.9, 0.95), 1e-8, 0.1, 1.0)
     assert order == ["join", "pb_grad_sumsq", "pb_zero_adamw_gather"]
     order.clear()
-    eng._readers = {1: "event"}
+    eng._grad_shard, eng._readers = None, {1: "event"}
     assert eng.grad_shard is not None and order == ["join"]
 
 
@@ -288,6 +288,7 @@ def graph_engine(monkeypatch):
 
         def replay(self):
             log.append(("replay", *self.shape))
+            getattr(eng, "on_replay", lambda: None)()
 
     def run(tokens, *a):
         log.append(("run", *tokens.shape))
@@ -352,3 +353,36 @@ def test_shard_optimizer_reads_the_gradient_shard_once(monkeypatch):
     assert len(reads) == 1
     for (name, _), q in zip(eng.named_master_shards(), eng._shard_params):
         assert q.grad.data_ptr() == eng.shard_view(eng._grad_shard, name).data_ptr()
+
+
+@pytest.mark.parametrize("graphed", [False, True])
+def test_a_gradient_shard_in_hand_follows_the_steps(graph_engine, monkeypatch, graphed):
+    """Without peers the shard is filled for those who ask for it: who keeps the tensor finds each step's gradients in it, and those
+    of the last step while the next one's accumulate."""
+    eng, _, log = graph_engine
+    eng._solo, eng._grad_shard = True, None
+    monkeypatch.setattr(eng, "_graphable", lambda *a: graphed)
+
+    def step(value):
+        def backward(*a):
+            eng.grads.fill_(value)
+            eng._accum = True
+        monkeypatch.setattr(eng, "_accumulate_micro_batches", backward)
+        x = torch.zeros(1, 8, dtype=torch.int64)
+        if graphed:
+            eng.on_replay = lambda: eng.grads.fill_(value)
+            eng.train_step(x, x, lr=1e-3, sync_loss=False)
+        else:                    # what train_step does on a GPU; the CPU has an update of its own
+            backward()
+            monkeypatch.setattr(eng, "device", torch.device("cuda"))
+            eng.optimizer_step(1e-3)
+            monkeypatch.setattr(eng, "device", torch.device("cpu"))
+    step(1.0)
+    assert eng._grad_shard is None                       # nobody asked yet
+    held = eng.grad_shard
+    assert (held == 1).all()
+    for v in (2.0, 3.0, 4.0):
+        step(v)
+        assert (held == v).all() and eng.grad_shard is held
+    eng.grads.fill_(9.0)                                 # the next step's backward
+    assert (eng.grad_shard == 4).all()

@@ -258,3 +258,17 @@ def test_steps_whose_graphs_give_way_to_each_other(monkeypatch):
             getattr(b, name).copy_(getattr(a, name))
     assert held == {(4, 256), (4, 200), (2, 64)}      # every shape had a graph at some time
     K.check_status()
+
+
+def test_a_gradient_shard_in_hand_follows_recorded_steps():
+    from prime_b200.engine.fused_llama import FusedLlama
+    from prime_b200.models.llama import ModelArgs
+    eng = FusedLlama(ModelArgs(dim=256, n_layers=2, n_heads=4, ffn_hidden=512, vocab_size=1024, max_seq_len=256, init_mode="normal"),
+                     device="cuda", ce_chunk_tokens=512)
+    eng.init_weights(seed=3)
+    held, g = eng.grad_shard, torch.Generator(device="cuda").manual_seed(1)
+    for _ in range(4):             # launched one by one, recorded, replayed
+        ids = torch.randint(0, 1024, (2, 129), device="cuda", generator=g)
+        eng.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3)
+        assert all(torch.equal(eng.shard_view(held, name), v.float()) for name, v in eng.g.items()) and held.any()
+    assert eng._graphs
