@@ -6,7 +6,7 @@ between iterations, achieved TFLOP/s or GB/s, and the fraction of the measured p
     python benchmarks/kernel_bench.py gemm --m 65536 --n 4096 --k 1024 [--a-mn --b-mn]
     python benchmarks/kernel_bench.py attn_fwd --batch 32 --seq 1024 --heads 16 --kv 16 --hd 64
     python benchmarks/kernel_bench.py attn_bwd ...
-    python benchmarks/kernel_bench.py rmsnorm|swiglu|adamw --rows 65536 --cols 1024
+    python benchmarks/kernel_bench.py rmsnorm|swiglu|adamw|cross_entropy|quantize --rows 65536 --cols 1024
 
 The same commands are what the ncu captures under profiles/ were taken with (small shapes there).
 """
@@ -115,7 +115,14 @@ def main():
         # HBM bytes per element: read 4, write 1 (A); read 1, write 1 (B, one rank); read 1, write 4 (C) = 12
         out.update(shape=[n], ms=ms, gbs=12.0 * n / ms / 1e6, frac=12.0 * n / ms / 1e6 / gbs, frac_of=tag)
         dist.destroy_process_group()
-    elif a.kernel in ("rmsnorm", "rmsnorm_bwd", "swiglu", "swiglu_bwd", "adamw"):
+    elif a.kernel == "quantize":
+        from prime_b200.ops import quant
+        n = a.rows * a.cols
+        x = torch.randn(n, device=dev) * 1e-3
+        ms = timeit(lambda: quant.uniform_8bit_quantize_cuda(x), a.iters, flush)
+        nbytes = 5 * n + 1024 * -(-n // 16384)      # fp32 in, a byte and a codebook per chunk out
+        out.update(shape=[n], ms=ms, gbs=nbytes / ms / 1e6, frac=nbytes / ms / 1e6 / gbs, frac_of=tag)
+    elif a.kernel in ("rmsnorm", "rmsnorm_bwd", "swiglu", "swiglu_bwd", "adamw", "cross_entropy"):
         R, Cn = a.rows, a.cols
         if a.kernel == "rmsnorm":
             x = torch.randn(R, Cn, device=dev, dtype=torch.bfloat16)
@@ -142,6 +149,12 @@ def main():
             d = torch.randn(R, Cn, device=dev, dtype=torch.bfloat16)
             ms = timeit(lambda: K.swiglu_bwd(h, d, dh13=h), a.iters, flush)
             nbytes = 5 * R * Cn * 2
+        elif a.kernel == "cross_entropy":
+            lg = torch.randn(R, Cn, device=dev).bfloat16()      # overwritten with gradients; the kernel's work does not depend on the values
+            lab, rows = torch.randint(0, Cn, (R,), device=dev), torch.empty(R, device=dev)
+            inv = K.count_valid(lab)
+            ms = timeit(lambda: K.cross_entropy_(lg, lab, inv, rows, None), a.iters, flush)
+            nbytes = 2 * R * Cn * 2
         else:
             n = R * Cn
             p, m, v = torch.randn(n, device=dev), torch.zeros(n, device=dev), torch.zeros(n, device=dev)

@@ -24,8 +24,8 @@ struct AttnBwdParams {
     const int* seq_start;
     const float* lse2;     // [H, M]
     const float* D;        // [H, M]
-    float* dq_acc;         // [M, H*hd] fp32, zero-initialised by the caller
-    __nv_bfloat16* dqkv;   // [M, (H+2KV)*HD]; the backward kernel writes the k and v column blocks
+    float* dq_acc;         // [M, H*hd] fp32, zeroed by the span pre-pass of the same call
+    __nv_bfloat16* dqkv;   // [M, (H+2KV)*hd]; the backward kernel writes the k and v column blocks
     long long dqkv_stride;
     float scale, scale_log2;
     int* status;

@@ -155,7 +155,9 @@ struct ItemRing {
 // predecessor has completed and its writes are visible, and only then lets the successor start, so at most one kernel waits at
 // a time and everything before the predecessor is complete as well. Rules: no global memory access before pdl_sync(),
 // every thread calls it, and kernels that talk to other GPUs are launched the ordinary way.
-// (pdl_sync() does nothing in an ordinary launch.)
+// In an ordinary launch pdl_sync() has nothing to wait for but still lets the successor start, if that is launched early: behind an
+// all-gather GEMM, say, whose CTAs are all resident by then. Such a successor waits like any other, on SM slots that a
+// communication kernel could have had meanwhile.
 // CTAs of an early launch go to the first SMs that have room and pile up there, while the grids of the streaming kernels are
 // made for an even share of every SM: the AdamW pass of the 10B blocks (148 CTAs, 58 GB) took 18 ms instead of 11.4. Such a
 // kernel says how many bytes it moves (LaunchCfg::traffic) and is launched early only below 32 MB, which take about as long as

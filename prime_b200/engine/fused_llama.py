@@ -109,7 +109,8 @@ class LocalComm:
 
 
 class _StepGraph:
-    """One recorded ``train_step``: its input buffers, the graph, and references to every buffer the graph touches."""
+    """One recorded ``train_step``: its input buffers, the graph, and references to the workspaces and the scratch that the graph
+    touches (parameters, gradients and optimizer state are the engine's for as long as it lives)."""
 
     def __init__(self, eng: "FusedLlama", B: int, T: int, micro_bs: int, packed: bool, betas, eps, weight_decay, max_norm, report):
         dev = eng.device
@@ -903,10 +904,11 @@ class FusedLlama:
     # steps replayed from a CUDA graph
     # ------------------------------------------------------------------------------------------
     def _graphable(self, tokens, labels, seq_start, n_micro: int) -> bool:
-        """Small steps without peers are replayed as one graph launch: a launch costs the host about 13 us through the Python
-        wrappers, so a step whose kernels average less than that waits for the host (two-block model, 512 tokens: 69 launches,
-        1.19 ms of host against 0.4 ms of kernels). The line: twice as much host time as the step's operations take at a
-        middling 600 TFLOP/s; above it the queue never runs dry and a graph changes nothing."""
+        """Small steps without peers are replayed as one graph launch: a launch costs the host 14 us through the Python wrappers, so
+        a step whose kernels average less than that waits for the host (two-block model, 512 tokens: 60 launches of this
+        package, 0.86 ms of host and 0.91 ms in all, replayed 0.37; debug model of 16 x 1024: 131 launches, 1.83 of 1.91 ms,
+        replayed 1.39). The line: twice the host time, at 13 us a launch, against the step's operations at a middling
+        600 TFLOP/s; above it the queue never runs dry and a graph changes nothing."""
         if not (self._direct_update and self.wgrad_stream is None and not self._accum and tokens.is_cuda and labels.is_cuda
                 and tokens.dtype == torch.int64 and labels.dtype == torch.int64 and tokens.device == self._counters.device
                 and (seq_start is None or (seq_start.is_cuda and seq_start.dtype == torch.int32))):
@@ -921,8 +923,7 @@ class FusedLlama:
                       max_norm: float) -> torch.Tensor:
         """The step as a graph: recorded at the second call with the same shapes and settings (the first one runs launch by
         launch and leaves the workspaces allocated; see _RUNS_TO_EVICT for a full table), replayed from then on. Inputs and the
-        step's scalars are copied into buffers of the graph, so nothing depends on whose tensors they are. A graph holds every
-        buffer it reads."""
+        step's scalars are copied into buffers of the graph, so nothing depends on whose tensors they are."""
         self.opt_step += 1
         B, T = tokens.shape
         key = (B, T, micro_bs, seq_start is not None, tuple(betas), eps, weight_decay, max_norm, self.z_mode, self.z_weight, self.ce_chunk,

@@ -50,10 +50,13 @@ def test_narrow_heads(hd):
     assert _rel(g, gref) < 3e-2
 
 
-@pytest.mark.parametrize("hd", [16, 32])
-def test_rope_epilogue_narrow_heads(hd):
+# (rows, positions): rows that divide neither tile nor positions, one position, whole tiles; one more rotated head than the epilogue's
+# 64-column boxes hold goes to the separate kernel
+@pytest.mark.parametrize("M,T", [(777, 200), (512, 1), (1024, 1024)])
+@pytest.mark.parametrize("hd,extra", [(8, 0), (16, 0), (32, 0), (8, 1), (16, 1), (32, 1)])
+def test_rope_epilogue_narrow_heads(hd, extra, M, T):
     torch.manual_seed(0)
-    M, K, T, H, KV = 777, 256, 200, 256 // hd, 128 // hd
+    K, H, KV = 256, 256 // hd, 128 // hd + extra
     N = (H + 2 * KV) * hd
     x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
     w = (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()

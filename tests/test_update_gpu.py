@@ -118,7 +118,7 @@ def test_graphed_steps_match_steps_launched_one_by_one(monkeypatch, hd, micro, p
             ss += torch.where(torch.arange(B * T, device="cuda") % T >= cut, cut, 0).int()
         res = [e.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3 * (i + 1), micro_bs=micro, seq_start=ss) for e in (a, b)]
         replayed += bool(a._graphs)
-        # the kernels are the same; only the embedding gradient's atomic adds may come in another order (bf16: 2^-8 each).
+        # the kernels are the same; the atomic adds of dQ and of the embedding gradient may come in another order (bf16: 2^-8 each).
         # Adam turns such a difference of a tiny gradient into one of the update's full size, so every step starts from one state
         assert res[0] == pytest.approx(res[1], rel=2e-3)
         assert ((a.master - b.master).norm() / b.master.norm()).item() < (1e-4 if fp32 else 5e-3)
@@ -272,3 +272,29 @@ def test_a_gradient_shard_in_hand_follows_recorded_steps():
         eng.train_step(ids[:, :-1], ids[:, 1:], lr=1e-3)
         assert all(torch.equal(eng.shard_view(held, name), v.float()) for name, v in eng.g.items()) and held.any()
     assert eng._graphs
+
+
+@pytest.mark.parametrize("segs", SEGS)
+@pytest.mark.parametrize("world", [2, 5, 9])      # the three widths of the kernel's rank loop
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_reduce_over_several_buffers(segs, world, dtype):
+    """One rank's part of the reduce, with every rank's buffer on this GPU: the kernel reads them all and waits for nobody."""
+    torch.manual_seed(0)
+    n_full, n_shard = max(s[0] + s[2] for s in segs) + 8, max(s[1] + s[2] for s in segs) + 8
+    gs = [torch.randn(n_full, device="cuda").to(dtype) for _ in range(world)]
+    full, shard, numel = _arrays(segs)
+    total = torch.zeros(n_full, device="cuda")
+    for g in gs:                                   # in rank order, like the kernel
+        total += g.float()
+    want = torch.cat([total[a: a + n] for a, _, n in segs]) * 0.25
+    out, sq, partial = torch.full((n_shard,), 7.0, device="cuda"), torch.zeros(1, device="cuda"), torch.zeros(4096, device="cuda")
+    check(native.cuda().pb_zero_reduce_grads((C.c_void_p * world)(*[g.data_ptr() for g in gs]), world, 1, int(dtype == torch.float32),
+                                             len(segs), full, shard, numel, ptr(out), 0.25, ptr(partial), ptr(sq), 0, 148, stream_ptr()),
+          "pb_zero_reduce_grads")
+    assert torch.equal(torch.cat([out[b: b + n] for _, b, n in segs]), want)
+    ref = want.double().square().sum().item()
+    assert abs(sq.item() - ref) < 1e-5 * ref       # fp32 sums of n squares in a tree, as above
+    keep = torch.ones(n_shard, dtype=torch.bool, device="cuda")
+    for _, b, n in segs:
+        keep[b: b + n] = False
+    assert (out[keep] == 7).all()
