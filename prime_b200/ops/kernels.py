@@ -94,7 +94,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, resi
         assert residual.dtype == out.dtype and residual.shape == out.shape and residual.stride(-1) == 1
     ldr = residual.stride(0) if residual is not None else 0
     # bn: 0 = choose; 128 / 256 = single-CTA tile width; 512 = the CTA-pair (cta_group::2) 256x256 kernel
-    slices = _splitk_slices(M, N, K, a.device) if bn == 0 and _GEMM_PAIR and _splitk_fits(out, residual) else 1
+    slices = _splitk_slices(M, N, K, a.device) if bn == 0 and _GEMM_PAIR else 1
+    if slices > 1 and not _splitk_fits(out, residual):
+        slices = 1
     use_pair = bn == 512 or slices > 1 or (bn == 0 and _GEMM_PAIR and M >= 512 and N >= 256)
     if use_pair:
         if slices > 1:
