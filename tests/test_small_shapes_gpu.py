@@ -226,3 +226,21 @@ def test_narrow_heads_in_any_layout():
         ops.check_status()
         # dQ is summed by atomic adds: their order moves its rounding to bf16 by one unit at most
         assert g2 is dqkv and _rel(dqkv, g) < 2.0 ** -8
+
+
+# K that ends inside a 16-byte unit: what lies behind an operand's last column is not read (a logits buffer's padding holds anything)
+@pytest.mark.parametrize("M,N", [(600, 512), (100, 128)])
+@pytest.mark.parametrize("K", [1025, 1031])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_operand_padding_is_not_read(M, N, K, b_mn):
+    torch.manual_seed(0)
+
+    def padded(rows):
+        wide = torch.full((rows, (K + 7) // 8 * 8), float("nan"), device="cuda", dtype=torch.bfloat16)
+        wide[:, :K] = torch.randn(rows, K, device="cuda")
+        return wide[:, :K]
+    a, b = padded(M), torch.randn(K, N, device="cuda").bfloat16() if b_mn else padded(N)
+    out = ops.gemm(a, b, b_mn=b_mn, out_dtype=torch.float32)
+    ops.check_status()
+    ref = a.double() @ (b.double() if b_mn else b.double().t())
+    assert _rel(out.double(), ref) < 2.0 ** -22 * K ** 0.5      # fp32 accumulation of K products
