@@ -908,7 +908,9 @@ class FusedLlama:
         a step whose kernels average less than that waits for the host (two-block model, 512 tokens: 60 launches of this
         package, 0.86 ms of host and 0.91 ms in all, replayed 0.37; debug model of 16 x 1024: 131 launches, 1.83 of 1.91 ms,
         replayed 1.39). The line: twice the host time, at 13 us a launch, against the step's operations at a middling
-        600 TFLOP/s; above it the queue never runs dry and a graph changes nothing."""
+        600 TFLOP/s. Above it the queue does not run dry, and what a graph saves is the 0.3 ms around each step's read of its
+        loss, in ms, replayed and one by one: below the line 70M 4 x 1024 tokens 2.47 and 2.77, 8 x 1024 3.5 and 3.65, 150M
+        2 x 1024 6.25 and 6.57; above it 70M 16 x 1024 6.2 and 6.4, 150M 4 x 1024 9.1 and 9.4, 6 x 1024 12.8 and 13.2."""
         if not (self._direct_update and self.wgrad_stream is None and not self._accum and tokens.is_cuda and labels.is_cuda
                 and tokens.dtype == torch.int64 and labels.dtype == torch.int64 and tokens.device == self._counters.device
                 and (seq_start is None or (seq_start.is_cuda and seq_start.dtype == torch.int32))):
