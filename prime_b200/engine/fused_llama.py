@@ -484,7 +484,10 @@ class FusedLlama:
     # ------------------------------------------------------------------------------------------
     # forward / backward of one block
     # ------------------------------------------------------------------------------------------
-    def _block_fwd(self, i: int, x: torch.Tensor, T: int, seq_start: torch.Tensor, out: torch.Tensor, recompute: bool = False) -> None:
+    def _block_fwd(self, i: int, x: torch.Tensor, T: int, seq_start: torch.Tensor, out: torch.Tensor | None) -> None:
+        """Without ``out`` (recomputation in the backward) the block stops at the activations that its backward reads: its own
+        output, the product with w2, is not one of them. 10B block, 8192 tokens: 0.65 of 2.95 ms of a recomputation."""
+        recompute = out is None
         a = self.args
         M = x.shape[0]
         D, F, hd, H, KV = a.dim, a.hidden_dim, a.head_dim, a.n_heads, a.kv_heads
@@ -522,6 +525,8 @@ class FusedLlama:
         h13 = self._saved(i, "h13", (M, 2 * F))
         act = self._saved(i, "act", (M, F))
         K.gemm_swiglu(hn, self.w13[i], h13, act)                          # SwiGLU in the GEMM epilogue
+        if recompute:
+            return
         K.gemm(act, self.w[pre + "feed_forward.w2.weight"], out=out, residual=h)
         if fetch:
             self._release_block(i)
@@ -565,7 +570,7 @@ class FusedLlama:
         pre = f"layers.{i}."
         if self._is_ckpt(i):   # recompute the block's activations into the shared workspace
             self._wait_all_wgrads()    # weight gradients of the block above still read that workspace
-            self._block_fwd(i, x, T, seq_start, self._buf("ckpt_out", (M, D)), recompute=True)
+            self._block_fwd(i, x, T, seq_start, None)
         sv = lambda n, shp, dt=torch.bfloat16: self._saved(i, n, shp, dt)  # noqa: E731
         xn, rstd1, qkv, o = sv("xn", (M, D)), sv("rstd1", (M,), torch.float32), sv("qkv", (M, (H + 2 * KV) * hd)), sv("o", (M, H * hd))
         lse2 = sv("lse2", (H, M), torch.float32)
