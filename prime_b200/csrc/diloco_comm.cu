@@ -131,7 +131,63 @@ __device__ __forceinline__ float dl_block_sum(float v) {
 constexpr float DL_MAGIC = 12582912.f;
 constexpr int DL_MAGIC_BITS = 0x4B400000;
 
-template <int G, bool FULL>
+// A whole chunk of finite values. |x| <= the chunk's L2 norm, so that |t| = |x / scale| < 2^13: the rounded value has its bin in its
+// low bits, clamped by one instruction. Every element goes to the table without a test: those of the two clamping bins leave
+// something in rows 0 and 255 that nobody reads. Whether there are any is asked once per four elements.
+template <int G>
+__device__ __forceinline__ void dl_quantize_finite(const float (&v)[DL_PER_THREAD], uint8_t* __restrict__ q_chunk, bool q_aligned,
+                                                   unsigned* my_bin, long long (&e_sum)[2], unsigned (&e_cnt)[2], float inv_scale) {
+    const unsigned long long inv2 = f32x2_pack(inv_scale, inv_scale), magic2 = f32x2_pack(DL_MAGIC, DL_MAGIC),
+                             nmagic2 = f32x2_pack(-DL_MAGIC, -DL_MAGIC), neg2 = f32x2_pack(-1.f, -1.f),
+                             fx2 = f32x2_pack(float(1 << DL_FX_BITS), float(1 << DL_FX_BITS)),
+                             off2 = f32x2_pack(DL_MAGIC + float(1 << (DL_FX_BITS - 1)), DL_MAGIC + float(1 << (DL_FX_BITS - 1)));
+#pragma unroll
+    for (int k = 0; k < DL_PER_THREAD / G; ++k) {
+        const int e0 = (k * DL_THREADS + int(threadIdx.x)) * G;
+        uint32_t w[G / 4];
+#pragma unroll
+        for (int j0 = 0; j0 < G; j0 += 4) {
+            int qi[4];
+            float t[4];
+#pragma unroll
+            for (int j = 0; j < 4; j += 2) {
+                const int e = G * k + j0 + j;
+                const unsigned long long t2 = f32x2_mul(f32x2_pack(v[e], v[e + 1]), inv2);
+                const unsigned long long m2 = f32x2_add(t2, magic2);
+                const unsigned long long d2 = f32x2_fma(f32x2_add(m2, nmagic2), neg2, t2);      // distance from the nearest bin
+                float m[2], o[2];
+                f32x2_unpack(t2, t[j], t[j + 1]);
+                f32x2_unpack(m2, m[0], m[1]);
+                f32x2_unpack(f32x2_fma(d2, fx2, off2), o[0], o[1]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    qi[j + h] = __viaddmin_s32_relu(__float_as_int(m[h]), 128 - DL_MAGIC_BITS, 255);
+                    atomicAdd(&my_bin[qi[j + h] << 5], unsigned(__float_as_int(o[h]) - (DL_MAGIC_BITS - (1 << DL_CNT_SHIFT))));
+                }
+            }
+            w[j0 / 4] = __byte_perm(__byte_perm(qi[0], qi[1], 0x0040), __byte_perm(qi[2], qi[3], 0x0040), 0x5410);
+            if (fmaxf(max3(fabsf(t[0]), fabsf(t[1]), fabsf(t[2])), fabsf(t[3])) >= 126.5f) {
+                // exact sums of the clamping bins, kept per thread (about one element in 400 lands here) and combined once per chunk
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (unsigned(qi[j] - 1) < 254u) continue;
+                    const long long fx = __float2int_rn(t[j] * float(1 << DL_EDGE_FX_BITS));
+                    if (qi[j]) { e_sum[1] += fx; ++e_cnt[1]; }
+                    else { e_sum[0] += fx; ++e_cnt[0]; }
+                }
+            }
+        }
+        if (q_aligned) {
+            if (G == 4) *reinterpret_cast<uint32_t*>(q_chunk + e0) = w[0];
+            else *reinterpret_cast<uint4*>(q_chunk + e0) = make_uint4(w[0], w[1 % (G / 4)], w[2 % (G / 4)], w[3 % (G / 4)]);
+        } else {
+            for (int j = 0; j < G; ++j) q_chunk[e0 + j] = uint8_t(w[j >> 2] >> (8 * (j & 3)));
+        }
+    }
+}
+
+// Any chunk: `cnt` of its elements are there, and they may hold infinities or NaN.
+template <int G>
 __device__ __forceinline__ void dl_quantize_body(const float (&v)[DL_PER_THREAD], int cnt, uint8_t* __restrict__ q_chunk,
                                                  bool q_aligned, unsigned* my_bin, long long (&e_sum)[2], unsigned (&e_cnt)[2],
                                                  float inv_scale) {
@@ -166,7 +222,7 @@ __device__ __forceinline__ void dl_quantize_body(const float (&v)[DL_PER_THREAD]
                     // nearest bin (a tie, one value in ~10^7, goes to the even one); far outside the magic range the sign and a
                     // large magnitude survive
                     const int raw = __float_as_int(m[h]) - (DL_MAGIC_BITS - 128);
-                    const bool live = FULL || e0 + j0 + j + h < cnt;
+                    const bool live = e0 + j0 + j + h < cnt;
                     const bool inner = unsigned(raw - 1) < 254u;
                     if (live && inner) atomicAdd(&my_bin[raw << 5], unsigned(__float_as_int(o[h]) - (DL_MAGIC_BITS - (1 << DL_CNT_SHIFT))));
                     edge |= live && !inner;
@@ -179,7 +235,7 @@ __device__ __forceinline__ void dl_quantize_body(const float (&v)[DL_PER_THREAD]
                 // per thread (about one element in 400 lands here) and combined once per chunk
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    if ((FULL || e0 + j0 + j < cnt) && unsigned(qi[j] - 1) >= 254u) {
+                    if (e0 + j0 + j < cnt && unsigned(qi[j] - 1) >= 254u) {
                         const float t = v[G * k + j0 + j] * inv_scale;
                         const long long fx = __float2ll_rn(fminf(fmaxf(t, -1.0e6f), 1.0e6f) * float(1 << DL_EDGE_FX_BITS));
                         if (qi[j]) { e_sum[1] += fx; ++e_cnt[1]; }
@@ -188,7 +244,7 @@ __device__ __forceinline__ void dl_quantize_body(const float (&v)[DL_PER_THREAD]
                 }
             }
         }
-        if (q_aligned && (FULL || e0 + G - 1 < cnt)) {
+        if (q_aligned && e0 + G - 1 < cnt) {
             if (G == 4) *reinterpret_cast<uint32_t*>(q_chunk + e0) = w[0];
             else *reinterpret_cast<uint4*>(q_chunk + e0) = make_uint4(w[0], w[1 % (G / 4)], w[2 % (G / 4)], w[3 % (G / 4)]);
         } else {
@@ -208,7 +264,8 @@ __device__ __forceinline__ void dl_quantize_chunk(float (&v)[DL_PER_THREAD], lon
     for (int i = 0; i < DL_PER_THREAD; ++i) ss += v[i] * v[i];
     __syncthreads();                                         // the table's previous use (look-ups, last chunk's codebook) is over
     loaded();
-    for (int i = threadIdx.x; i < DL_TABLE; i += DL_THREADS) s_bin[i] = 0u;
+#pragma unroll
+    for (int i = 0; i < DL_TABLE / 4; i += DL_THREADS) reinterpret_cast<uint4*>(s_bin)[i + threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
     if (threadIdx.x < 2) { s_edge_sum[threadIdx.x] = 0ull; s_edge_cnt[threadIdx.x] = 0u; }
     ss = dl_block_sum(ss);                                   // also orders the zeroing above before the atomics below
     const float sigma = sqrtf(ss / float(cnt > 1 ? cnt - 1 : 1));
@@ -218,8 +275,8 @@ __device__ __forceinline__ void dl_quantize_chunk(float (&v)[DL_PER_THREAD], lon
     unsigned* my_bin = s_bin + (threadIdx.x & 31);
     long long e_sum[2] = {0ll, 0ll};
     unsigned e_cnt[2] = {0u, 0u};
-    if (cnt == DL_CHUNK) dl_quantize_body<G, true>(v, DL_CHUNK, q_chunk, q_aligned, my_bin, e_sum, e_cnt, inv_scale);
-    else dl_quantize_body<G, false>(v, int(cnt), q_chunk, q_aligned, my_bin, e_sum, e_cnt, inv_scale);
+    if (cnt == DL_CHUNK && ss < 3.0e38f) dl_quantize_finite<G>(v, q_chunk, q_aligned, my_bin, e_sum, e_cnt, inv_scale);
+    else dl_quantize_body<G>(v, int(cnt), q_chunk, q_aligned, my_bin, e_sum, e_cnt, inv_scale);
 #pragma unroll
     for (int b = 0; b < 2; ++b) {                            // one shared atomic per warp and clamping bin, and only if it has members
         unsigned c = e_cnt[b];
@@ -235,24 +292,26 @@ __device__ __forceinline__ void dl_quantize_chunk(float (&v)[DL_PER_THREAD], lon
         }
     }
     __syncthreads();
-    if (threadIdx.x < 256) {
-        const int b = threadIdx.x;
+    {
+        // two threads per bin, each over 16 of its copies
+        const int b = threadIdx.x >> 1, h = threadIdx.x & 1;
+        unsigned sum = 0, c = 0;
+#pragma unroll
+        for (int l = 0; l < 16; ++l) {
+            const unsigned x = s_bin[(b << 5) + ((16 * h + l + b) & 31)];     // rotated: a warp reads 32 different banks
+            c += x >> DL_CNT_SHIFT;
+            sum += x & ((1u << DL_CNT_SHIFT) - 1u);
+        }
+        c += __shfl_xor_sync(0xffffffffu, c, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         float mean = 0.f;
         if (b > 0 && b < 255) {
-            unsigned long long sum = 0;
-            unsigned c = 0;
-#pragma unroll
-            for (int l = 0; l < 32; ++l) {
-                const unsigned x = s_bin[(b << 5) + ((l + b) & 31)];      // rotated: the 32 bins of a warp read 32 different banks
-                c += x >> DL_CNT_SHIFT;
-                sum += x & ((1u << DL_CNT_SHIFT) - 1u);
-            }
             if (c) mean = (float(b) - 128.5f + float(double(sum) / double(1 << DL_FX_BITS) / double(c))) * scale;
         } else {
-            const unsigned c = s_edge_cnt[b ? 1 : 0];
+            c = s_edge_cnt[b ? 1 : 0];
             if (c) mean = float(double(static_cast<long long>(s_edge_sum[b ? 1 : 0])) / double(1 << DL_EDGE_FX_BITS) / double(c)) * scale;
         }
-        lut_chunk[b] = mean;
+        if (!h) lut_chunk[b] = mean;
     }
     __syncthreads();       // the shared table is reused by the CTA's next chunk
 }
@@ -276,7 +335,7 @@ __global__ void __launch_bounds__(DL_THREADS, 2) dl_stage_a_kernel(DlPeers p, co
     uint8_t* q = p.q[p.rank];
     float* lut = p.lut[p.rank];
     const bool q_aligned = (reinterpret_cast<uintptr_t>(q) & 3) == 0;
-    __shared__ unsigned s_tab[DL_TABLE];
+    __shared__ __align__(16) unsigned s_tab[DL_TABLE];
     extern __shared__ float4 s_next[];     // [DL_CHUNK / 4] without b
     const bool ahead = !HAS_B && aligned && !fake;
     auto fetch = [&](long long chunk) {    // whole chunks only; a ragged last one is loaded directly
@@ -338,7 +397,7 @@ __device__ __forceinline__ int dl_owner(unsigned mask, long long chunk, long lon
 // ---- stage B: pull every active rank's bytes for my chunks, dequantise with that rank's codebook, sum, re-quantise ----
 __global__ void __launch_bounds__(DL_THREADS, 2) dl_stage_b_kernel(DlPeers p, long long n, int epoch, int prev_epoch, unsigned* counter,
                                                                 int* status, unsigned long long budget_ns) {
-    __shared__ unsigned s_tab[DL_TABLE];   // histogram of the re-quantisation
+    __shared__ __align__(16) unsigned s_tab[DL_TABLE];   // histogram of the re-quantisation
     extern __shared__ float s_lut[];       // [world][256]: every active rank's codebook of the current chunk
     const long long chunks = (n + DL_CHUNK - 1) / DL_CHUNK;
     const int m = __popc(p.mask);
