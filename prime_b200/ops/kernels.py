@@ -175,7 +175,7 @@ def gemm_swiglu(x: torch.Tensor, w13: torch.Tensor, h13: torch.Tensor, act: torc
     back to GEMM + swiglu_fwd where the fused kernel does not apply (CPU, small or odd shapes)."""
     M, K = x.shape
     F = w13.shape[0] // 2
-    if x.is_cuda and _pair_ok(M, 2 * F) and F % 128 == 0 and h13.stride(-1) == 1 and act.stride(-1) == 1:
+    if x.is_cuda and _pair_ok(M, 2 * F) and F % 64 == 0 and h13.stride(-1) == 1 and act.stride(-1) == 1:
         _gemm_epi(x, w13, h13, M, 2 * F, K, False, 1, F, 0, 0, act, "swiglu")
         return h13, act
     gemm(x, w13, out=h13)
