@@ -6,81 +6,38 @@
 //   P  = exp2(S*c - lse2),  dS = P * (dP - D) -> bf16 in shared memory (softmax warps)
 //   dV += P^T dO,  dK += dS^T Q               -> TMEM accumulators kept for the whole item
 //   dQ  = dS K                                -> TMEM -> shared memory -> bulk reduce-add (TMA) into dq_acc
-// For head size 64 the pairs are software-pipelined: the tensor core computes S/dP of pair i+1 and dV/dK/dQ of
-// pair i-1 while the softmax warps work on pair i from registers.
+// Heads of up to 64 columns (the kernel for wider ones is in attn_bwd128_sm100.cu). The pairs are software-pipelined: the tensor
+// core computes S/dP of pair i+1 and dV/dK/dQ of pair i-1 while the softmax warps work on pair i from registers.
 // D[h, m] = rowsum(dO * O) comes from a small pre-pass. dK/dV of a KV head are reduced over the
 // query heads of its group inside the CTA (no repeat_kv materialisation, no cross-CTA atomics
 // for them). The same shared-memory tile is consumed K-major by one MMA and MN-major by another
 // (e.g. Q is A of S and B of dK), which the 128-byte-swizzled layout allows without a copy.
 // Gradient semantics match autograd through the reference attention
 // (models/llama/model.py:282-302) for scores scaled by `scale`.
-#include "common.cuh"
+#include "attn_bwd.cuh"
 
 namespace pb {
 
-struct AttnBwdParams {
-    int M, H, KV, n_tiles;
-    int hd;                // columns of a head, <= HD (narrower heads are zero-filled by the tensor maps)
-    const int* seq_start;
-    const float* lse2;     // [H, M]
-    const float* D;        // [H, M]
-    float* dq_acc;         // [M, H*hd] fp32, zeroed by the span pre-pass of the same call
-    __nv_bfloat16* dqkv;   // [M, (H+2KV)*hd]; the backward kernel writes the k and v column blocks
-    long long dqkv_stride;
-    float scale, scale_log2;
-    int* status;
-    // query-tile count per kv tile (set by a pre-pass of the launch) and work-item count (= n_tiles * KV)
-    int* nq;
-    int n_items;
-    int* counter;          // the global work counter (next item number)
-};
-
-template <int HD>
 struct AttnBwdCfg {
+    static constexpr int HD = 64;
     static constexpr int TILE_BYTES = 128 * HD * 2;
     static constexpr int PS_BYTES = 128 * 128 * 2;
-    static constexpr int STAGES = (HD == 64) ? 3 : 1;
-    // HD=64: S/dP of pair it+1 are issued as soon as the softmax warps hold pair it in registers
-    static constexpr bool PIPE = (HD == 64);
+    static constexpr int STAGES = 3;
     static constexpr int DQ_STAGE_BYTES = 8 * 4096;   // one 32-row x 32-float box per softmax warp
     static constexpr int SMEM_BYTES = TILE_BYTES * (2 + 2 * STAGES) + 2 * PS_BYTES + DQ_STAGE_BYTES + 1024 + 256;
     static constexpr int T_S = 0, T_DP = 128;
-    static constexpr int T_DV = 256, T_DK = 256 + HD;
-    static constexpr int T_DQ = (HD == 64) ? 384 : 0;   // HD=128: dQ reuses the S columns
-    static constexpr bool DQ_ALIASES_S = (HD != 64);
+    static constexpr int T_DV = 256, T_DK = 256 + HD, T_DQ = 384;
 };
-
-__device__ __forceinline__ void reg_dealloc_64() { asm volatile("setmaxnreg.dec.sync.aligned.u32 64;"); }
-__device__ __forceinline__ void reg_dealloc_88() { asm volatile("setmaxnreg.dec.sync.aligned.u32 88;"); }
-__device__ __forceinline__ void reg_alloc_176() { asm volatile("setmaxnreg.inc.sync.aligned.u32 176;"); }
-
-// A work item is one (kv tile, kv head). The grid is one CTA per SM; every CTA draws items from a global counter
-// (the producer warp does, and hands the numbers to the other warps through a four-entry ring in shared memory), so
-// barriers, tensor memory and the Q/dO ring are set up once per SM and the next item's K/V/Q/dO loads run under the
-// current item's dK/dV write-out. Items are numbered head by head, kv tiles in row order, so the CTAs that run at the
-// same time share Q, dO and the dQ accumulator rows in L2.
-struct BwdItem {
-    int kv_tile, g;
-};
-
-__device__ __forceinline__ BwdItem bwd_item_of(const AttnBwdParams& p, int idx) {
-    BwdItem it;
-    it.g = idx / p.n_tiles;
-    it.kv_tile = idx - it.g * p.n_tiles;
-    return it;
-}
 
 // 512 threads in four warpgroups (register budgets are re-split with setmaxnreg):
 //   warps 0-3   : warp 0 = TMA producer, warp 1 = MMA issuer (2 and 3 only hold the warpgroup together)
 //   warps 4-11  : softmax warps; warp w reads TMEM lane quadrant w & 3 and column half (w - 4) >> 2
 //   warps 12-15 : dQ drain warps; warp w moves the 32 query rows of quadrant w & 3 to dq_acc
-template <int HD>
 __global__ void __launch_bounds__(512, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant__ CUtensorMap tmDO,
                 const __grid_constant__ CUtensorMap tmDQ, const AttnBwdParams p) {
-    using Cfg = AttnBwdCfg<HD>;
-    constexpr int NB = HD / 64;
-    constexpr int STAGES = Cfg::STAGES;
+    using Cfg = AttnBwdCfg;
+    constexpr int HD = Cfg::HD, STAGES = Cfg::STAGES;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -165,11 +122,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                 }
                 if (lane == 0) {
                     mbar_expect_tx(bar_kv, 2 * Cfg::TILE_BYTES);
-#pragma unroll
-                    for (int b = 0; b < NB; ++b) {
-                        tma_load_3d(sK + b * 16384, &tmQKV, bar_kv, 64 * b, p.H + item.g, kv0);
-                        tma_load_3d(sV + b * 16384, &tmQKV, bar_kv, 64 * b, p.H + p.KV + item.g, kv0);
-                    }
+                    tma_load_3d(sK, &tmQKV, bar_kv, 0, p.H + item.g, kv0);
+                    tma_load_3d(sV, &tmQKV, bar_kv, 0, p.H + p.KV + item.g, kv0);
                 }
                 int hq = item.g * G, qi = 0;
                 const int n_it = n_q * G;
@@ -182,12 +136,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                     if (lane == 0) {
                         const int q0 = (item.kv_tile + qi) * 128;
                         mbar_expect_tx(bar_qfull + 8 * st, 2 * Cfg::TILE_BYTES);   // Q and dO land on one barrier
-#pragma unroll
-                        for (int b = 0; b < NB; ++b)
-                            tma_load_3d(sQ + st * Cfg::TILE_BYTES + b * 16384, &tmQKV, bar_qfull + 8 * st, 64 * b, hq, q0);
-#pragma unroll
-                        for (int b = 0; b < NB; ++b)
-                            tma_load_3d(sDO + st * Cfg::TILE_BYTES + b * 16384, &tmDO, bar_qfull + 8 * st, 64 * b, hq, q0);
+                        tma_load_3d(sQ + st * Cfg::TILE_BYTES, &tmQKV, bar_qfull + 8 * st, 0, hq, q0);
+                        tma_load_3d(sDO + st * Cfg::TILE_BYTES, &tmDO, bar_qfull + 8 * st, 0, hq, q0);
                     }
                     __syncwarp();
                     if (++qi == n_q) { qi = 0; ++hq; }
@@ -219,22 +169,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                         ok = mbar_wait(bar_qfull + 8 * st, ph, abort_flag, p.status, PB_ERR_TIMEOUT_FULL);
                         if (!ok) return false;
                     }
-                    if (Cfg::DQ_ALIASES_S && gi > 0) {
-                        ok = mbar_wait(bar_dqempty, (gi - 1) & 1, abort_flag, p.status, PB_ERR_TIMEOUT_TMEM_EMPTY);
-                        if (!ok) return false;
-                    }
                     tc_fence_after();
                     const uint32_t q = sQ + st * Cfg::TILE_BYTES, d = sDO + st * Cfg::TILE_BYTES;
-                    uint32_t got = 0;
-#pragma unroll
-                    for (int b = 0; b < NB; ++b)
-                        umma4_f16_ss_peek(tS, umma_smem_desc(q + b * 16384, 16, 1024), umma_smem_desc(sK + b * 16384, 16, 1024), 2, 2,
-                                          idesc_s, b ? 1u : 0u, 0, 0, 0, 0, 0, 0, 0);
-#pragma unroll
-                    for (int b = 0; b < NB; ++b)
-                        got |= umma4_f16_ss_peek(tDP, umma_smem_desc(d + b * 16384, 16, 1024), umma_smem_desc(sV + b * 16384, 16, 1024), 2, 2,
-                                                 idesc_s, b ? 1u : 0u, b == NB - 1 ? bar_sdpfull : 0, 0, 0,
-                                                 b == NB - 1 ? peek : 0, par, 0, 0);
+                    umma4_f16_ss_peek(tS, umma_smem_desc(q, 16, 1024), umma_smem_desc(sK, 16, 1024), 2, 2, idesc_s, 0u, 0, 0, 0, 0, 0, 0, 0);
+                    const uint32_t got = umma4_f16_ss_peek(tDP, umma_smem_desc(d, 16, 1024), umma_smem_desc(sV, 16, 1024), 2, 2, idesc_s, 0u,
+                                                           bar_sdpfull, 0, 0, peek, par, 0, 0);
                     return got & 1;
                 };
                 uint32_t gi = 0;      // running pair count over all items of this CTA
@@ -244,7 +183,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                     const int n_it = p.nq[bwd_item_of(p, idx).kv_tile] * G;
                     ok = mbar_wait(bar_kv, k & 1, abort_flag, p.status, PB_ERR_TIMEOUT_FULL);
                     if (!ok) break;
-                    if (Cfg::PIPE && gi > 0) {   // the softmax warps hold the previous item's last pair in registers (long since)
+                    if (gi > 0) {   // the softmax warps hold the previous item's last pair in registers (long since)
                         ok = mbar_wait(bar_sdpfree, (gi - 1) & 1, abort_flag, p.status, PB_ERR_TIMEOUT_TMEM_EMPTY);
                         if (!ok) break;
                     }
@@ -253,7 +192,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                     for (int it = 0; it < n_it && ok; ++it, ++gi) {
                         const int st = gi % STAGES;
                         bool pds_ready = false;
-                        if (Cfg::PIPE && it + 1 < n_it) {
+                        if (it + 1 < n_it) {
                             if (!sdpfree_ready) {
                                 ok = mbar_wait(bar_sdpfree, gi & 1, abort_flag, p.status, PB_ERR_TIMEOUT_TMEM_EMPTY);
                                 if (!ok) break;
@@ -267,7 +206,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                         }
                         tc_fence_after();
                         const uint32_t q = sQ + st * Cfg::TILE_BYTES, d = sDO + st * Cfg::TILE_BYTES;
-                        const bool wait_dqe = !Cfg::DQ_ALIASES_S && gi > 0;   // the drain warps have read dQ of the previous pair
+                        const bool wait_dqe = gi > 0;   // the drain warps have read dQ of the previous pair
                         uint32_t got = 0;
                         // dV += P^T dO, dK += dS^T Q: reduction over the 128 query rows, 16 per MMA; the first pair of an
                         // item starts new accumulators (the softmax warps wrote the previous item's dK/dV out before they
@@ -287,18 +226,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                         }
                         if (wait_dqe) tc_fence_after();
                         // dQ = dS K: reduction over the 128 kv rows. Meanwhile poll what the next iteration needs first.
-                        const int nx = Cfg::PIPE ? it + 2 : it + 1;            // pair (of this item) whose Q/dO stage is needed next
-                        const uint32_t gnx = gi + (Cfg::PIPE ? 2 : 1);
-                        const bool peek_q = nx < n_it;
-                        const bool peek_free = Cfg::PIPE && it + 2 < n_it;
+                        const uint32_t gnx = gi + 2;                           // pair whose Q/dO stage is needed next
+                        const bool more = it + 2 < n_it;                       // ... if it is one of this item
                         got = umma4_f16_ss_peek(tDQ, umma_smem_desc(sDS, 16, 1024), umma_smem_desc(sK, 16384, 1024), 2, 128, idesc_dq, 0u,
-                                                0, 0, 0, peek_q ? bar_qfull + 8 * (gnx % STAGES) : 0, (gnx / STAGES) & 1,
-                                                peek_free ? bar_sdpfree : 0, (gi + 1) & 1);
+                                                0, 0, 0, more ? bar_qfull + 8 * (gnx % STAGES) : 0, (gnx / STAGES) & 1,
+                                                more ? bar_sdpfree : 0, (gi + 1) & 1);
                         umma4_f16_ss_peek(tDQ, umma_smem_desc(sDS + 16384, 16, 1024), umma_smem_desc(sK + 8192, 16384, 1024), 2, 128, idesc_dq,
                                           1u, bar_dqfull, bar_qdoempty + 8 * st, it == n_it - 1 ? bar_final : 0, 0, 0, 0, 0);
                         qnext_ready = got & 1;
                         sdpfree_ready = got & 2;
-                        if (!Cfg::PIPE && it + 1 < n_it) issue_s_dp(gi + 1, qnext_ready, 0, 0);
                     }
                 }
             }
@@ -328,33 +264,22 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                 if (!ok) break;
                 tc_fence_after();
                 const int dq_y = (item.kv_tile + qi) * 128 + quad * 32;
-#pragma unroll 1
-                for (int c0 = 0; c0 < HD; c0 += 64) {
-                    uint32_t v[64];
-                    tmem_ld32(tDQ + c0, *reinterpret_cast<uint32_t(*)[32]>(v));
-                    tmem_ld32(tDQ + c0 + 32, *reinterpret_cast<uint32_t(*)[32]>(v + 32));
-                    if (lane == 0) tma_store_wait_read<0>();   // earlier reduce-adds have read the staging boxes
-                    __syncwarp();
-                    tmem_ld_wait();
-                    if (c0 + 64 >= HD) {   // dQ of this pair is out of TMEM
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_dqempty);
-                    }
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) {
-                        float4 f;
-                        f.x = __uint_as_float(v[4 * q]) * p.scale;     f.y = __uint_as_float(v[4 * q + 1]) * p.scale;
-                        f.z = __uint_as_float(v[4 * q + 2]) * p.scale; f.w = __uint_as_float(v[4 * q + 3]) * p.scale;
-                        *reinterpret_cast<float4*>(g_dq + (q >> 3) * 4096 + lane * 128 + (((q & 7) ^ (lane & 7)) << 4)) = f;
-                    }
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) {
-                        if (c0 < p.hd) tma_reduce_add_3d(&tmDQ, my_dq, c0, hq, dq_y);
-                        if (c0 + 32 < p.hd) tma_reduce_add_3d(&tmDQ, my_dq + 4096, c0 + 32, hq, dq_y);
-                        tma_store_commit();
-                    }
+                uint32_t v[64];
+                tmem_ld32(tDQ, *reinterpret_cast<uint32_t(*)[32]>(v));
+                tmem_ld32(tDQ + 32, *reinterpret_cast<uint32_t(*)[32]>(v + 32));
+                if (lane == 0) tma_store_wait_read<0>();   // earlier reduce-adds have read the staging boxes
+                __syncwarp();
+                tmem_ld_wait();
+                tc_fence_before();                         // dQ of this pair is out of TMEM
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_dqempty);
+                bwd_stage_dq(g_dq, v, lane, p.scale);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_reduce_add_3d(&tmDQ, my_dq, 0, hq, dq_y);
+                    if (p.hd > 32) tma_reduce_add_3d(&tmDQ, my_dq + 4096, 32, hq, dq_y);
+                    tma_store_commit();
                 }
                 if (++qi == n_q) { qi = 0; ++hq; }
             }
@@ -374,24 +299,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         const float c = p.scale_log2;
         bool ok = true;
         // Per (head, query tile) pair: this thread's row constants, then its 64 S and 64 dP values in
-        // registers. With Cfg::PIPE the pair after the one being exponentiated is already in TMEM.
-        struct RowCtx {
-            float lse, Dr;
-            int my_start;
-            int q0, tile_last_start;
-        };
+        // registers. The pair after the one being exponentiated is already in TMEM.
         // (query head, query tile) of the pair whose row constants are loaded next, inside the current item
         int kv_tile = 0, n_q = 0, hq_n = 0, qi_n = 0;
         auto row_ctx = [&]() {
-            RowCtx x;
-            const int q0 = (kv_tile + qi_n) * 128;
-            const int row = q0 + r;
-            const bool row_ok = row < p.M;
-            x.lse = row_ok ? p.lse2[(long long)hq_n * p.M + row] : 0.f;
-            x.Dr = row_ok ? p.D[(long long)hq_n * p.M + row] : 0.f;
-            x.my_start = row_ok ? p.seq_start[row] : 0x7fffffff;   // a row past M sees no kv position
-            x.q0 = q0;
-            x.tile_last_start = p.seq_start[min(q0 + 127, p.M - 1)];
+            const BwdRow x = bwd_row(p, hq_n, kv_tile + qi_n, r);
             if (++qi_n == n_q) { qi_n = 0; ++hq_n; }
             return x;
         };
@@ -406,14 +318,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
             tmem_ld32(tDP + half * 64, *reinterpret_cast<uint32_t(*)[32]>(dv));
             tmem_ld32(tDP + half * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(dv + 32));
             tmem_ld_wait();
-            if (Cfg::PIPE) {
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_sdpfree);
-            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_sdpfree);
             return true;
         };
-        RowCtx cur = {}, nxt = {};
+        BwdRow cur = {}, nxt = {};
         uint32_t gi = 0;
         BwdItem item = {};
         int idx = items.take(0);
@@ -432,50 +342,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                 --left;
                 if (left) nxt = row_ctx();      // global loads land while this pair is exponentiated
                 const int row = cur.q0 + r;
-                // Exponentials are taken two at a time on packed bf16 pairs (ex2.approx.bf16x2): the result is
-                // P as the MMA will read it, and dS is formed from those same rounded values.
-                const bool need_mask = (kv0 + 127 > cur.q0) || (kv0 < cur.tile_last_start) || (cur.q0 + 127 >= p.M);
-                if (need_mask) {
-#pragma unroll
-                    for (int i = 0; i < 64; i += 2) {
-                        const int s0 = kv0 + half * 64 + i;
-                        float x0 = __uint_as_float(sv[i]) * c - cur.lse;
-                        float x1 = __uint_as_float(sv[i + 1]) * c - cur.lse;
-                        if (s0 > row || s0 < cur.my_start) x0 = -INFINITY;
-                        if (s0 + 1 > row || s0 + 1 < cur.my_start) x1 = -INFINITY;
-                        uint32_t e;
-                        asm("ex2.approx.ftz.bf16x2 %0, %1;" : "=r"(e) : "r"(pack_bf16x2(x0, x1)));
-                        const float d0 = __uint_as_float(e << 16) * (__uint_as_float(dv[i]) - cur.Dr);
-                        const float d1 = __uint_as_float(e & 0xffff0000u) * (__uint_as_float(dv[i + 1]) - cur.Dr);
-                        sv[i >> 1] = e;
-                        dv[i >> 1] = pack_bf16x2(d0, d1);
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 64; i += 2) {
-                        const float x0 = __uint_as_float(sv[i]) * c - cur.lse;
-                        const float x1 = __uint_as_float(sv[i + 1]) * c - cur.lse;
-                        uint32_t e;
-                        asm("ex2.approx.ftz.bf16x2 %0, %1;" : "=r"(e) : "r"(pack_bf16x2(x0, x1)));
-                        const float d0 = __uint_as_float(e << 16) * (__uint_as_float(dv[i]) - cur.Dr);
-                        const float d1 = __uint_as_float(e & 0xffff0000u) * (__uint_as_float(dv[i + 1]) - cur.Dr);
-                        sv[i >> 1] = e;
-                        dv[i >> 1] = pack_bf16x2(d0, d1);
-                    }
-                }
+                if (bwd_needs_mask(p, cur, kv0)) bwd_probs<true>(sv, cur, row, kv0 + half * 64, c);
+                else bwd_probs<false>(sv, cur, row, kv0 + half * 64, c);
+                bwd_dscores(sv, dv, cur.Dr);
                 if (gi > 0) {
                     // the MMAs of the previous pair have read its P/dS out of shared memory
                     ok = mbar_wait(bar_dqfull, (gi - 1) & 1, abort_flag, p.status, PB_ERR_TIMEOUT_TMEM_FULL);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                 }
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int chunk = half * 8 + q;
-                    const uint32_t off = (chunk >> 3) * 16384 + r * 128 + (((chunk & 7) ^ (r & 7)) << 4);
-                    *reinterpret_cast<uint4*>(gP + off) = make_uint4(sv[4 * q], sv[4 * q + 1], sv[4 * q + 2], sv[4 * q + 3]);
-                    *reinterpret_cast<uint4*>(gDS + off) = make_uint4(dv[4 * q], dv[4 * q + 1], dv[4 * q + 2], dv[4 * q + 3]);
-                }
+                bwd_store_half(gP, sv, half, r);
+                bwd_store_half(gDS, dv, half, r);
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_pdsfull);
@@ -498,33 +375,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                 cur = row_ctx();
             }
             tc_fence_after();
-            const int row = kv0 + r;
-            __nv_bfloat16* dk_row = p.dqkv + (long long)row * p.dqkv_stride + (p.H + g) * p.hd;
-            __nv_bfloat16* dv_row = p.dqkv + (long long)row * p.dqkv_stride + (p.H + p.KV + g) * p.hd;
-#pragma unroll 1
-            for (int cidx = half * (HD / 2); cidx < (half + 1) * (HD / 2); cidx += 32) {
-                uint32_t a[32], b[32];
-                tmem_ld32(tDK + cidx, a);
-                tmem_ld32(tDV + cidx, b);
-                tmem_ld_wait();
-                if (row < p.M) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        if (cidx + i >= p.hd) break;
-                        uint4 u, w;
-                        u.x = pack_bf16x2(__uint_as_float(a[i]) * p.scale, __uint_as_float(a[i + 1]) * p.scale);
-                        u.y = pack_bf16x2(__uint_as_float(a[i + 2]) * p.scale, __uint_as_float(a[i + 3]) * p.scale);
-                        u.z = pack_bf16x2(__uint_as_float(a[i + 4]) * p.scale, __uint_as_float(a[i + 5]) * p.scale);
-                        u.w = pack_bf16x2(__uint_as_float(a[i + 6]) * p.scale, __uint_as_float(a[i + 7]) * p.scale);
-                        w.x = pack_bf16x2(__uint_as_float(b[i]), __uint_as_float(b[i + 1]));
-                        w.y = pack_bf16x2(__uint_as_float(b[i + 2]), __uint_as_float(b[i + 3]));
-                        w.z = pack_bf16x2(__uint_as_float(b[i + 4]), __uint_as_float(b[i + 5]));
-                        w.w = pack_bf16x2(__uint_as_float(b[i + 6]), __uint_as_float(b[i + 7]));
-                        *reinterpret_cast<uint4*>(dk_row + cidx + i) = u;
-                        *reinterpret_cast<uint4*>(dv_row + cidx + i) = w;
-                    }
-                }
-            }
+            bwd_write_dkdv<HD>(p, tDK, tDV, kv0 + r, g, half);
             tc_fence_before();
         }
     }
@@ -580,49 +431,31 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
     }
 }
 
-// dq (fp32 accumulator, [M, H*HD]) -> inverse RoPE -> bf16 q columns of dqkv. In the same pass the
-// k columns of dqkv (already bf16, written by the backward kernel) get their inverse RoPE in place.
+// dq (fp32 accumulator, [M, H*HD]) -> inverse RoPE -> bf16 q columns of dqkv
 __global__ void attn_bwd_finish_kernel(const float* __restrict__ dq_acc, __nv_bfloat16* __restrict__ dqkv,
-                                       const float* __restrict__ table, long long M, int T, int H, int KV, int HD,
-                                       long long stride, int apply_rope) {
+                                       const float* __restrict__ table, long long M, int T, int H, int HD, long long stride) {
     pdl_sync();
-    const int vph = HD / 8;
-    const long long total = M * (H + KV) * vph;
+    const int vpr = H * HD / 8, vph = HD / 8;
+    const long long total = M * vpr;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int v = int(i % vph);
-        const long long t = i / vph;
-        const int h = int(t % (H + KV));
-        const long long m = t / (H + KV);
-        float f[8];
-        __nv_bfloat16* dst = dqkv + m * stride + h * HD + v * 8;
-        if (h < H) {
-            const float4* src = reinterpret_cast<const float4*>(dq_acc + m * (H * HD) + h * HD + v * 8);
-            const float4 a = src[0], b = src[1];
-            f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-        } else {
-            const uint4 u = *reinterpret_cast<const uint4*>(dst);
-            float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), cc = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
-            f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = cc.x; f[5] = cc.y; f[6] = d.x; f[7] = d.y;
-        }
-        float o[8];
-        if (apply_rope) {
-            const int pos = int(m % T);
-            const float4* cs = reinterpret_cast<const float4*>(table + ((long long)pos * (HD / 2) + v * 4) * 2);
+        const long long m = i / vpr;
+        const int c = int(i - m * vpr);
+        const float4* src = reinterpret_cast<const float4*>(dq_acc + 8 * i);
+        const float4 a = src[0], b = src[1];
+        const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        uint32_t u[4];
+        if (table) {
+            const float4* cs = reinterpret_cast<const float4*>(table + (m % T) * HD + (c % vph) * 8);
             const float4 c0 = cs[0], c1 = cs[1];
-            const float co[4] = {c0.x, c0.z, c1.x, c1.z};
-            const float si[4] = {-c0.y, -c0.w, -c1.y, -c1.w};
+            const float co[4] = {c0.x, c0.z, c1.x, c1.z}, si[4] = {c0.y, c0.w, c1.y, c1.w};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                o[2 * k] = f[2 * k] * co[k] - f[2 * k + 1] * si[k];
-                o[2 * k + 1] = f[2 * k] * si[k] + f[2 * k + 1] * co[k];
-            }
+            for (int k = 0; k < 4; ++k)
+                u[k] = pack_bf16x2(f[2 * k] * co[k] + f[2 * k + 1] * si[k], f[2 * k + 1] * co[k] - f[2 * k] * si[k]);
         } else {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) o[k] = f[k];
+            for (int k = 0; k < 4; ++k) u[k] = pack_bf16x2(f[2 * k], f[2 * k + 1]);
         }
-        uint4 u;
-        u.x = pack_bf16x2(o[0], o[1]); u.y = pack_bf16x2(o[2], o[3]); u.z = pack_bf16x2(o[4], o[5]); u.w = pack_bf16x2(o[6], o[7]);
-        *reinterpret_cast<uint4*>(dst) = u;
+        *reinterpret_cast<uint4*>(dqkv + m * stride + c * 8) = make_uint4(u[0], u[1], u[2], u[3]);
     }
 }
 
@@ -652,39 +485,37 @@ __global__ void __launch_bounds__(256) attn_bwd_span_kernel(const int* __restric
     if (lane == 0) nq[kv_tile] = n_q;
 }
 
-int sm_count();
 int make_tmap_heads(CUtensorMap* out, const void* ptr, int elem_bytes, uint64_t hd, uint64_t n_heads, uint64_t outer, uint64_t ld,
                     uint32_t box_inner, uint32_t box_outer);
 
-template <int HD>
-static int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tdq, const AttnBwdParams& p,
-                           cudaStream_t st) {
-    using Cfg = AttnBwdCfg<HD>;
-    auto kern = attn_bwd_kernel<HD>;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess) return -20;
-        configured = true;
-    }
-    const int grid = p.n_items < sm_count() ? p.n_items : sm_count();     // one CTA per SM draws items until none are left
+static void launch_span(const AttnBwdParams& p, cudaStream_t st) {
     const long long n16 = (long long)p.M * p.H * p.hd / 4;                // a head is a multiple of 8 columns
     long long blocks = (n16 + 1023) / 1024;                               // four stores per thread, at most 8 CTAs per SM ...
     if (blocks > 148 * 8) blocks = 148 * 8;
     if (blocks < (p.n_tiles + 7) / 8) blocks = (p.n_tiles + 7) / 8;       // ... and a warp for every kv tile
     launch_pdl(attn_bwd_span_kernel, LaunchCfg(unsigned(blocks), 256, 0, st).traffic(16.0 * n16), p.seq_start, p.n_tiles, p.nq, p.counter,
                reinterpret_cast<uint4*>(p.dq_acc), n16);
-    launch_pdl(kern, LaunchCfg(grid, 512, Cfg::SMEM_BYTES, st), tq, tdo, tdq, p);
+}
+
+static int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const CUtensorMap& tdq, const AttnBwdParams& p, cudaStream_t st) {
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnBwdCfg::SMEM_BYTES) != cudaSuccess) return -20;
+        configured = true;
+    }
+    const int grid = p.n_items < sm_count() ? p.n_items : sm_count();     // one CTA per SM draws items until none are left
+    launch_pdl(attn_bwd_kernel, LaunchCfg(grid, 512, AttnBwdCfg::SMEM_BYTES, st), tq, tdo, tdq, p);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }
 
 }  // namespace pb
 
 // dq_acc: fp32 [M, H*HD] scratch (zeroed here); D: fp32 [H, M] scratch, computed here from o and dout unless o is
-// null (then the caller has already filled it). Writes all of dqkv.
+// null (then the caller has already filled it with [H, d_parts, M] partial sums). Writes all of dqkv.
 // rope_table != null: the inverse rotation is applied to dq and dk on the way out (position = row % T).
 // tile_scratch: >= ceil(M / 128) + 1 ints of device scratch (query-tile count of every kv tile and the work counter).
 extern "C" int pb_attn_bwd(const void* qkv, const void* o, const void* dout, const float* lse2, const int* seq_start,
-                           void* dqkv, float* dq_acc, float* D, const float* rope_table, int T, int M, int H, int KV, int HD,
+                           void* dqkv, float* dq_acc, float* D, int d_parts, const float* rope_table, int T, int M, int H, int KV, int HD,
                            long long qkv_stride, long long o_stride, long long do_stride, long long dqkv_stride, float scale,
                            int* tile_scratch, int* status, void* stream) {
     using namespace pb;
@@ -716,14 +547,16 @@ extern "C" int pb_attn_bwd(const void* qkv, const void* o, const void* dout, con
     p.M = M; p.H = H; p.KV = KV; p.hd = HD; p.n_tiles = (M + 127) / 128; p.seq_start = seq_start; p.lse2 = lse2; p.D = D;
     p.dq_acc = dq_acc; p.dqkv = reinterpret_cast<__nv_bfloat16*>(dqkv); p.dqkv_stride = dqkv_stride;
     p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
+    p.d_parts = o ? 1 : d_parts; p.rope = rope_table; p.T = T;
     if (tile_scratch == nullptr) return -3;
     p.nq = tile_scratch; p.counter = tile_scratch + p.n_tiles; p.n_items = p.n_tiles * KV;
-    rc = HD <= 64 ? launch_attn_bwd<64>(tq, tdo, tdq, p, st) : launch_attn_bwd<128>(tq, tdo, tdq, p, st);
+    launch_span(p, st);
+    rc = HD <= 64 ? launch_attn_bwd(tq, tdo, tdq, p, st) : launch_attn_bwd128(tq, tdo, tdq, p, st);
     if (rc) return rc;
-    const long long total = (long long)M * (H + KV) * (HD / 8);
+    const long long total = (long long)M * H * (HD / 8);
     long long blocks = (total + 255) / 256;
     if (blocks > 148 * 8) blocks = 148 * 8;
-    launch_pdl(attn_bwd_finish_kernel, LaunchCfg(unsigned(blocks), 256, 0, st).traffic(6.0 * M * H * HD), dq_acc, (__nv_bfloat16*)dqkv, rope_table, M, T, H, KV, HD, dqkv_stride,
-                                                              rope_table != nullptr);
+    launch_pdl(attn_bwd_finish_kernel, LaunchCfg(unsigned(blocks), 256, 0, st).traffic(6.0 * M * H * HD), dq_acc, (__nv_bfloat16*)dqkv, rope_table, M, T, H, HD,
+               dqkv_stride);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }

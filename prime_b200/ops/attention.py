@@ -19,7 +19,7 @@ from .kernels import _scratch_buf, status_word
 native.register_cuda_sigs({
     "pb_attn_fwd": [native.vp, native.vp, native.vp, native.vp, native.i32, native.i32, native.i32, native.i32,
                     native.i64, native.i64, native.f32, native.vp, native.vp],
-    "pb_attn_bwd": [native.vp] * 9 + [native.i32] * 5 + [native.i64] * 4 + [native.f32, native.vp, native.vp, native.vp],
+    "pb_attn_bwd": [native.vp] * 8 + [native.i32, native.vp] + [native.i32] * 5 + [native.i64] * 4 + [native.f32, native.vp, native.vp, native.vp],
 })
 
 
@@ -151,9 +151,9 @@ def attention_fwd(qkv: torch.Tensor, seq_start: torch.Tensor, H: int, KV: int, h
     return out if o is out else out.copy_(o), lse2
 
 
-def row_dots_buffer(device, M: int, H: int) -> torch.Tensor:
-    """fp32 [H * M] scratch for the dO . O row sums (shared with the backward kernel's own pre-pass)."""
-    return _scratch_buf(device, "attn_D", M * H)
+def row_dots_buffer(device, M: int, H: int, parts: int = 1) -> torch.Tensor:
+    """fp32 [H * parts * M] scratch for the dO . O row sums (shared with the backward kernel's own pre-pass)."""
+    return _scratch_buf(device, "attn_D", M * H * parts)[: M * H * parts]
 
 
 def attention_bwd(qkv: torch.Tensor, o: torch.Tensor, dout: torch.Tensor, lse2: torch.Tensor, seq_start: torch.Tensor,
@@ -161,8 +161,9 @@ def attention_bwd(qkv: torch.Tensor, o: torch.Tensor, dout: torch.Tensor, lse2: 
                   rope_table: torch.Tensor | None = None, seq_len: int = 0, row_dots: torch.Tensor | None = None):
     """Gradient of the fused qkv buffer. With ``rope_table`` the inverse rotation of dq and dk is
     folded into the final pass (so the result is the gradient w.r.t. the *unrotated* projection).
-    ``row_dots`` ([H, M] fp32 = sum over a head's columns of dout * o), when the caller already has it
-    (``kernels.gemm_rowdot``), replaces the kernel's own pre-pass over ``o`` and ``dout``."""
+    ``row_dots`` (fp32 [H, M] = sum over a head's columns of dout * o, or [H, 2, M] for heads of 128 columns = the sums over
+    either half of them), when the caller already has it (``kernels.gemm_rowdot``), replaces the kernel's own pre-pass over ``o``
+    and ``dout``."""
     M = qkv.shape[0]
     scale = scale if scale is not None else hd ** -0.5
     if dqkv is None:
@@ -182,10 +183,11 @@ def attention_bwd(qkv: torch.Tensor, o: torch.Tensor, dout: torch.Tensor, lse2: 
         return _dense_bwd(qkv, dout, seq_start, H, KV, hd, scale, dqkv, rope_table, seq_len)
     dq_acc = _scratch_buf(qkv.device, "attn_dq", M * H * hd)
     D = row_dots if row_dots is not None else _scratch_buf(qkv.device, "attn_D", M * H)
+    d_parts = 2 if row_dots is not None and hd == 128 and row_dots.numel() == 2 * M * H else 1
     tiles = _scratch_buf(qkv.device, "attn_tiles", (M + 127) // 128 + 1, torch.int32)
     assert rope_table is None or seq_len > 0
     qkv, o, dout, g = _fitting_input(qkv, hd), _fitting_input(o, hd), _fitting_input(dout, hd), _fitting_output(dqkv, hd)
-    check(native.cuda().pb_attn_bwd(ptr(qkv), ptr(o) if row_dots is None else None, ptr(dout), ptr(lse2), ptr(seq_start), ptr(g), ptr(dq_acc), ptr(D),
+    check(native.cuda().pb_attn_bwd(ptr(qkv), ptr(o) if row_dots is None else None, ptr(dout), ptr(lse2), ptr(seq_start), ptr(g), ptr(dq_acc), ptr(D), d_parts,
                                     ptr(rope_table), max(int(seq_len), 1), M, H, KV, hd, qkv.stride(0),
                                     o.stride(0), dout.stride(0), g.stride(0), scale, ptr(tiles), ptr(status_word(qkv.device)),
                                     stream_ptr()), "pb_attn_bwd")
