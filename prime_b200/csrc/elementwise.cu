@@ -613,12 +613,24 @@ extern "C" int pb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd
 // number of CTAs (= rows of the fp32 partial buffer [ctas, N]) the backward uses at most
 extern "C" int pb_rmsnorm_bwd_ctas() { return 148 * 2; }
 
+static int rmsnorm_bwd_used_ctas(int M, int N) {
+    const int rows_per_cta = N <= 1024 ? 8 : N <= 2048 ? 4 : 2;      // of one iteration; a CTA without rows would only add a zero partial
+    return std::max(1, std::min(pb_rmsnorm_bwd_ctas(), (M + rows_per_cta - 1) / rows_per_cta));
+}
+
+// The second half of pb_rmsnorm_bwd by itself: the weight gradient from the partial sums that pb_rmsnorm_bwd left for M rows of N
+// columns when it was given no dw.
+extern "C" int pb_rmsnorm_bwd_dw(const float* dw_partial, void* dw, int dw_fp32, int dw_accumulate, int M, int N, void* stream) {
+    launch_pdl(colsum_partials_kernel, LaunchCfg((N + 31) / 32, 32 * COLSUM_GROUPS, 0, ST(stream)), dw_partial, dw, rmsnorm_bwd_used_ctas(M, N), N,
+               dw_fp32, dw_accumulate);
+    return CHECK_LAUNCH();
+}
+
 extern "C" int pb_rmsnorm_bwd(const void* x, const void* w, const float* rstd, const void* dy, const void* dres,
                               void* dx, float* dw_partial, void* dw, int dw_fp32, int dw_accumulate, int M, int N,
                               void* stream) {
     if (N % 256 || N > 4096) return -1;
-    const int rows_per_cta = N <= 1024 ? 8 : N <= 2048 ? 4 : 2;      // of one iteration; a CTA without rows would only add a zero partial
-    const int ctas = std::max(1, std::min(pb_rmsnorm_bwd_ctas(), (M + rows_per_cta - 1) / rows_per_cta));
+    const int ctas = rmsnorm_bwd_used_ctas(M, N);
     auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w; auto DY = (const __nv_bfloat16*)dy;
     auto DR = (const __nv_bfloat16*)dres; auto DX = (__nv_bfloat16*)dx;
     // rows wider than 1024 are shared by two or four warps (at most four 256-column chunks per warp)
@@ -629,8 +641,7 @@ extern "C" int pb_rmsnorm_bwd(const void* x, const void* w, const float* rstd, c
     }
 #undef RB
     if (cudaGetLastError() != cudaSuccess) return -30;
-    launch_pdl(colsum_partials_kernel, LaunchCfg((N + 31) / 32, 32 * COLSUM_GROUPS, 0, ST(stream)), dw_partial, dw, ctas, N, dw_fp32, dw_accumulate);
-    return CHECK_LAUNCH();
+    return dw ? pb_rmsnorm_bwd_dw(dw_partial, dw, dw_fp32, dw_accumulate, M, N, stream) : 0;
 }
 
 extern "C" int pb_rope(void* qkv, const float* table, long long M, int T, int n_rot_heads, int hd, int row_stride,
@@ -791,6 +802,42 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
             *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(out) + r * ld_out + c) = o;
         }
     }
+}
+
+// The same sum of partials whose rows belong to up to four outputs of their own (contiguous fp32, rows[p] rows each, one below the
+// other in the partials): the weight gradients of stacked projections out of one GEMM.
+struct ReduceParts {
+    float* out[4];
+    int row0[5];
+};
+__global__ void __launch_bounds__(256) splitk_reduce_parts_kernel(const float* __restrict__ ws, int slices, long long M, int N, const ReduceParts parts) {
+    pdl_sync();
+    const int vpr = N / 4;
+    const long long total = M * vpr, slice_stride = M * (long long)N;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const int r = int(i / vpr);
+        float4 acc = *reinterpret_cast<const float4*>(ws + 4 * i);
+        for (int s = 1; s < slices; ++s) {
+            const float4 v = *reinterpret_cast<const float4*>(ws + s * slice_stride + 4 * i);
+            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        }
+        int p = 0;
+        while (r >= parts.row0[p + 1]) ++p;
+        *reinterpret_cast<float4*>(parts.out[p] + 4 * (i - (long long)parts.row0[p] * vpr)) = acc;
+    }
+}
+
+extern "C" int pb_splitk_reduce_parts(const float* ws, int slices, int N, int n_parts, const int* rows, void* const* outs, void* stream) {
+    if (n_parts < 1 || n_parts > 4 || N % 4 || reinterpret_cast<uintptr_t>(ws) % 16) return -1;
+    ReduceParts parts{};
+    for (int p = 0; p < n_parts; ++p) {
+        if (rows[p] <= 0 || reinterpret_cast<uintptr_t>(outs[p]) % 16) return -1;
+        parts.out[p] = reinterpret_cast<float*>(outs[p]);
+        parts.row0[p + 1] = parts.row0[p] + rows[p];
+    }
+    const long long M = parts.row0[n_parts];
+    launch_pdl(splitk_reduce_parts_kernel, LaunchCfg(grid_for(M * (N / 4), 256), 256, 0, ST(stream)).traffic(4.0 * slices * M * N), ws, slices, M, N, parts);
+    return CHECK_LAUNCH();
 }
 
 extern "C" int pb_splitk_reduce(const float* ws, int slices, long long M, int N, const void* res, long long ld_res, void* out,

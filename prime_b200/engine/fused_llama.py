@@ -119,9 +119,15 @@ class _StepGraph:
         self.seq_start = torch.empty(B * T, dtype=torch.int32, device=dev) if packed else None
         self.hyper = torch.empty(4, dtype=torch.float32, device=dev)
         self.graph = torch.cuda.CUDAGraph()
-        main, side = torch.cuda.current_stream(dev), torch.cuda.Stream(device=dev)
+        main, side, wgrads = torch.cuda.current_stream(dev), torch.cuda.Stream(device=dev), torch.cuda.Stream(device=dev)
         side.wait_stream(main)
-        K.take_scratch(side)                             # of earlier users of this handle: the graph gets its own
+        for st in (side, wgrads):
+            K.take_scratch(st)                           # of earlier users of this handle: the graph gets its own
+        # The kernels of a step small enough for a graph leave most SMs idle, so the weight gradients become a branch beside the
+        # chain of input gradients
+        eng.wgrad_stream = wgrads
+        # the norms' too, as long as their partial sums fit the scratch table side by side
+        eng._norm_dw_stream = wgrads if eng.args.n_layers <= 15 else None
         before = native.launch_counter()
         with torch.cuda.stream(side):
             self.graph.capture_begin(capture_error_mode="thread_local")
@@ -132,10 +138,12 @@ class _StepGraph:
             finally:
                 self.graph.capture_end()
                 eng._accum = False
+                eng.wgrad_stream = eng._norm_dw_stream = None
+                eng._readers.clear()
         main.wait_stream(side)
         self.launches = native.launch_counter() - before
         native.add_launches(-self.launches)              # recorded, not run
-        self.refs = [report, *eng._ws.values(), *eng._seq_start_cache.values(), *K.take_scratch(side)]
+        self.refs = [report, *eng._ws.values(), *eng._seq_start_cache.values(), *K.take_scratch(side), *K.take_scratch(wgrads)]
 
 
 class FusedLlama:
@@ -217,6 +225,7 @@ class FusedLlama:
         self.wgrad_stream = torch.cuda.Stream(device=dev) if (dev.type == "cuda" and os.environ.get("PRIME_B200_WGRAD_STREAM", "0") == "1") \
             else None
         self._readers: dict[int, torch.cuda.Event] = {}
+        self._norm_dw_stream = None     # norm weight gradients beside the chain of input gradients: recorded steps only
         # parameter views -----------------------------------------------------------------------
         self.w: dict[str, torch.Tensor] = {}
         self.g: dict[str, torch.Tensor] = {}
@@ -588,7 +597,7 @@ class FusedLlama:
         dh = self._buf("dh", (M, D))
         self._before_write(dh)
         K.rmsnorm_bwd(h, self.w[pre + "ffn_norm.weight"], rstd2, dhn, self.g[pre + "ffn_norm.weight"], dres=dout, dx=dh,
-                      accumulate_dw=self._accum)
+                      accumulate_dw=self._accum, dw_stream=self._norm_dw_stream)
         # h = x + o @ wo^T
         do = self._buf("do", (M, H * hd))
         # dO = dh @ wo; the dO . O row sums of the attention backward come out of the same kernel where it applies
@@ -605,7 +614,7 @@ class FusedLlama:
         self._wgrad(dqkv, xn, self.gqkv[i])
         self._before_write(dx)
         K.rmsnorm_bwd(x, self.w[pre + "attention_norm.weight"], rstd1, dxn, self.g[pre + "attention_norm.weight"], dres=dh,
-                      dx=dx, accumulate_dw=self._accum)
+                      dx=dx, accumulate_dw=self._accum, dw_stream=self._norm_dw_stream)
         if self._reduce_in_backward:
             self._reduce_group(1 + i, overlapped=True)     # this block's gradients are final: reduce them under the next block's backward
 
@@ -663,7 +672,7 @@ class FusedLlama:
         K.loss_sums(loss_rows, z_rows, inv, self.z_weight, out, self._partials if on_gpu else None,
                     self._counters[3:] if on_gpu else None, acc=loss_acc, acc_scale=loss_scale, acc_first=first_microbatch)
         dx = self._buf("dx_a", (M, D))
-        K.rmsnorm_bwd(xs[L], self.w["norm.weight"], rstd, dhn, self.g["norm.weight"], dx=dx, accumulate_dw=self._accum)
+        K.rmsnorm_bwd(xs[L], self.w["norm.weight"], rstd, dhn, self.g["norm.weight"], dx=dx, accumulate_dw=self._accum, dw_stream=self._norm_dw_stream)
         if self._reduce_in_backward:
             self._reduce_group(L + 1, overlapped=True)     # head group (final norm + output projection)
         # ---- blocks in reverse ----

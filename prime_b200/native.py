@@ -29,9 +29,11 @@ _CUDA_SIGS = {
                               vp, vp, vp],
     "pb_gemm_bf16_pair_splitk": [vp, vp, vp, i32, i32, i32, i64, i64, i32, i32, i32, i32, vp, vp],
     "pb_gemm_splitk_slices": [i32, i32],
+    "pb_splitk_reduce_parts": [vp, i32, i32, i32, vp, vp, vp],
     "pb_splitk_reduce": [vp, i32, i64, i32, vp, i64, vp, i64, i32, vp],
     "pb_rmsnorm_fwd": [vp, vp, vp, vp, i32, i32, f32, vp],
     "pb_rmsnorm_bwd_ctas": [],
+    "pb_rmsnorm_bwd_dw": [vp, vp, i32, i32, i32, i32, vp],
     "pb_rmsnorm_bwd": [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp],
     "pb_rope": [vp, vp, i64, i32, i32, i32, i32, i32, vp],
     "pb_swiglu_fwd": [vp, vp, i64, i32, vp],

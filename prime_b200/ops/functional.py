@@ -153,6 +153,8 @@ def _stack_bf16(*ws: torch.Tensor) -> torch.Tensor:
 
 def _stacked_wgrads(ctx, dy: torch.Tensor, xb: torch.Tensor, first: int, rows) -> list[torch.Tensor | None]:
     """One weight gradient per stacked weight, each from its columns of ``dy`` in place and into a tensor of its own."""
+    if all(ctx.needs_input_grad[first + i] for i in range(len(rows))):
+        return [dw.to(dt) for dw, dt in zip(K.gemm_row_parts(dy, xb, tuple(rows)), ctx.w_dtypes)]
     out, r = [], 0
     for i, n in enumerate(rows):
         dw = None

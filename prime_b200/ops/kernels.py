@@ -7,6 +7,7 @@ use and what the GPU numerics tests compare against.
 """
 from __future__ import annotations
 
+import ctypes
 import functools
 import threading
 
@@ -124,6 +125,31 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, resi
         ptr(a), ptr(b), ptr(out), ptr(residual), M, N, K, a.stride(0), b.stride(0), out.stride(0), ldr, int(a_mn), int(b_mn),
         int(out.dtype == torch.float32), bn if bn in (128, 256) else 0, max_ctas, ptr(status_word(a.device)), stream_ptr())
     check(rc, f"pb_gemm_bf16(M={M},N={N},K={K},a_mn={a_mn},b_mn={b_mn})")
+    return out
+
+
+def gemm_row_parts(a: torch.Tensor, b: torch.Tensor, rows: tuple[int, ...]) -> list[torch.Tensor]:
+    """``a.T @ b`` in fp32 with every ``rows[i]`` rows of the product in a tensor of their own (``a`` is ``[K, sum(rows)]``, ``b`` is
+    ``[K, N]``). A product that is split over K anyway is one GEMM and one reduce that writes all the tensors; others are one GEMM
+    each. Three gradients [512 x 512] over 8192 tokens: 58 us in six launches, 25 in two."""
+    M, N, K = a.shape[1], b.shape[1], a.shape[0]
+    slices = _splitk_slices(M, N, K, a.device) if a.is_cuda and _GEMM_PAIR and len(rows) <= 4 else 1
+    if slices == 1 or not (a.stride(-1) == b.stride(-1) == 1):
+        out, r = [], 0
+        for n in rows:
+            out.append(gemm(a[:, r: r + n], b, a_mn=True, b_mn=True, out_dtype=torch.float32))
+            r += n
+        return out
+    assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and b.shape[0] == K and sum(rows) == M
+    lib = native.cuda()
+    ws = _scratch_buf(a.device, "splitk", slices * M * N)
+    rc = lib.pb_gemm_bf16_pair_splitk(ptr(a), ptr(b), ptr(ws), M, N, K, a.stride(0), b.stride(0), 1, 1, slices, 0,
+                                      ptr(status_word(a.device)), stream_ptr())
+    check(rc, f"pb_gemm_bf16_pair_splitk(M={M},N={N},K={K},slices={slices})")
+    out = [torch.empty(n, N, dtype=torch.float32, device=a.device) for n in rows]
+    rc = lib.pb_splitk_reduce_parts(ptr(ws), lib.pb_gemm_splitk_slices(K, slices), N, len(rows), (ctypes.c_int * len(rows))(*rows),
+                                    (ctypes.c_void_p * len(rows))(*[t.data_ptr() for t in out]), stream_ptr())
+    check(rc, "pb_splitk_reduce_parts")
     return out
 
 
@@ -249,8 +275,9 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float, out: torch.Tensor 
 
 
 def rmsnorm_bwd(x, w, rstd, dy, dw: torch.Tensor, dres: torch.Tensor | None = None, dx: torch.Tensor | None = None,
-                accumulate_dw: bool = True):
-    """Returns dx (= norm input gradient + ``dres``) and adds the weight gradient into ``dw``."""
+                accumulate_dw: bool = True, dw_stream: torch.cuda.Stream | None = None):
+    """Returns dx (= norm input gradient + ``dres``) and adds the weight gradient into ``dw``, on ``dw_stream`` if there is one (the
+    partial sums then lie in a scratch of this ``dw``'s own)."""
     M, N = x.shape
     if dx is None:
         dx = torch.empty_like(x)
@@ -266,9 +293,13 @@ def rmsnorm_bwd(x, w, rstd, dy, dw: torch.Tensor, dres: torch.Tensor | None = No
         return dx
     lib = native.cuda()
     ctas = lib.pb_rmsnorm_bwd_ctas()
-    part = _scratch_buf(x.device, "rms_bwd", ctas * N)
-    check(lib.pb_rmsnorm_bwd(ptr(x), ptr(w), ptr(rstd), ptr(dy), ptr(dres), ptr(dx), ptr(part), ptr(dw),
+    part = _scratch_buf(x.device, "rms_bwd" if dw_stream is None else f"rms_bwd.{dw.data_ptr()}", ctas * N)
+    check(lib.pb_rmsnorm_bwd(ptr(x), ptr(w), ptr(rstd), ptr(dy), ptr(dres), ptr(dx), ptr(part), ptr(dw) if dw_stream is None else None,
                              int(dw.dtype == torch.float32), int(accumulate_dw), M, N, stream_ptr()), "pb_rmsnorm_bwd")
+    if dw_stream is not None:
+        dw_stream.wait_stream(torch.cuda.current_stream(x.device))
+        check(lib.pb_rmsnorm_bwd_dw(ptr(part), ptr(dw), int(dw.dtype == torch.float32), int(accumulate_dw), M, N, stream_ptr(dw_stream)),
+              "pb_rmsnorm_bwd_dw")
     return dx
 
 

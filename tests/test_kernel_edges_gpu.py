@@ -1,0 +1,205 @@
+"""Kernels at the sizes where a tile, a ring or a path of the dispatch ends, against plain fp32 (or fp64) torch."""
+import pytest
+import torch
+
+from prime_b200.ops import attention as A
+from prime_b200.ops import kernels as ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return ((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-12)).item()
+
+
+def _attention_case(starts, M, H, KV, hd, seed=0):
+    torch.manual_seed(seed)
+    qkv = (torch.randn(M, (H + 2 * KV) * hd, device="cuda") * 0.7).bfloat16()
+    ss = torch.zeros(M, dtype=torch.int32)
+    for s, e in zip(starts, list(starts[1:]) + [M]):
+        ss[s:e] = s
+    ss = ss.cuda()
+    o, lse2 = A.attention_fwd(qkv, ss, H, KV, hd)
+    x = qkv.float().requires_grad_(True)
+    ref = A.attention_reference(x, ss, H, KV, hd)
+    # bf16 P (2^-9) and output (2^-9)
+    assert _rel(o, ref.detach()) < 1e-2
+    _, lse_ref = A.attention_fwd(qkv.cpu(), ss.cpu(), H, KV, hd)
+    assert (lse2.cpu() - lse_ref).abs().max().item() < 1e-2
+    dout = (torch.randn(M, H * hd, device="cuda") * 0.5).bfloat16()
+    table = ops.rope_table(M, hd, 10000.0, "cuda")
+    g = A.attention_bwd(qkv, o, dout, lse2, ss, H, KV, hd, rope_table=table, seq_len=M)
+    ops.check_status()
+    (gref,) = torch.autograd.grad(ref, x, dout.float())
+    gref = ops.rope_(gref.cpu(), table.cpu(), M, H + KV, hd, backward=True).cuda()
+    for cols in (slice(0, H * hd), slice(H * hd, (H + KV) * hd), slice((H + KV) * hd, None)):
+        # (a row that sees only itself has P = 1 and dS = 0: nothing but rounding in dQ and dK)
+        if len(starts) < M or cols.stop is None:
+            assert _rel(g[:, cols], gref[:, cols]) < 2e-2
+
+
+# The forward takes two 128-row query tiles at a time: one tile only, an odd number of them, a last tile of one row, documents that
+# start in the second tile of a pair (its kv tiles begin later), at tile edges and one row beside them, and one row per document
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("M,starts", [(1, (0,)), (128, (0,)), (129, (0,)), (257, (0, 256)), (640, (0, 128, 384)), (900, (0, 127, 129, 300, 511, 513)),
+                                      (512, tuple(range(512)))])
+def test_attention_tile_pairs(hd, M, starts):
+    _attention_case(starts, M, 4, 2, hd)
+
+
+# More pairs of query tiles than SMs, so that CTAs take over the work of others, rings wrap and heads change on the way; odd tile count
+@pytest.mark.parametrize("hd,H,KV", [(64, 16, 4), (128, 12, 3), (32, 16, 16)])
+def test_attention_more_pairs_than_sms(hd, H, KV):
+    M = 128 * 33 - 5
+    _attention_case((0, 700, 1400, 1401, 3000), M, H, KV, hd, seed=3)
+
+
+@pytest.mark.parametrize("hd,parts", [(64, 1), (128, 2)])
+def test_attention_backward_takes_row_dots_in_parts(hd, parts):
+    torch.manual_seed(0)
+    M, H, KV = 700, 4, 2
+    qkv = (torch.randn(M, (H + 2 * KV) * hd, device="cuda") * 0.7).bfloat16()
+    ss = A.seq_start_from_batch(1, M, "cuda")
+    o, lse2 = A.attention_fwd(qkv, ss, H, KV, hd)
+    dh = torch.randn(M, 512, device="cuda").bfloat16()
+    wo = (torch.randn(512, H * hd, device="cuda") * 512 ** -0.5).bfloat16()
+    do = torch.empty(M, H * hd, device="cuda", dtype=torch.bfloat16)
+    dots = A.row_dots_buffer(do.device, M, H, parts)
+    assert ops.gemm_rowdot(dh, wo, do, o, dots, hd, b_mn=True)
+    want_dots = (dh.float() @ wo.float() * o.float()).reshape(M, H, parts, 64).sum(-1).permute(1, 2, 0)
+    assert _rel(dots.view(H, parts, M), want_dots) < 1e-3
+    got = A.attention_bwd(qkv, o, do, lse2, ss, H, KV, hd, row_dots=dots.clone())
+    want = A.attention_bwd(qkv, o, do, lse2, ss, H, KV, hd)
+    ops.check_status()
+    assert _rel(got, want) < 1e-2                            # the sums are over dO before and after its rounding to bf16
+
+
+# Tile widths of the CTA-pair GEMM: outputs for which each width is chosen, with ragged last rows, a last tile that is cut inside a
+# 64-column box, and every epilogue
+@pytest.mark.parametrize("M,N,K", [(512, 256, 128), (520, 1024, 1024), (2331, 1024, 320), (2331, 1000, 256), (700, 1416, 512), (8192, 256, 256),
+                                   (1300, 3072, 512)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_gemm_tile_widths(M, N, K, b_mn):
+    torch.manual_seed(0)
+    x = torch.randn(M, K, device="cuda").bfloat16()
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()
+    b = w.t().contiguous() if b_mn else w
+    ref = x.float() @ w.float().t()
+    r = torch.randn(M, N, device="cuda").bfloat16()
+    wide = torch.full((M, N + 8), 7.0, device="cuda").bfloat16()
+    ops.gemm(x, b, out=wide[:, :N], b_mn=b_mn)
+    assert _rel(wide[:, :N], ref) < 1e-2 and bool((wide[:, N:] == 7).all())
+    assert _rel(ops.gemm(x, b, residual=r, b_mn=b_mn), ref + r.float()) < 1e-2
+    f = torch.randn(M, N, device="cuda")
+    want = f + ref
+    assert _rel(ops.gemm(x, b, out=f, residual=f, b_mn=b_mn), want) < 1e-3
+    assert _rel(ops.gemm(x, b, out_dtype=torch.float32, b_mn=b_mn), ref) < 1e-3
+    if N % 64 == 0 and b_mn:
+        o, dots = torch.empty_like(r), torch.empty(N // 64 * M, device="cuda")
+        assert ops.gemm_rowdot(x, b, o, r, dots, 64, b_mn=True)
+        assert _rel(o, ref) < 1e-2
+        assert _rel(dots.view(N // 64, M), (ref * r.float()).view(M, N // 64, 64).sum(-1).t()) < 1e-3
+    ops.check_status()
+
+
+@pytest.mark.parametrize("M", [512, 777, 2331, 8192])
+@pytest.mark.parametrize("F", [192, 704, 1536])
+def test_swiglu_epilogues_of_narrow_tiles(M, F):
+    torch.manual_seed(0)
+    K = 256
+    x = torch.randn(M, K, device="cuda").bfloat16()
+    w13 = (torch.randn(2 * F, K, device="cuda") * K ** -0.5).bfloat16()
+    h13, act = torch.empty(M, 2 * F, device="cuda", dtype=torch.bfloat16), torch.empty(M, F, device="cuda", dtype=torch.bfloat16)
+    ops.gemm_swiglu(x, w13, h13, act)
+    ref = x.float() @ w13.float().t()
+    assert _rel(h13, ref) < 1e-2
+    assert _rel(act, torch.nn.functional.silu(ref[:, :F]) * ref[:, F:]) < 1e-2
+    w2 = (torch.randn(128, F, device="cuda") * F ** -0.5).bfloat16()
+    dout = torch.randn(M, 128, device="cuda").bfloat16()
+    gb, ub, d = h13[:, :F].float(), h13[:, F:].float(), dout.float() @ w2.float()
+    sg = torch.sigmoid(gb)
+    want = torch.cat([d * ub * sg * (1 + gb * (1 - sg)), d * gb * sg], 1)
+    ops.gemm_dswiglu(dout, w2, h13)
+    ops.check_status()
+    assert _rel(h13, want) < 1.5e-2
+
+
+# heads whose columns divide the epilogue's 128-column rounds and one (192) whose table differs from round to round; rows that wrap
+# around the positions inside a tile
+@pytest.mark.parametrize("hd", [8, 32, 64, 128, 192])
+@pytest.mark.parametrize("M,T", [(600, 200), (2331, 777), (1024, 1024)])
+def test_rope_epilogue_heads(hd, M, T):
+    torch.manual_seed(0)
+    K, H, KV = 192, 768 // hd, 384 // hd
+    N = (H + 2 * KV) * hd
+    x = torch.randn(M, K, device="cuda").bfloat16()
+    w = (torch.randn(N, K, device="cuda") * K ** -0.5).bfloat16()
+    table = ops.rope_table(T, hd, 10000.0, "cuda")
+    out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    ops.gemm_rope(x, w, out, table, T, H + KV, hd)
+    ref = ops.rope_((x.float() @ w.float().t()).cpu(), table.cpu(), T, H + KV, hd).cuda()
+    ops.check_status()
+    assert _rel(out, ref) < 1e-2
+
+
+# Whole chunks of finite values take a path of their own; a ragged last chunk, one with an infinity or NaN and one whose sum of squares
+# overflows take the general one. Zeros, outliers (clamping bins) and tiny values on the first.
+@pytest.mark.parametrize("what", ["normal", "outliers", "zeros", "tiny", "constant", "inf", "nan", "huge"])
+def test_quantizer_paths(what):
+    from prime_b200 import native
+    from prime_b200.ops.quant import uniform_8bit_quantize_cuda
+    chunk = native.cuda().pb_dl_chunk()
+    torch.manual_seed(0)
+    x = torch.randn(2 * chunk + 37, device="cuda") * 1e-3
+    if what == "outliers":
+        x[::97] *= 300
+    elif what == "zeros":
+        x[:chunk] = 0
+    elif what == "tiny":
+        x[:chunk] *= 1e-24
+    elif what == "constant":
+        x[:chunk] = 3.0
+    elif what == "inf":
+        x[5], x[9] = float("inf"), -float("inf")
+    elif what == "nan":
+        x[5] = float("nan")
+    elif what == "huge":
+        x[:chunk] *= 1e30
+    q, lut = uniform_8bit_quantize_cuda(x)
+    for c in range(3):
+        v = x[c * chunk: (c + 1) * chunk]
+        n = v.numel()
+        ss = (v * v).double().sum()             # squared in fp32: tiny squares vanish, huge ones overflow
+        scale = (6 * (ss / max(n - 1, 1)).sqrt() / 256).float().item()
+        if not (0 < scale < 3e38):
+            scale = 1.0
+        t = v.double() / scale
+        fin = torch.isfinite(t)
+        want = (torch.round(t) + 128).clamp(0, 255)
+        got = q[c * chunk: (c + 1) * chunk].double()
+        # a value within the fp32 rounding of scale and t of a bin's edge may go either way
+        near = ((t - torch.floor(t)) - 0.5).abs() < 1e-5 * t.abs().clamp_min(1)
+        assert bool(((got == want) | near | ~fin | (t.abs() > 1e6)).all()), (what, c)
+        if not bool(fin.all()) or float(t.abs().max()) > 1e6:
+            continue
+        for b in (0, 1, 100, 128, 200, 255):
+            m = got == b
+            if bool(m.any()):
+                mean = v[m].double().mean().item()
+                # inner bins: offsets in steps of 1/512 of a bin
+                assert abs(lut[c, b].item() - mean) <= 2e-3 * scale + 1e-5 * abs(mean), (what, c, b)
+
+
+# Three outputs of one split product, outputs too large or too short in K to be split (one GEMM each), rows that share 256-row tiles
+@pytest.mark.parametrize("K,N,rows", [(8192, 512, (512, 512, 512)), (8192, 512, (1536, 1536)), (4096, 256, (256, 128, 128)), (512, 512, (512, 256)),
+                                      (2304, 260, (300, 20, 192, 8))])
+def test_gemm_row_parts(K, N, rows):
+    torch.manual_seed(0)
+    a = torch.randn(K, sum(rows), device="cuda").bfloat16()
+    b = torch.randn(K, (N + 7) // 8 * 8, device="cuda").bfloat16()[:, :N]
+    outs = ops.gemm_row_parts(a, b, rows)
+    ref = a.float().t() @ b.float()
+    ops.check_status()
+    assert [tuple(o.shape) for o in outs] == [(n, N) for n in rows] and all(o.is_contiguous() and o.dtype == torch.float32 for o in outs)
+    assert len({o.untyped_storage().data_ptr() for o in outs}) == len(outs)
+    assert _rel(torch.cat(outs), ref) < 1e-3
