@@ -514,10 +514,10 @@ static int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const 
 // null (then the caller has already filled it with [H, d_parts, M] partial sums). Writes all of dqkv.
 // rope_table != null: the inverse rotation is applied to dq and dk on the way out (position = row % T).
 // tile_scratch: >= ceil(M / 128) + 1 ints of device scratch (query-tile count of every kv tile and the work counter).
-extern "C" int pb_attn_bwd(const void* qkv, const void* o, const void* dout, const float* lse2, const int* seq_start,
-                           void* dqkv, float* dq_acc, float* D, int d_parts, const float* rope_table, int T, int M, int H, int KV, int HD,
-                           long long qkv_stride, long long o_stride, long long do_stride, long long dqkv_stride, float scale,
-                           int* tile_scratch, int* status, void* stream) {
+extern "C" int pb_attn_bwd_parts(const void* qkv, const void* o, const void* dout, const float* lse2, const int* seq_start,
+                                 void* dqkv, float* dq_acc, float* D, int d_parts, const float* rope_table, int T, int M, int H, int KV, int HD,
+                                 long long qkv_stride, long long o_stride, long long do_stride, long long dqkv_stride, float scale,
+                                 int* tile_scratch, int* status, void* stream) {
     using namespace pb;
     if (HD <= 0 || HD > 128 || HD % 8) return -1;
     if (H % KV) return -1;
@@ -559,4 +559,13 @@ extern "C" int pb_attn_bwd(const void* qkv, const void* o, const void* dout, con
     launch_pdl(attn_bwd_finish_kernel, LaunchCfg(unsigned(blocks), 256, 0, st).traffic(6.0 * M * H * HD), dq_acc, (__nv_bfloat16*)dqkv, rope_table, M, T, H, HD,
                dqkv_stride);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
+}
+
+// D whole: [H, M]
+extern "C" int pb_attn_bwd(const void* qkv, const void* o, const void* dout, const float* lse2, const int* seq_start,
+                           void* dqkv, float* dq_acc, float* D, const float* rope_table, int T, int M, int H, int KV, int HD,
+                           long long qkv_stride, long long o_stride, long long do_stride, long long dqkv_stride, float scale,
+                           int* tile_scratch, int* status, void* stream) {
+    return pb_attn_bwd_parts(qkv, o, dout, lse2, seq_start, dqkv, dq_acc, D, 1, rope_table, T, M, H, KV, HD, qkv_stride, o_stride, do_stride,
+                             dqkv_stride, scale, tile_scratch, status, stream);
 }

@@ -19,7 +19,6 @@ struct GemmParams {
     int num_tiles, tiles_n;
     // CTA-pair kernel: tiles are numbered in bands of group_m tile rows (see gemm_tile_mn); tiles_m = rows of tiles
     int tiles_m, group_m;
-    int bn;          // CTA-pair kernel: columns of a tile (256, 192, 128 or 64)
     int tn_rot;      // tile columns are visited starting at this one (all-gather GEMM: the n-block fetched first)
     // split-K: work item w = slice * num_tiles + tile; slice s covers k-blocks [s * kb_per_split, ...) and
     // stores its fp32 partial tile in plane s of the output tensor map (staged fp32 epilogue)

@@ -19,7 +19,8 @@ from .kernels import _scratch_buf, status_word
 native.register_cuda_sigs({
     "pb_attn_fwd": [native.vp, native.vp, native.vp, native.vp, native.i32, native.i32, native.i32, native.i32,
                     native.i64, native.i64, native.f32, native.vp, native.vp],
-    "pb_attn_bwd": [native.vp] * 8 + [native.i32, native.vp] + [native.i32] * 5 + [native.i64] * 4 + [native.f32, native.vp, native.vp, native.vp],
+    "pb_attn_bwd": [native.vp] * 9 + [native.i32] * 5 + [native.i64] * 4 + [native.f32, native.vp, native.vp, native.vp],
+    "pb_attn_bwd_parts": [native.vp] * 8 + [native.i32, native.vp] + [native.i32] * 5 + [native.i64] * 4 + [native.f32, native.vp, native.vp, native.vp],
 })
 
 
@@ -187,7 +188,7 @@ def attention_bwd(qkv: torch.Tensor, o: torch.Tensor, dout: torch.Tensor, lse2: 
     tiles = _scratch_buf(qkv.device, "attn_tiles", (M + 127) // 128 + 1, torch.int32)
     assert rope_table is None or seq_len > 0
     qkv, o, dout, g = _fitting_input(qkv, hd), _fitting_input(o, hd), _fitting_input(dout, hd), _fitting_output(dqkv, hd)
-    check(native.cuda().pb_attn_bwd(ptr(qkv), ptr(o) if row_dots is None else None, ptr(dout), ptr(lse2), ptr(seq_start), ptr(g), ptr(dq_acc), ptr(D), d_parts,
+    check(native.cuda().pb_attn_bwd_parts(ptr(qkv), ptr(o) if row_dots is None else None, ptr(dout), ptr(lse2), ptr(seq_start), ptr(g), ptr(dq_acc), ptr(D), d_parts,
                                     ptr(rope_table), max(int(seq_len), 1), M, H, KV, hd, qkv.stride(0),
                                     o.stride(0), dout.stride(0), g.stride(0), scale, ptr(tiles), ptr(status_word(qkv.device)),
                                     stream_ptr()), "pb_attn_bwd")

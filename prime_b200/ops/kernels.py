@@ -295,7 +295,8 @@ def rmsnorm_bwd(x, w, rstd, dy, dw: torch.Tensor, dres: torch.Tensor | None = No
     ctas = lib.pb_rmsnorm_bwd_ctas()
     part = _scratch_buf(x.device, "rms_bwd" if dw_stream is None else f"rms_bwd.{dw.data_ptr()}", ctas * N)
     check(lib.pb_rmsnorm_bwd(ptr(x), ptr(w), ptr(rstd), ptr(dy), ptr(dres), ptr(dx), ptr(part), ptr(dw) if dw_stream is None else None,
-                             int(dw.dtype == torch.float32), int(accumulate_dw), M, N, stream_ptr()), "pb_rmsnorm_bwd")
+                             int(dw.dtype == torch.float32), int(accumulate_dw), M, N, stream_ptr()),
+          "pb_rmsnorm_bwd" if dw_stream is None else "pb_rmsnorm_bwd without dw")
     if dw_stream is not None:
         dw_stream.wait_stream(torch.cuda.current_stream(x.device))
         check(lib.pb_rmsnorm_bwd_dw(ptr(part), ptr(dw), int(dw.dtype == torch.float32), int(accumulate_dw), M, N, stream_ptr(dw_stream)),
