@@ -299,7 +299,7 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
         if (idx >= 0) {
             item = bwd_item_of(p, idx);
             n_q = p.nq[item.kv_tile];
-            cur = bwd_row(p, item.g * G, item.kv_tile, r);
+            cur = bwd_row<true>(p, item.g * G, item.kv_tile, r);
         }
         for (int k = 0; idx >= 0; ++k) {
             const int kv0 = item.kv_tile * 128, g = item.g, n_it = n_q * G;
@@ -317,7 +317,7 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
                 if (lane == 0) mbar_arrive(bar_sfree);
                 const BwdRow x = cur;
                 if (++qi == n_q) { qi = 0; ++hq; }
-                if (it + 1 < n_it) cur = bwd_row(p, hq, item.kv_tile + qi, r);      // lands while this pair is exponentiated
+                if (it + 1 < n_it) cur = bwd_row<true>(p, hq, item.kv_tile + qi, r);      // lands while this pair is exponentiated
                 if (bwd_needs_mask(p, x, kv0)) bwd_probs<true>(sv, x, x.q0 + r, kv0 + half * 64, c);
                 else bwd_probs<false>(sv, x, x.q0 + r, kv0 + half * 64, c);
                 if (gi > 0) {   // dV of the previous pair has read its P, and the dQ boxes that followed it there have left
@@ -351,7 +351,7 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_const
             if (idx >= 0) {
                 item = bwd_item_of(p, idx);
                 n_q = p.nq[item.kv_tile];
-                cur = bwd_row(p, item.g * G, item.kv_tile, r);
+                cur = bwd_row<true>(p, item.g * G, item.kv_tile, r);
             }
             tc_fence_after();
             bwd_write_dkdv<128>(p, tDK, tDV, kv0 + r, g, half);

@@ -303,7 +303,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
         // (query head, query tile) of the pair whose row constants are loaded next, inside the current item
         int kv_tile = 0, n_q = 0, hq_n = 0, qi_n = 0;
         auto row_ctx = [&]() {
-            const BwdRow x = bwd_row(p, hq_n, kv_tile + qi_n, r);
+            const BwdRow x = bwd_row<false>(p, hq_n, kv_tile + qi_n, r);
             if (++qi_n == n_q) { qi_n = 0; ++hq_n; }
             return x;
         };
@@ -342,17 +342,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
                 --left;
                 if (left) nxt = row_ctx();      // global loads land while this pair is exponentiated
                 const int row = cur.q0 + r;
-                if (bwd_needs_mask(p, cur, kv0)) bwd_probs<true>(sv, cur, row, kv0 + half * 64, c);
-                else bwd_probs<false>(sv, cur, row, kv0 + half * 64, c);
-                bwd_dscores(sv, dv, cur.Dr);
+                if (bwd_needs_mask(p, cur, kv0)) bwd_probs_dscores<true>(sv, dv, cur, row, kv0 + half * 64, c);
+                else bwd_probs_dscores<false>(sv, dv, cur, row, kv0 + half * 64, c);
                 if (gi > 0) {
                     // the MMAs of the previous pair have read its P/dS out of shared memory
                     ok = mbar_wait(bar_dqfull, (gi - 1) & 1, abort_flag, p.status, PB_ERR_TIMEOUT_TMEM_FULL);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                 }
-                bwd_store_half(gP, sv, half, r);
-                bwd_store_half(gDS, dv, half, r);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const uint32_t off = half * 16384 + r * 128 + ((q ^ (r & 7)) << 4);
+                    *reinterpret_cast<uint4*>(gP + off) = make_uint4(sv[4 * q], sv[4 * q + 1], sv[4 * q + 2], sv[4 * q + 3]);
+                    *reinterpret_cast<uint4*>(gDS + off) = make_uint4(dv[4 * q], dv[4 * q + 1], dv[4 * q + 2], dv[4 * q + 3]);
+                }
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_pdsfull);
