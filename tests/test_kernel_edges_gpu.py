@@ -54,6 +54,32 @@ def test_attention_more_pairs_than_sms(hd, H, KV):
     _attention_case((0, 700, 1400, 1401, 3000), M, H, KV, hd, seed=3)
 
 
+# recorded and replayed on other inputs, behind a kernel that is still running: work is drawn anew in every replay
+def test_attention_of_wide_heads_in_a_graph():
+    M, H, KV, hd = 128 * 41, 16, 4, 128
+    torch.manual_seed(0)
+    qkv = (torch.randn(M, (H + 2 * KV) * hd, device="cuda") * 0.7).bfloat16()
+    ss = A.seq_start_from_batch(1, M, "cuda")
+    o, lse2, g = torch.empty(M, H * hd, device="cuda", dtype=torch.bfloat16), torch.empty(H, M, device="cuda"), torch.empty_like(qkv)
+    dout = torch.randn(M, H * hd, device="cuda").bfloat16()
+
+    def step():
+        A.attention_fwd(qkv, ss, H, KV, hd, out=o, lse2=lse2)
+        A.attention_bwd(qkv, o, dout, lse2, ss, H, KV, hd, dqkv=g)
+    step()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    for seed in (1, 2):
+        qkv.copy_((torch.randn(M, qkv.shape[1], device="cuda", generator=torch.Generator("cuda").manual_seed(seed)) * 0.7).bfloat16())
+        step()
+        want_o, want_l, want_g = o.clone(), lse2.clone(), g.clone()
+        o.zero_(), lse2.zero_(), g.zero_()
+        graph.replay()
+        ops.check_status()
+        assert torch.equal(o, want_o) and torch.equal(lse2, want_l) and _rel(g, want_g) < 1e-3      # dQ is summed in the order of arrival
+
+
 @pytest.mark.parametrize("hd,parts", [(64, 1), (128, 2)])
 def test_attention_backward_takes_row_dots_in_parts(hd, parts):
     torch.manual_seed(0)
