@@ -133,7 +133,9 @@ constexpr int DL_MAGIC_BITS = 0x4B400000;
 
 // A whole chunk of finite values. |x| <= the chunk's L2 norm, so that |t| = |x / scale| < 2^13: the rounded value has its bin in its
 // low bits, clamped by one instruction. Every element goes to the table without a test: those of the two clamping bins leave
-// something in rows 0 and 255 that nobody reads. Whether there are any is asked once per four elements.
+// something in rows 0 and 255 that nobody reads. Whether there are any is asked once per four elements. 266M values 453 -> 386 us,
+// 67M 124 -> 108 (of 52 for the bytes); no unit is full then (ALU 37 %, issue 57 %, shared-memory wavefronts 42 %): the warps wait at
+// the barriers between a chunk's phases and for the table's atomics.
 template <int G>
 __device__ __forceinline__ void dl_quantize_finite(const float (&v)[DL_PER_THREAD], uint8_t* __restrict__ q_chunk, bool q_aligned,
                                                    unsigned* my_bin, long long (&e_sum)[2], unsigned (&e_cnt)[2], float inv_scale) {

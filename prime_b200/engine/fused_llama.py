@@ -149,8 +149,8 @@ class _StepGraph:
 class FusedLlama:
     """See module docstring. One instance per process / GPU."""
     _MAX_GRAPHS = 8
-    # Recording costs 7-30 ms and a replay saves 0.5 ms (two-block model of 512 tokens: launch by launch 914 us, replayed 374 us,
-    # recorded and replayed 7-24 ms; the debug model's step 1913, 1388 us and 17-30 ms). With room left a shape is recorded
+    # Recording costs 7-30 ms and a replay saves 0.5 ms (two-block model of 512 tokens: launch by launch 914 us, replayed 273 us,
+    # recorded and replayed 7-24 ms; the debug model's step 1913, 1164 us and 17-30 ms). With room left a shape is recorded
     # at its second call. With none left it takes the place of the least recently used only after this many calls, so that a
     # program with more shapes than graphs pays for a recording once in a few hundred steps.
     _RUNS_TO_EVICT = 32
