@@ -11,7 +11,10 @@
 //   dV(i), dQ(i), dK(i) when P(i) and dS(i) are in shared memory; dO's tile is refilled behind dV, Q's behind dK
 //   dP(i+1)            when the drain warps have read dQ(i), which they do under dK(i)
 // so that between "P and dS are there" of two pairs stand the four MMAs, one read of dP, and dS = P (dP - D). With one Q / dO
-// stage, S and dP issued together and dQ in the place of S (the earlier form of this kernel) every step waited for the one before.
+// stage, S and dP issued together and dQ in the place of S (the earlier form of this kernel) every step waited for the one before:
+// whole backward, 8 x 2048 tokens, 16 heads 771 -> 626 us, 1 x 8192, 32 / 8 heads 2733 -> 2047.
+// What bounds it: shared memory. The five MMAs of a pair read 2560 cycles' worth of operands there, which is what they need at full
+// rate; P, dS, the dQ boxes (written and sent) and the next Q and dO are another 2000.
 #include "attn_bwd.cuh"
 
 namespace pb {
