@@ -124,7 +124,7 @@ class _StepGraph:
         for st in (side, wgrads):
             K.take_scratch(st)                           # of earlier users of this handle: the graph gets its own
         # The kernels of a step small enough for a graph leave most SMs idle, so the weight gradients become a branch beside the
-        # chain of input gradients
+        # chain of input gradients: two-block model of 512 tokens 328 -> 272 us, debug model's step 1331 -> 1165
         eng.wgrad_stream = wgrads
         # the norms' too, as long as their partial sums fit the scratch table side by side
         eng._norm_dw_stream = wgrads if eng.args.n_layers <= 15 else None
