@@ -36,7 +36,8 @@ constexpr int DL_MAX_RANKS = 16;
 constexpr int DL_CHUNK = 16384;           // elements per quantisation chunk = one CTA's register-resident tile
 constexpr int DL_THREADS = 512;           // two CTAs per SM: one loads or waits at a barrier while the other computes
 constexpr int DL_PER_THREAD = DL_CHUNK / DL_THREADS;   // 32
-constexpr int DL_TABLE = 256 * 32;        // words of the CTA's shared table: 256 entries x one copy per lane (32 KB)
+constexpr int DL_TABLE = 256 * 32;        // words of the CTA's shared table: 256 entries x one copy per lane (32 KB) ...
+constexpr int DL_TABLE_WORDS = DL_TABLE + 6;   // ... and the clamping bins' two 64-bit sums and two counts
 // One 32-bit shared-memory atomic per element: an inner bin holds (count << 20) | sum of the 9-bit fixed-point
 // offsets of its members from the bin's lower edge. The histogram has one copy per lane (word bin * 32 + lane), so the 32
 // atomics of a warp instruction always go to 32 different banks and never to the same word, whatever the values are.
@@ -108,19 +109,9 @@ __device__ __forceinline__ bool dl_wait_peers(const DlPeers& p, int slot, int ep
     return ok;
 }
 
-__device__ __forceinline__ float dl_block_sum(float v) {
-    __shared__ float red[DL_THREADS / 32];
-    __shared__ float total;
-    v = warp_sum(v);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.f;
-        for (int i = 0; i < DL_THREADS / 32; ++i) t += red[i];      // fixed order
-        total = t;
-    }
-    __syncthreads();
-    return total;
+// The CTA's table starts out empty; whoever turns a chunk's sums into its codebook leaves it empty for the next one.
+__device__ __forceinline__ void dl_table_clear(unsigned* s_bin) {
+    for (int i = threadIdx.x; i < DL_TABLE_WORDS; i += DL_THREADS) s_bin[i] = 0u;
 }
 
 // Quantise the CTA's register-resident chunk and write bytes + codebook. Thread t holds 32 / G groups of G
@@ -133,9 +124,8 @@ constexpr int DL_MAGIC_BITS = 0x4B400000;
 
 // A whole chunk of finite values. |x| <= the chunk's L2 norm, so that |t| = |x / scale| < 2^13: the rounded value has its bin in its
 // low bits, clamped by one instruction. Every element goes to the table without a test: those of the two clamping bins leave
-// something in rows 0 and 255 that nobody reads. Whether there are any is asked once per four elements. 266M values 453 -> 386 us,
-// 67M 124 -> 108 (of 52 for the bytes); no unit is full then (ALU 37 %, issue 57 %, shared-memory wavefronts 42 %): the warps wait at
-// the barriers between a chunk's phases and for the table's atomics.
+// something in rows 0 and 255 that nobody reads. Whether there are any is asked once per four elements. 266M values 453 -> 386 us
+// (of 207 for the bytes); no unit was full then (ALU 37 %, issue 57 %, shared-memory wavefronts 42 %).
 template <int G>
 __device__ __forceinline__ void dl_quantize_finite(const float (&v)[DL_PER_THREAD], uint8_t* __restrict__ q_chunk, bool q_aligned,
                                                    unsigned* my_bin, long long (&e_sum)[2], unsigned (&e_cnt)[2], float inv_scale) {
@@ -255,21 +245,26 @@ __device__ __forceinline__ void dl_quantize_body(const float (&v)[DL_PER_THREAD]
     }
 }
 
-// `loaded` is called once, behind a barrier that every thread reaches with its values in registers.
+// `loaded` is called once, when this thread's values are in registers. The table is empty before and after. Two barriers a chunk: the
+// first says that the warps' sums of squares are there and that the last chunk's codebook is done, the second that all values are in
+// the table. With five (a table cleared between two of them, a sum that one thread took and handed out between two more) the warps
+// stood there a sixth of the time: 266M values 386 -> 334 us.
 template <int G, typename F>
 __device__ __forceinline__ void dl_quantize_chunk(float (&v)[DL_PER_THREAD], long long cnt, uint8_t* __restrict__ q_chunk,
                                                   float* __restrict__ lut_chunk, bool q_aligned, unsigned* s_bin, F&& loaded) {
-    __shared__ unsigned long long s_edge_sum[2];
-    __shared__ unsigned s_edge_cnt[2];
+    __shared__ float red[DL_THREADS / 32];
+    unsigned long long* s_edge_sum = reinterpret_cast<unsigned long long*>(s_bin + DL_TABLE);
+    unsigned* s_edge_cnt = s_bin + DL_TABLE + 4;
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < DL_PER_THREAD; ++i) ss += v[i] * v[i];
-    __syncthreads();                                         // the table's previous use (look-ups, last chunk's codebook) is over
     loaded();
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < DL_TABLE / 4; i += DL_THREADS) reinterpret_cast<uint4*>(s_bin)[i + threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
-    if (threadIdx.x < 2) { s_edge_sum[threadIdx.x] = 0ull; s_edge_cnt[threadIdx.x] = 0u; }
-    ss = dl_block_sum(ss);                                   // also orders the zeroing above before the atomics below
+    for (int i = 0; i < DL_THREADS / 32; ++i) ss += red[i];  // fixed order; read between the chunk's two barriers, written outside of them
     const float sigma = sqrtf(ss / float(cnt > 1 ? cnt - 1 : 1));
     float scale = 6.f * sigma / 256.f;
     if (!(scale > 0.f) || isinf(scale)) scale = 1.f;         // all-zero chunk (e.g. a fake pseudo-gradient)
@@ -300,7 +295,9 @@ __device__ __forceinline__ void dl_quantize_chunk(float (&v)[DL_PER_THREAD], lon
         unsigned sum = 0, c = 0;
 #pragma unroll
         for (int l = 0; l < 16; ++l) {
-            const unsigned x = s_bin[(b << 5) + ((16 * h + l + b) & 31)];     // rotated: a warp reads 32 different banks
+            unsigned& word = s_bin[(b << 5) + ((16 * h + l + b) & 31)];       // rotated: a warp reads 32 different banks
+            const unsigned x = word;
+            word = 0u;
             c += x >> DL_CNT_SHIFT;
             sum += x & ((1u << DL_CNT_SHIFT) - 1u);
         }
@@ -313,9 +310,12 @@ __device__ __forceinline__ void dl_quantize_chunk(float (&v)[DL_PER_THREAD], lon
             c = s_edge_cnt[b ? 1 : 0];
             if (c) mean = float(double(static_cast<long long>(s_edge_sum[b ? 1 : 0])) / double(1 << DL_EDGE_FX_BITS) / double(c)) * scale;
         }
-        if (!h) lut_chunk[b] = mean;
+        __syncwarp();
+        if (!h) {
+            lut_chunk[b] = mean;
+            if (b == 0 || b == 255) { s_edge_sum[b ? 1 : 0] = 0ull; s_edge_cnt[b ? 1 : 0] = 0u; }
+        }
     }
-    __syncthreads();       // the shared table is reused by the CTA's next chunk
 }
 
 __device__ __forceinline__ void dl_cp_async16(uint32_t dst, const void* src) {
@@ -337,7 +337,8 @@ __global__ void __launch_bounds__(DL_THREADS, 2) dl_stage_a_kernel(DlPeers p, co
     uint8_t* q = p.q[p.rank];
     float* lut = p.lut[p.rank];
     const bool q_aligned = (reinterpret_cast<uintptr_t>(q) & 3) == 0;
-    __shared__ __align__(16) unsigned s_tab[DL_TABLE];
+    __shared__ __align__(16) unsigned s_tab[DL_TABLE_WORDS];
+    dl_table_clear(s_tab);
     extern __shared__ float4 s_next[];     // [DL_CHUNK / 4] without b
     const bool ahead = !HAS_B && aligned && !fake;
     auto fetch = [&](long long chunk) {    // whole chunks only; a ragged last one is loaded directly
@@ -399,7 +400,8 @@ __device__ __forceinline__ int dl_owner(unsigned mask, long long chunk, long lon
 // ---- stage B: pull every active rank's bytes for my chunks, dequantise with that rank's codebook, sum, re-quantise ----
 __global__ void __launch_bounds__(DL_THREADS, 2) dl_stage_b_kernel(DlPeers p, long long n, int epoch, int prev_epoch, unsigned* counter,
                                                                 int* status, unsigned long long budget_ns) {
-    __shared__ __align__(16) unsigned s_tab[DL_TABLE];   // histogram of the re-quantisation
+    __shared__ __align__(16) unsigned s_tab[DL_TABLE_WORDS];   // histogram of the re-quantisation
+    dl_table_clear(s_tab);
     extern __shared__ float s_lut[];       // [world][256]: every active rank's codebook of the current chunk
     const long long chunks = (n + DL_CHUNK - 1) / DL_CHUNK;
     const int m = __popc(p.mask);
