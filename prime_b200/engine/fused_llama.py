@@ -602,7 +602,7 @@ class FusedLlama:
         do = self._buf("do", (M, H * hd))
         # dO = dh @ wo; the dO . O row sums of the attention backward come out of the same kernel where it applies
         dots = A.row_dots_buffer(dh.device, M, H, max(hd // 64, 1)) if dh.is_cuda else None
-        if dots is None or not K.gemm_rowdot(dh, self.w[pre + "attention.wo.weight"], do, o, dots, hd, b_mn=True):
+        if dots is None or not K.gemm_rowdot(dh, self.w[pre + "attention.wo.weight"], do, o, dots, hd, b_mn=True, as_stored=True):
             K.gemm(dh, self.w[pre + "attention.wo.weight"], out=do, b_mn=True)
             dots = None
         self._wgrad(dh, o, self.g[pre + "attention.wo.weight"])

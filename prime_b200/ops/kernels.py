@@ -241,16 +241,19 @@ def gemm_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, table: torch.
 
 
 def gemm_rowdot(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, other: torch.Tensor, dots: torch.Tensor, group: int,
-                b_mn: bool = False) -> bool:
+                b_mn: bool = False, as_stored: bool = False) -> bool:
     """``out = a @ op(b).T`` (bf16) and ``dots[g, m] = sum_{c in group g} out_fp32[m, c] * other[m, c]`` for column groups of
-    ``group`` columns (64, or a multiple: then ``dots`` holds the partial sums of every 64, ``[N / group, group / 64, M]``), in one kernel (the dO . O row sums of the attention backward, taken in the epilogue of the
-    GEMM that produces dO). Returns False without touching anything when the fused kernel does not apply."""
+    ``group`` columns (64, or a multiple: then ``dots`` holds the partial sums of every 64, ``[N / group, group / 64, M]``), in one
+    kernel, in the epilogue of the GEMM. Returns False without touching anything when the fused kernel does not apply.
+    ``as_stored``: the sums are over ``out`` as it is stored. The dO . O sums of the attention backward have to be those:
+    dS = P * (dO V^T - dO . O) is a small difference wherever the rows of V have much in common, and it keeps the rounding of dO
+    unless both terms have the same one."""
     M = a.shape[0]
     N = b.shape[1] if b_mn else b.shape[0]
     if not (a.is_cuda and _pair_ok(M, N) and group % 64 == 0 and N % group == 0 and out.stride(-1) == 1 and other.stride(-1) == 1
             and other.shape == out.shape and dots.is_contiguous() and dots.numel() >= (N // 64) * M):
         return False
-    _gemm_epi(a, b, out, M, N, a.shape[1], b_mn, 4, 64, 0, 0, other, "rowdot", aux2=dots)
+    _gemm_epi(a, b, out, M, N, a.shape[1], b_mn, 4, 64, int(as_stored), 0, other, "rowdot", aux2=dots)
     return True
 
 

@@ -229,3 +229,49 @@ def test_gemm_row_parts(K, N, rows):
     assert [tuple(o.shape) for o in outs] == [(n, N) for n in rows] and all(o.is_contiguous() and o.dtype == torch.float32 for o in outs)
     assert len({o.untyped_storage().data_ptr() for o in outs}) == len(outs)
     assert _rel(torch.cat(outs), ref) < 1e-3
+
+
+# dP and the dO . O sums have to come from one and the same dO: rows of V that have a large part in common (here five times their
+# spread) leave of dP - D little but what the two terms differ by
+@pytest.mark.parametrize("hd", [64, 128])
+def test_row_dots_of_the_engine_are_those_of_the_stored_gradient(hd, monkeypatch):
+    from prime_b200.engine.fused_llama import FusedLlama
+    from prime_b200.models.llama import ModelArgs
+    T, H = 600, 512 // hd
+    eng = FusedLlama(ModelArgs(dim=512, n_layers=1, n_heads=H, ffn_hidden=512, vocab_size=1024, max_seq_len=T, init_mode="normal"),
+                     device="cuda", ce_chunk_tokens=512)
+    eng.init_weights(seed=3)
+    seen = []
+    whole = A.attention_bwd
+
+    def check_dots(qkv, o, do, *args, row_dots=None, **kw):
+        terms = (do.double() * o.double()).view(T, H, hd // 64, 64)
+        want, size = terms.sum(-1).permute(1, 2, 0), terms.abs().sum(-1).permute(1, 2, 0)
+        # 64 products of bf16 pairs are exact in fp32, their sum takes 64 roundings
+        seen.append(bool(((row_dots.view(H, hd // 64, T).double() - want).abs() <= 64 * 2.0 ** -24 * size).all()))
+        return whole(qkv, o, do, *args, row_dots=row_dots, **kw)
+    monkeypatch.setattr(A, "attention_bwd", check_dots)
+    ids = torch.randint(0, 1024, (1, T + 1), device="cuda")
+    eng.forward_backward(ids[:, :-1].contiguous(), ids[:, 1:].contiguous())
+    ops.check_status()
+    assert seen == [True]
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_attention_backward_of_values_with_a_common_part(hd):
+    torch.manual_seed(0)
+    M, H, KV = 1024, 4, 2
+    qkv = torch.randn(M, (H + 2 * KV) * hd, device="cuda") * 0.7
+    qkv[:, (H + KV) * hd:] += 3.5
+    qkv, ss = qkv.bfloat16(), A.seq_start_from_batch(1, M, "cuda")
+    o, lse2 = A.attention_fwd(qkv, ss, H, KV, hd)
+    dh = torch.randn(M, 512, device="cuda").bfloat16()
+    wo = (torch.randn(512, H * hd, device="cuda") * 512 ** -0.5).bfloat16()
+    do = torch.empty(M, H * hd, device="cuda", dtype=torch.bfloat16)
+    dots = A.row_dots_buffer(do.device, M, H, hd // 64)
+    assert ops.gemm_rowdot(dh, wo, do, o, dots, hd, b_mn=True, as_stored=True)
+    got = A.attention_bwd(qkv, o, do, lse2, ss, H, KV, hd, row_dots=dots.clone())
+    want = A.attention_bwd(qkv, o, do, lse2, ss, H, KV, hd)
+    ops.check_status()
+    # the two differ in the order of fp32 sums only: now and then a value falls on the other side of a bf16 rounding (2^-8)
+    assert _rel(got, want) < 1e-3
