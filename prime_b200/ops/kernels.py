@@ -168,7 +168,7 @@ def _splitk_slices(M: int, N: int, K: int, device) -> int:
     which its pipeline never fills."""
     if N % 4 or K < 2048 or M < 256 or N < 256:
         return 1
-    pairs = torch.cuda.get_device_properties(device).multi_processor_count // 2
+    pairs = _cta_pairs(device)
     tiles = ((M + 255) // 256) * ((N + 255) // 256)
     if tiles * 4 > pairs * 3:
         return 1
@@ -187,6 +187,21 @@ def _pair_ok(M: int, N: int) -> bool:
     return _GEMM_PAIR and M >= 512 and N >= 256
 
 
+@functools.lru_cache(maxsize=16)
+def _cta_pairs(device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count // 2
+
+
+def _narrow_swiglu_pays(M: int, F: int, K: int, pairs: int) -> bool:
+    """Whether an odd number of 64-feature blocks is worth the fused kernel. Its tiles are then 128 columns wide (64 gate, 64 up)
+    whatever their number, and read an operand half more often per product than the 256-wide ones of the plain GEMM; what they
+    save is the pass of swiglu_fwd. GEMM + pass against fused, us: a short K always pays ([16384 x 2 * 704 x 384] 42.0 and 37.9,
+    [65536 x 2 * 320 x 384] 74.7 and 60.4), a longer one while every tile has a CTA pair to itself ([1024 x 2 * 704 x 1536] 21.5
+    and 19.5), but not with more tiles than pairs ([16384 x 2 * 1472 x 512] 74.7 and 76.2, [4096 x 2 * 320 x 1024] 21.5 and 23.5,
+    [65536 x 2 * 704 x 1024] 189 and 236), nor from where the plain GEMM may split K ([512 x 2 * 192 x 2048] 19.5 and 21.5)."""
+    return K <= 384 or (K < 2048 and (M + 255) // 256 * (F // 64) <= pairs)
+
+
 def _gemm_epi(a, b, out, M, N, K, b_mn, epi, i0, i1, i2, aux, what, aux2=None, a_mn=False):
     rc = native.cuda().pb_gemm_bf16_pair_epi(ptr(a), ptr(b), ptr(out), None, M, N, K, a.stride(0), b.stride(0),
                                              out.stride(0) if out is not None else 0, 0, int(a_mn), int(b_mn), 0, 0, epi, i0, i1, i2,
@@ -201,7 +216,8 @@ def gemm_swiglu(x: torch.Tensor, w13: torch.Tensor, h13: torch.Tensor, act: torc
     back to GEMM + swiglu_fwd where the fused kernel does not apply (CPU, small or odd shapes)."""
     M, K = x.shape
     F = w13.shape[0] // 2
-    if x.is_cuda and _pair_ok(M, 2 * F) and F % 64 == 0 and h13.stride(-1) == 1 and act.stride(-1) == 1:
+    if (x.is_cuda and _pair_ok(M, 2 * F) and (F % 128 == 0 or F % 64 == 0 and _narrow_swiglu_pays(M, F, K, _cta_pairs(x.device)))
+            and h13.stride(-1) == 1 and act.stride(-1) == 1):
         _gemm_epi(x, w13, h13, M, 2 * F, K, False, 1, F, 0, 0, act, "swiglu")
         return h13, act
     gemm(x, w13, out=h13)

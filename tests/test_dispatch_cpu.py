@@ -89,3 +89,9 @@ def test_scratch_belongs_to_one_thread_and_is_bounded(monkeypatch):
         assert K._scratch_buf(dev, "splitk", 100).data_ptr() == mine.data_ptr() and len(K._scratch) <= 64
     got = K.take_scratch(type("S", (), {"cuda_stream": 7})())
     assert any(g.data_ptr() == mine.data_ptr() for g in got) and not any(k[3] == threading.get_ident() for k in K._scratch)
+
+
+def test_odd_swiglu_blocks_are_fused_up_to_the_measured_lines():
+    fits = [(512, 192, 1536), (1024, 704, 1536), (65536, 2752, 384)]
+    loses = [(1024, 1472, 1024), (65536, 704, 392), (512, 192, 2048), (4736, 320, 512)]
+    assert all(K._narrow_swiglu_pays(*s, 74) for s in fits) and not any(K._narrow_swiglu_pays(*s, 74) for s in loses)

@@ -275,3 +275,21 @@ def test_attention_backward_of_values_with_a_common_part(hd):
     ops.check_status()
     # the two differ in the order of fp32 sums only: now and then a value falls on the other side of a bf16 rounding (2^-8)
     assert _rel(got, want) < 1e-3
+
+
+# An odd number of 64-feature blocks: one launch where the narrow tiles of the fused kernel pay, GEMM and SwiGLU pass where they do not
+@pytest.mark.parametrize("M,F,K,launches", [(1024, 704, 384, 1), (16384, 704, 384, 1), (1024, 704, 1536, 1), (16384, 704, 392, 2), (4096, 320, 1024, 2),
+                                            (512, 192, 2048, 3)])
+def test_swiglu_of_odd_blocks_is_fused_where_that_is_faster(M, F, K, launches):
+    from prime_b200 import native
+    torch.manual_seed(0)
+    x = torch.randn(M, K, device="cuda").bfloat16()
+    w13 = (torch.randn(2 * F, K, device="cuda") * K ** -0.5).bfloat16()
+    h13, act = torch.empty(M, 2 * F, device="cuda", dtype=torch.bfloat16), torch.empty(M, F, device="cuda", dtype=torch.bfloat16)
+    before = native.launch_counter()
+    ops.gemm_swiglu(x, w13, h13, act)
+    assert native.launch_counter() - before == launches          # (a product that is split over K has a reduce)
+    ref = x.float() @ w13.float().t()
+    ops.check_status()
+    assert _rel(h13, ref) < 1e-2
+    assert _rel(act, torch.nn.functional.silu(ref[:, :F]) * ref[:, F:]) < 1e-2
