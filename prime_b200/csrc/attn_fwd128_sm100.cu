@@ -6,7 +6,7 @@
 // each; warp 1 owns TMEM), warp 3 only fills the warpgroup; warps 4-7 and 8-11 softmax of the first and the second tile (one
 // thread per query row: row max / sum are thread-local). The exponentials of one tile run under the MMAs of the other; the first
 // warpgroup gives registers up (setmaxnreg) so that a softmax thread can hold its 128-wide score row without spilling.
-// The grid has a CTA for every pair of tiles, but a CTA that runs takes over the work of CTAs that have not started
+// The grid has a CTA for every pair of tiles of every head, but a CTA that runs takes over the work of CTAs that have not started
 // (clusterlaunchcontrol), so that barriers and tensor memory are set up once per SM and the next pair's Q, K and V arrive under the
 // end of this one, while the hardware still deals the pairs out one by one. Every issuer and softmax group moves on to the next
 // pair by itself.
@@ -38,18 +38,16 @@ __device__ __forceinline__ void clc_request(uint32_t answer, uint32_t bar) {
     mbar_expect_tx(bar, 16);
     asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer), "r"(bar) : "memory");
 }
-__device__ __forceinline__ bool clc_answer(uint32_t answer, int& x, int& y) {
+__device__ __forceinline__ bool clc_answer(uint32_t answer, int& x) {
     uint32_t got;
     asm volatile(
         "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\t"
-        "ld.shared.b128 h, [%3];\n\t"
+        "ld.shared.b128 h, [%2];\n\t"
         "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t"
         "mov.b32 %1, 0;\n\t"
-        "mov.b32 %2, 0;\n\t"
-        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t"
-        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::y.b32.b128 %2, h;\n\t}\n"
-        : "=r"(got), "=r"(x), "=r"(y)
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}\n"
+        : "=r"(got), "=r"(x)
         : "r"(answer)
         : "memory");
     return got != 0;
@@ -62,7 +60,7 @@ struct FwdItem {
 };
 
 __global__ void __launch_bounds__(384, 1)
-attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p, const int per_cta) {
+attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p, const int per_cta, const int n_units) {
     using Cfg = AttnFwd128Cfg;
     constexpr int HD = 128, TILE = Cfg::TILE_BYTES, RING = Cfg::RING;
     extern __shared__ uint8_t smem_raw[];
@@ -143,11 +141,11 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p
         if (warp == 0) {
             // ------------------------------ TMA producer ------------------------------
             bool ok = true;
-            int x = blockIdx.x, head = blockIdx.y;
+            int x = blockIdx.x;                  // number of the CTA whose work this is; -1: none left
             uint32_t nq[2] = {0, 0};             // query tiles loaded
             int slot = 0;                        // next K / V slot of the ring
             uint32_t ph = 0;
-            auto load_q = [&](int g, int tile) -> bool {
+            auto load_q = [&](int g, int head, int tile) -> bool {
                 if (!wait_warp(bar_qempty + 8 * g, nq[g] ^ 1, PB_ERR_TIMEOUT_EMPTY)) return false;
                 ++nq[g];
                 if (lane == 0) {
@@ -170,8 +168,9 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p
                 return true;
             };
             for (int k = 0;; ++k) {
-                const bool have = head >= 0;
-                const int tile = (int(gridDim.x) - 1 - x) * per_cta;          // latest (heaviest) tiles first
+                const bool have = x >= 0;
+                const int head = have ? x % p.H : -1;
+                const int tile = have ? (n_units - 1 - x / p.H) * per_cta : 0;     // latest (heaviest) tiles of all heads first
                 int lo0 = 0, lo1 = 0;
                 const bool two = per_cta == 2 && tile + 1 < n_tiles;
                 if (have) {
@@ -182,17 +181,17 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p
                 if (!ok) break;
                 if (lane == 0) {
                     volatile int* e = ring + 4 * (k & 3);
-                    e[0] = tile; e[1] = have ? head : -1; e[2] = lo0; e[3] = lo1;
+                    e[0] = tile; e[1] = head; e[2] = lo0; e[3] = lo1;
                     mbar_arrive(bar_ifull + 8 * (k & 3));
                 }
                 __syncwarp();
                 if (!have) break;
                 const int kvh = head / (p.H / p.KV);
                 const int lo = min(lo0, lo1), hi = two ? tile + 1 : tile;
-                ok = load_q(0, tile);
+                ok = load_q(0, head, tile);
                 for (int j = lo; j <= hi && ok; ++j) {
                     ok = load_kv(p.H + kvh, j);
-                    if (ok && j == lo && two) ok = load_q(1, tile + 1);
+                    if (ok && j == lo && two) ok = load_q(1, head, tile + 1);
                     if (ok) ok = load_kv(p.H + p.KV + kvh, j);
                 }
                 if (!ok) break;
@@ -204,11 +203,10 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p
                 __syncwarp();
                 ok = wait_warp(bar_clc, k, PB_ERR_TIMEOUT_MISC);
                 if (!ok) break;
-                int nx, ny;
-                const bool got = clc_answer(clc_slot, nx, ny);
+                int nx;
+                const bool got = clc_answer(clc_slot, nx);
                 __syncwarp();
-                x = nx;
-                head = got ? ny : -1;
+                x = got ? nx : -1;
             }
             if (!ok) for (int i = 0; i < 64; ++i) __nanosleep(10000);
         } else if (warp < 3) {
@@ -426,7 +424,13 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p
     }
 }
 
-// Two tiles per CTA, but one where every tile then has an SM to itself.
+// Two tiles per CTA, but one where every tile then has an SM to itself. CTAs are numbered with the head running fastest, so that the
+// long rows of all heads start first and the short ones fill the end: with the tiles running fastest the last heads' longest pairs
+// started late, and from 150 to 1000 tiles of long rows two to a CTA lost 5-8 % against one each. One CTA per tile; tiles fastest; heads
+// fastest, us: 1 x 4096 tokens, 16 heads 140, 149, 100; 1 x 8192, 8 heads 246, 268, 187; 32 / 8 heads 703, 666, 606; 64 x 1024, 16 heads
+// 503, 441, 429. What still loses to one CTA per tile: up to two tiles per SM of one long row (1 x 4096, 8 heads 94 and 98; one
+// tile per CTA takes 72 there, but 45 instead of 35 at 37 x 777, one head, and the launch does not know where rows end), and rows of
+// 128 tokens (8 x 128, 8 heads, one launch behind the other, 7.3 and 7.8).
 int launch_attn_fwd128(const CUtensorMap& tm, const AttnFwdParams& p, cudaStream_t st) {
     using Cfg = AttnFwd128Cfg;
     static bool configured = false;
@@ -434,9 +438,10 @@ int launch_attn_fwd128(const CUtensorMap& tm, const AttnFwdParams& p, cudaStream
         if (cudaFuncSetAttribute(attn_fwd128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess) return -20;
         configured = true;
     }
-    const int n_tiles = (p.M + 127) / 128;
-    const int per_cta = n_tiles * p.H <= sm_count() ? 1 : 2;
-    launch_pdl(attn_fwd128_kernel, LaunchCfg(dim3((n_tiles + per_cta - 1) / per_cta, p.H), 384, Cfg::SMEM_BYTES, st), tm, p, per_cta);
+    const int n_tiles = (p.M + 127) / 128, n_sm = sm_count();
+    const int per_cta = n_tiles * p.H <= n_sm ? 1 : 2;
+    const int n_units = (n_tiles + per_cta - 1) / per_cta;
+    launch_pdl(attn_fwd128_kernel, LaunchCfg(n_units * p.H, 384, Cfg::SMEM_BYTES, st), tm, p, per_cta, n_units);
     return cudaGetLastError() == cudaSuccess ? 0 : -30;
 }
 

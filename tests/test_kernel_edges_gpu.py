@@ -293,3 +293,9 @@ def test_swiglu_of_odd_blocks_is_fused_where_that_is_faster(M, F, K, launches):
     ops.check_status()
     assert _rel(h13, ref) < 1e-2
     assert _rel(act, torch.nn.functional.silu(ref[:, :F]) * ref[:, F:]) < 1e-2
+
+
+# more heads than SMs, which all come before the second tile of any; a pair and a single tile per head
+@pytest.mark.parametrize("M", [128, 300])
+def test_attention_of_more_heads_than_sms(M):
+    _attention_case((0, 100), M, 160, 80, 72, seed=5)
