@@ -203,6 +203,10 @@ def _narrow_swiglu_pays(M: int, F: int, K: int, pairs: int) -> bool:
 
 
 def _gemm_epi(a, b, out, M, N, K, b_mn, epi, i0, i1, i2, aux, what, aux2=None, a_mn=False):
+    # what the C entry cannot see from addresses and pitches, for the products that would otherwise have gone through gemm() too
+    assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.stride(-1) == 1 and b.stride(-1) == 1
+    assert tuple(a.shape) == ((K, M) if a_mn else (M, K)) and tuple(b.shape) == ((K, N) if b_mn else (N, K)), "operands do not fit each other"
+    assert out is None or out.dtype == torch.bfloat16
     rc = native.cuda().pb_gemm_bf16_pair_epi(ptr(a), ptr(b), ptr(out), None, M, N, K, a.stride(0), b.stride(0),
                                              out.stride(0) if out is not None else 0, 0, int(a_mn), int(b_mn), 0, 0, epi, i0, i1, i2,
                                              ptr(aux), aux.stride(0) if aux.dim() == 2 else 0, ptr(aux2),
@@ -256,6 +260,13 @@ def gemm_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, table: torch.
     return out
 
 
+def _rowdot_fits(M: int, N: int, out: torch.Tensor, other: torch.Tensor, dots: torch.Tensor, group: int) -> bool:
+    """Both matrices come and go by TMA: bf16 rows of whole 16-byte units."""
+    return (_pair_ok(M, N) and group % 64 == 0 and N % group == 0 and out.shape == other.shape == (M, N)
+            and all(t.dtype == torch.bfloat16 and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (out, other))
+            and dots.dtype == torch.float32 and dots.is_contiguous() and dots.numel() >= (N // 64) * M)
+
+
 def gemm_rowdot(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, other: torch.Tensor, dots: torch.Tensor, group: int,
                 b_mn: bool = False, as_stored: bool = False) -> bool:
     """``out = a @ op(b).T`` (bf16) and ``dots[g, m] = sum_{c in group g} out_fp32[m, c] * other[m, c]`` for column groups of
@@ -266,8 +277,7 @@ def gemm_rowdot(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, other: torc
     unless both terms have the same one."""
     M = a.shape[0]
     N = b.shape[1] if b_mn else b.shape[0]
-    if not (a.is_cuda and _pair_ok(M, N) and group % 64 == 0 and N % group == 0 and out.stride(-1) == 1 and other.stride(-1) == 1
-            and other.shape == out.shape and dots.is_contiguous() and dots.numel() >= (N // 64) * M):
+    if not (a.is_cuda and _rowdot_fits(M, N, out, other, dots, group)):
         return False
     _gemm_epi(a, b, out, M, N, a.shape[1], b_mn, 4, 64, int(as_stored), 0, other, "rowdot", aux2=dots)
     return True

@@ -95,3 +95,43 @@ def test_odd_swiglu_blocks_are_fused_up_to_the_measured_lines():
     fits = [(512, 192, 1536), (1024, 704, 1536), (65536, 2752, 384)]
     loses = [(1024, 1472, 1024), (65536, 704, 392), (512, 192, 2048), (4736, 320, 512)]
     assert all(K._narrow_swiglu_pays(*s, 74) for s in fits) and not any(K._narrow_swiglu_pays(*s, 74) for s in loses)
+
+
+class _NoLaunch:
+    """Stands in for the CUDA library: every entry only notes that it was reached."""
+    def __init__(self):
+        self.reached = []
+
+    def __getattr__(self, name):
+        return lambda *a: self.reached.append(name) or 0
+
+
+def test_fused_products_refuse_operands_that_the_plain_product_refuses(monkeypatch):
+    lib = _NoLaunch()
+    monkeypatch.setattr(native, "cuda", lambda: lib)
+    monkeypatch.setattr(native, "stream_ptr", lambda *a: None)
+    monkeypatch.setattr(K, "stream_ptr", lambda *a: None)
+    monkeypatch.setattr(K, "status_word", lambda d: torch.zeros(1, dtype=torch.int32))
+    x, w, h, act = (torch.zeros(*s, dtype=torch.bfloat16) for s in ((512, 128), (384, 128), (512, 384), (512, 192)))
+
+    def call(x, w, h13=h):
+        K._gemm_epi(x, w, h13, 512, 384, 128, False, 1, 192, 0, 0, act, "swiglu")
+    wide = torch.zeros(512, 256, dtype=torch.bfloat16)
+    for bad in ((x.float(), w), (x, w.float()), (x.half(), w), (wide[:, ::2], w), (x, torch.zeros(384, 256, dtype=torch.bfloat16)[:, ::2]),
+                (x, torch.zeros(384, 136, dtype=torch.bfloat16)), (x, w, h.float())):
+        with pytest.raises(AssertionError):
+            call(*bad)
+    assert not lib.reached
+    call(x, w)
+    assert lib.reached
+
+
+@pytest.mark.parametrize("group", [64, 128])
+def test_row_dots_do_not_apply_to_rows_that_tma_cannot_move(group):
+    out, dots = torch.zeros(512, 256, dtype=torch.bfloat16), torch.zeros(4 * 512)
+    wide = torch.zeros(512, 272, dtype=torch.bfloat16)
+    assert K._rowdot_fits(512, 256, out, out, dots, group) and K._rowdot_fits(512, 256, wide[:, 8:264], out, dots, group)
+    for bad in (wide[:, 1:257], torch.zeros(512, 260, dtype=torch.bfloat16)[:, :256], torch.zeros(256, 512, dtype=torch.bfloat16).t(), out.float(),
+                out[:, :128]):
+        assert not K._rowdot_fits(512, 256, bad, out, dots, group) and not K._rowdot_fits(512, 256, out, bad, dots, group)
+    assert not K._rowdot_fits(512, 256, out, out, dots[:-1], group) and not K._rowdot_fits(512, 256, out, out, dots.double(), group)
