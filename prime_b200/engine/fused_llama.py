@@ -125,9 +125,7 @@ class _StepGraph:
             K.take_scratch(st)                           # of earlier users of this handle: the graph gets its own
         # The kernels of a step small enough for a graph leave most SMs idle, so the weight gradients become a branch beside the
         # chain of input gradients: two-block model of 512 tokens 328 -> 272 us, debug model's step 1331 -> 1165
-        eng.wgrad_stream = wgrads
-        # the norms' too, as long as their partial sums fit the scratch table side by side
-        eng._norm_dw_stream = wgrads if eng.args.n_layers <= 15 else None
+        eng.wgrad_stream = eng._norm_dw_stream = wgrads
         before = native.launch_counter()
         with torch.cuda.stream(side):
             self.graph.capture_begin(capture_error_mode="thread_local")
@@ -139,6 +137,7 @@ class _StepGraph:
                 self.graph.capture_end()
                 eng._accum = False
                 eng.wgrad_stream = eng._norm_dw_stream = None
+                eng._branch_open = False
                 eng._readers.clear()
         main.wait_stream(side)
         self.launches = native.launch_counter() - before
@@ -225,6 +224,7 @@ class FusedLlama:
         self.wgrad_stream = torch.cuda.Stream(device=dev) if (dev.type == "cuda" and os.environ.get("PRIME_B200_WGRAD_STREAM", "0") == "1") \
             else None
         self._readers: dict[int, torch.cuda.Event] = {}
+        self._branch_open = False       # the weight-gradient stream has work that the main stream has not waited for
         self._norm_dw_stream = None     # norm weight gradients beside the chain of input gradients: recorded steps only
         # parameter views -----------------------------------------------------------------------
         self.w: dict[str, torch.Tensor] = {}
@@ -554,8 +554,15 @@ class FusedLlama:
             K.gemm(dy, x, out=g, residual=g if self._accum else None, a_mn=True, b_mn=True)
             done = torch.cuda.Event()
             done.record(ws)
+        self._branch_open = True
         self._readers[dy.data_ptr()] = done
         self._readers[x.data_ptr()] = done
+
+    def _norm_bwd(self, x: torch.Tensor, name: str, rstd: torch.Tensor, dy: torch.Tensor, dx: torch.Tensor,
+                  dres: torch.Tensor | None = None) -> None:
+        """dx = (gradient of the norm's input) + dres; the gradient of its weight beside the chain where there is a stream for it"""
+        K.rmsnorm_bwd(x, self.w[name], rstd, dy, self.g[name], dres=dres, dx=dx, accumulate_dw=self._accum, dw_stream=self._norm_dw_stream)
+        self._branch_open |= self._norm_dw_stream is not None
 
     def _before_write(self, *tensors: torch.Tensor) -> None:
         """The main stream is about to overwrite these tensors: wait for weight-gradient GEMMs that still read them."""
@@ -568,8 +575,9 @@ class FusedLlama:
                 main.wait_event(ev)
 
     def _wait_all_wgrads(self) -> None:
-        if self.wgrad_stream is not None and self._readers:
+        if self.wgrad_stream is not None and (self._branch_open or self._readers):
             torch.cuda.current_stream().wait_stream(self.wgrad_stream)
+            self._branch_open = False
             self._readers.clear()
 
     def _block_bwd(self, i: int, x: torch.Tensor, dout: torch.Tensor, T: int, seq_start: torch.Tensor, dx: torch.Tensor) -> None:
@@ -596,8 +604,7 @@ class FusedLlama:
         self._wgrad(h13, hn, self.g13[i])
         dh = self._buf("dh", (M, D))
         self._before_write(dh)
-        K.rmsnorm_bwd(h, self.w[pre + "ffn_norm.weight"], rstd2, dhn, self.g[pre + "ffn_norm.weight"], dres=dout, dx=dh,
-                      accumulate_dw=self._accum, dw_stream=self._norm_dw_stream)
+        self._norm_bwd(h, pre + "ffn_norm.weight", rstd2, dhn, dh, dres=dout)
         # h = x + o @ wo^T
         do = self._buf("do", (M, H * hd))
         # dO = dh @ wo; the dO . O row sums of the attention backward come out of the same kernel where it applies
@@ -613,8 +620,7 @@ class FusedLlama:
         K.gemm(dqkv, self.wqkv[i], out=dxn, b_mn=True)
         self._wgrad(dqkv, xn, self.gqkv[i])
         self._before_write(dx)
-        K.rmsnorm_bwd(x, self.w[pre + "attention_norm.weight"], rstd1, dxn, self.g[pre + "attention_norm.weight"], dres=dh,
-                      dx=dx, accumulate_dw=self._accum, dw_stream=self._norm_dw_stream)
+        self._norm_bwd(x, pre + "attention_norm.weight", rstd1, dxn, dx, dres=dh)
         if self._reduce_in_backward:
             self._reduce_group(1 + i, overlapped=True)     # this block's gradients are final: reduce them under the next block's backward
 
@@ -672,7 +678,7 @@ class FusedLlama:
         K.loss_sums(loss_rows, z_rows, inv, self.z_weight, out, self._partials if on_gpu else None,
                     self._counters[3:] if on_gpu else None, acc=loss_acc, acc_scale=loss_scale, acc_first=first_microbatch)
         dx = self._buf("dx_a", (M, D))
-        K.rmsnorm_bwd(xs[L], self.w["norm.weight"], rstd, dhn, self.g["norm.weight"], dx=dx, accumulate_dw=self._accum, dw_stream=self._norm_dw_stream)
+        self._norm_bwd(xs[L], "norm.weight", rstd, dhn, dx)
         if self._reduce_in_backward:
             self._reduce_group(L + 1, overlapped=True)     # head group (final norm + output projection)
         # ---- blocks in reverse ----

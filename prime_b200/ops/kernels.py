@@ -305,8 +305,9 @@ def rmsnorm_fwd(x: torch.Tensor, w: torch.Tensor, eps: float, out: torch.Tensor 
 
 def rmsnorm_bwd(x, w, rstd, dy, dw: torch.Tensor, dres: torch.Tensor | None = None, dx: torch.Tensor | None = None,
                 accumulate_dw: bool = True, dw_stream: torch.cuda.Stream | None = None):
-    """Returns dx (= norm input gradient + ``dres``) and adds the weight gradient into ``dw``, on ``dw_stream`` if there is one (the
-    partial sums then lie in a scratch of this ``dw``'s own)."""
+    """Returns dx (= norm input gradient + ``dres``) and adds the weight gradient into ``dw``: with ``dw_stream`` on that stream, beside
+    what the current one does next. The partial sums then are a tensor of this call's own, which the allocator keeps until that
+    stream has read it; whoever reads or writes ``dw`` elsewhere waits for ``dw_stream`` first."""
     M, N = x.shape
     if dx is None:
         dx = torch.empty_like(x)
@@ -322,7 +323,7 @@ def rmsnorm_bwd(x, w, rstd, dy, dw: torch.Tensor, dres: torch.Tensor | None = No
         return dx
     lib = native.cuda()
     ctas = lib.pb_rmsnorm_bwd_ctas()
-    part = _scratch_buf(x.device, "rms_bwd" if dw_stream is None else f"rms_bwd.{dw.data_ptr()}", ctas * N)
+    part = _scratch_buf(x.device, "rms_bwd", ctas * N) if dw_stream is None else torch.empty(ctas * N, dtype=torch.float32, device=x.device)
     check(lib.pb_rmsnorm_bwd(ptr(x), ptr(w), ptr(rstd), ptr(dy), ptr(dres), ptr(dx), ptr(part), ptr(dw) if dw_stream is None else None,
                              int(dw.dtype == torch.float32), int(accumulate_dw), M, N, stream_ptr()),
           "pb_rmsnorm_bwd" if dw_stream is None else "pb_rmsnorm_bwd without dw")
@@ -330,6 +331,7 @@ def rmsnorm_bwd(x, w, rstd, dy, dw: torch.Tensor, dres: torch.Tensor | None = No
         dw_stream.wait_stream(torch.cuda.current_stream(x.device))
         check(lib.pb_rmsnorm_bwd_dw(ptr(part), ptr(dw), int(dw.dtype == torch.float32), int(accumulate_dw), M, N, stream_ptr(dw_stream)),
               "pb_rmsnorm_bwd_dw")
+        part.record_stream(dw_stream)
     return dx
 
 

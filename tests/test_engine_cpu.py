@@ -254,6 +254,27 @@ def test_update_without_peers_waits_for_the_weight_gradient_stream(monkeypatch):
     assert eng.grad_shard is not None and order == ["join"]
 
 
+def test_norm_gradients_beside_the_chain_are_waited_for_by_themselves(monkeypatch):
+    """No weight-gradient GEMM that could stand for them has left an entry."""
+    from prime_b200.engine import fused_llama
+    _, eng = _mk(_tiny())
+    joined = []
+
+    class Stream:
+        def wait_stream(self, s):
+            joined.append(s)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: Stream())
+    monkeypatch.setattr(fused_llama.K, "rmsnorm_bwd", lambda *a, dw_stream, **k: None)
+    side = object()
+    for stream, want in ((side, [side]), (None, [])):
+        joined.clear()
+        eng.wgrad_stream, eng._norm_dw_stream = side, stream
+        eng._norm_bwd(None, "norm.weight", None, None, None)
+        for _ in range(2):                     # the second time there is nothing left to wait for
+            eng._wait_all_wgrads()
+            assert joined == want
+
+
 @pytest.mark.parametrize("micro", [1, 2, 4])
 def test_row_maps_reach_the_kernels_dense(monkeypatch, micro):
     """Every second element of a longer tensor, or one value for all rows: a micro-batch gets its own dense part, the first one too."""
