@@ -514,7 +514,8 @@ static int launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tdo, const 
 }  // namespace pb
 
 // dq_acc: fp32 [M, H*HD] scratch (zeroed here); D: fp32 [H, M] scratch, computed here from o and dout unless o is
-// null (then the caller has already filled it with [H, d_parts, M] partial sums). Writes all of dqkv.
+// null (then the caller has already filled it with [H, d_parts, M] partial sums: one, or two for heads of more than 64 columns).
+// Writes all of dqkv.
 // rope_table != null: the inverse rotation is applied to dq and dk on the way out (position = row % T).
 // tile_scratch: >= ceil(M / 128) + 1 ints of device scratch (query-tile count of every kv tile and the work counter).
 extern "C" int pb_attn_bwd_parts(const void* qkv, const void* o, const void* dout, const float* lse2, const int* seq_start,
@@ -524,6 +525,7 @@ extern "C" int pb_attn_bwd_parts(const void* qkv, const void* o, const void* dou
     using namespace pb;
     if (HD <= 0 || HD > 128 || HD % 8) return -1;
     if (H % KV) return -1;
+    if (!o && d_parts != 1 && (d_parts != 2 || HD <= 64)) return -4;      // the kernel for heads of up to 64 columns reads whole sums
     if ((qkv_stride % 8) || (o_stride % 8) || (do_stride % 8) || (dqkv_stride % 8) ||
         ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dqkv)) & 15))
         return -2;

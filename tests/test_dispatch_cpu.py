@@ -135,3 +135,18 @@ def test_row_dots_do_not_apply_to_rows_that_tma_cannot_move(group):
                 out[:, :128]):
         assert not K._rowdot_fits(512, 256, bad, out, dots, group) and not K._rowdot_fits(512, 256, out, bad, dots, group)
     assert not K._rowdot_fits(512, 256, out, out, dots[:-1], group) and not K._rowdot_fits(512, 256, out, out, dots.double(), group)
+
+
+@no_device
+def test_attention_backward_refuses_partial_sums_that_its_kernels_do_not_read():
+    lib = _lib()
+    from prime_b200.ops import attention  # noqa: F401  (declares the C signatures)
+    base = C.c_void_p(1 << 40)
+
+    def call(hd, d_parts, o=None):
+        n = 4 * hd
+        return lib.pb_attn_bwd_parts(base, o, base, base, base, base, base, base, d_parts, None, 1, 256, 4, 2, hd, 2 * n, n, n, 2 * n, 0.125, None, None, None)
+    for hd, parts in ((64, 2), (32, 2), (128, 3), (128, 0), (64, 0), (128, -1)):
+        assert call(hd, parts) == -4
+    # accepted as far as this check goes (without a device the next step fails), and not asked where the kernel takes the sums itself
+    assert all(call(hd, parts) != -4 for hd, parts in ((64, 1), (128, 1), (128, 2), (96, 2))) and call(64, 2, base) != -4
