@@ -22,7 +22,7 @@
 //                     applies  m = mu*m + g ; outer -= lr*(g + mu*m) ; inner = outer   (or just writes g)
 // Values are quantised twice in total (reference: W-1 times plus a re-quantisation per all-gather
 // hop), and all ranks decode the same bytes, so they end bit-identical. Quantiser semantics follow
-// the reference (round half away from zero, empty bin -> 0, codebook = mean of the bin's members).
+// the reference (nearest bin, empty bin -> 0, codebook = mean of the bin's members), but for exact ties, which go to the even bin.
 // Bin sums are integers (fixed point), so codebooks are bit-reproducible run to run.
 // Ordering: the last CTA of a stage publishes "stage done, epoch e" to every active peer's flag pad
 // (st.release.sys); the next stage's CTAs wait for the flags they depend on with a bounded spin that reports
@@ -575,9 +575,13 @@ extern "C" int pb_dl_allreduce(void* const* q, void* const* lut, void* const* q2
     const long long chunks = (n + DL_CHUNK - 1) / DL_CHUNK;
     const int m = __builtin_popcount(mask);
     const long long per = (chunks + m - 1) / m;
+    // The codebooks of more than 15 ranks take stage B's shared memory beyond the 48 KB that need no asking (32.9 KB of table). Asked for
+    // ahead of stage A, which lets the peers start: a launch that fails behind it would leave them waiting.
+    const int lut_bytes = world * 256 * int(sizeof(float));
+    if (cudaFuncSetAttribute(dl_stage_b_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lut_bytes) != cudaSuccess) return -20;
     const unsigned long long budget = budget_ns > 0 ? (unsigned long long)budget_ns : PB_WAIT_BUDGET_NS;
     if (const int rc = dl_launch_stage_a(p, a, b, scale, fake, n, epoch, counters, 1, ST(stream))) return rc;
-    dl_stage_b_kernel<<<dl_grid(per), DL_THREADS, world * 256 * sizeof(float), ST(stream)>>>(p, n, epoch, prev_epoch, counters + 1, status,
+    dl_stage_b_kernel<<<dl_grid(per), DL_THREADS, lut_bytes, ST(stream)>>>(p, n, epoch, prev_epoch, counters + 1, status,
                                                                                           budget);
     dl_stage_c_kernel<<<dl_grid(chunks), DL_THREADS, 0, ST(stream)>>>(p, n, outer, inner, mom, lr, mu, g_out, epoch, counters + 2, status,
                                                                      budget);

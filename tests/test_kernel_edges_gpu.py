@@ -299,3 +299,76 @@ def test_swiglu_of_odd_blocks_is_fused_where_that_is_faster(M, F, K, launches):
 @pytest.mark.parametrize("M", [128, 300])
 def test_attention_of_more_heads_than_sms(M):
     _attention_case((0, 100), M, 160, 80, 72, seed=5)
+
+
+def _chunks_of_every_kind(n, chunk, grid):
+    """Neighbours, and the chunks that one CTA takes one after the other, are of different kinds: clamping bins with members, without
+    any (uniform values stay within 1.8 sigma of 3), infinities (general path), zeros, bell-shaped."""
+    torch.manual_seed(0)
+    x = torch.randn(n, device="cuda") * 1e-3
+    for c in range((n + chunk - 1) // chunk):
+        v = x[c * chunk: (c + 1) * chunk]
+        kind = (c + c // grid) % 5
+        if kind == 0:
+            v[::97] *= 300
+        elif kind == 1:
+            v.uniform_(-1e-3, 1e-3)
+        elif kind == 2:
+            v[1], v[-1] = float("inf"), -float("inf")
+        elif kind == 3:
+            v.zero_()
+    return x
+
+
+# A CTA carries its table and its clamping bins' sums from chunk to chunk: of three chunks and more per CTA, every one has to come out
+# as it does alone
+@pytest.mark.parametrize("off", [0, 1])                      # staged through shared memory, and read directly
+def test_quantizer_chunks_do_not_depend_on_those_before(off):
+    from prime_b200 import native
+    from prime_b200.ops.quant import uniform_8bit_quantize_cuda
+    chunk = native.cuda().pb_dl_chunk()
+    grid = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    n = (2 * grid + 11) * chunk + 37
+    x = torch.empty(n + off, device="cuda")[off:].copy_(_chunks_of_every_kind(n, chunk, grid))
+    q, lut = uniform_8bit_quantize_cuda(x)
+    for c in range((n + chunk - 1) // chunk):
+        s = slice(c * chunk, (c + 1) * chunk)
+        q1, lut1 = uniform_8bit_quantize_cuda(x[s])
+        assert torch.equal(q[s], q1) and torch.equal(lut[c], lut1[0]), c
+
+
+# One active rank of a group: it waits for nobody but its own earlier stages. 16 ranks are the most that there may be; their
+# codebooks take stage B beyond 48 KB of shared memory.
+@pytest.mark.parametrize("world,rank,with_b", [(1, 0, True), (16, 5, False)])
+def test_exchange_chunks_do_not_depend_on_those_before(world, rank, with_b):
+    import ctypes as C
+
+    from prime_b200 import native
+    from prime_b200.parallel import diloco_comm  # noqa: F401  (declares the C signatures)
+    lib, ptr = native.cuda(), native.ptr
+    chunk = lib.pb_dl_chunk()
+    grid = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    n = (2 * grid + 11) * chunk + 37
+    x = _chunks_of_every_kind(n, chunk, grid)
+    b = x.flip(0).contiguous().nan_to_num_(0, 0, 0) if with_b else None
+    chunks = (n + chunk - 1) // chunk
+    epoch = 0
+
+    def exchange(a, b):
+        nonlocal epoch
+        epoch += 1
+        m = a.numel()
+        bufs = [torch.zeros(m, dtype=torch.uint8, device="cuda"), torch.zeros((m + chunk - 1) // chunk, 256, device="cuda")]
+        bufs += [torch.zeros_like(t) for t in bufs]
+        flags, counters, g = torch.zeros(3 * 16, dtype=torch.int32, device="cuda"), torch.zeros(3, dtype=torch.int32, device="cuda"), torch.empty_like(a)
+        tables = [(C.c_void_p * world)(*[t.data_ptr()] * world) for t in (*bufs, flags)]
+        native.check(lib.pb_dl_allreduce(*tables, world, rank, 1 << rank, epoch, 0, 0, m, ptr(a), ptr(b), 1.0, 0, None, None, None, 0.0, 0.0, ptr(g),
+                                         ptr(counters), ptr(ops.status_word(a.device)), 1_000_000_000, native.stream_ptr()), "pb_dl_allreduce")
+        return *bufs, g
+    q, lut, q2, lut2, g = exchange(x, b)
+    ops.check_status()
+    for c in range(chunks):
+        s = slice(c * chunk, (c + 1) * chunk)
+        one = exchange(x[s], b[s] if with_b else None)
+        assert all(torch.equal(t, o) for t, o in zip((q[s], lut[c:c + 1], q2[s], lut2[c:c + 1], g[s]), one)), c
+    ops.check_status()
