@@ -32,10 +32,14 @@ def _attention_case(starts, M, H, KV, hd, seed=0):
     ops.check_status()
     (gref,) = torch.autograd.grad(ref, x, dout.float())
     gref = ops.rope_(gref.cpu(), table.cpu(), M, H + KV, hd, backward=True).cuda()
+    qk, v = qkv[:, : (H + KV) * hd].float().abs().max(), qkv[:, (H + KV) * hd:].float().view(M, KV, hd).repeat_interleave(H // KV, 1)
+    dp = (dout.float().view(M, H, hd) * v).sum(-1).abs().max()
     for cols in (slice(0, H * hd), slice(H * hd, (H + KV) * hd), slice((H + KV) * hd, None)):
-        # (a row that sees only itself has P = 1 and dS = 0: nothing but rounding in dQ and dK)
+        # a row that sees only itself has P = 1 and dS = 0: nothing but rounding in dQ and dK, a bf16 unit (2^-8) of P and one of O at most
         if len(starts) < M or cols.stop is None:
             assert _rel(g[:, cols], gref[:, cols]) < 2e-2
+        else:
+            assert g[:, cols].float().abs().max().item() <= 2 * 2.0 ** -8 * (H // KV) * (dp * qk).item() * hd ** -0.5      # (false for NaN)
 
 
 # The forward takes two 128-row query tiles at a time: one tile only, an odd number of them, a last tile of one row, documents that
