@@ -204,9 +204,9 @@ def _narrow_swiglu_pays(M: int, F: int, K: int, pairs: int) -> bool:
 
 def _gemm_epi(a, b, out, M, N, K, b_mn, epi, i0, i1, i2, aux, what, aux2=None, a_mn=False):
     # what the C entry cannot see from addresses and pitches, for the products that would otherwise have gone through gemm() too
-    assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.stride(-1) == 1 and b.stride(-1) == 1
-    assert tuple(a.shape) == ((K, M) if a_mn else (M, K)) and tuple(b.shape) == ((K, N) if b_mn else (N, K)), "operands do not fit each other"
-    assert out is None or out.dtype == torch.bfloat16
+    bf16 = torch.bfloat16
+    assert a.dtype is bf16 and b.dtype is bf16 and a.stride(1) == 1 and b.stride(1) == 1 and (out is None or out.dtype is bf16)
+    assert a.shape[0 if a_mn else 1] == b.shape[0 if b_mn else 1] == K, "inner dimensions differ"
     rc = native.cuda().pb_gemm_bf16_pair_epi(ptr(a), ptr(b), ptr(out), None, M, N, K, a.stride(0), b.stride(0),
                                              out.stride(0) if out is not None else 0, 0, int(a_mn), int(b_mn), 0, 0, epi, i0, i1, i2,
                                              ptr(aux), aux.stride(0) if aux.dim() == 2 else 0, ptr(aux2),
