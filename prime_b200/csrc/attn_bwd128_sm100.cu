@@ -13,8 +13,10 @@
 // so that between "P and dS are there" of two pairs stand the four MMAs, one read of dP, and dS = P (dP - D). With one Q / dO
 // stage, S and dP issued together and dQ in the place of S (the earlier form of this kernel) every step waited for the one before:
 // whole backward, 8 x 2048 tokens, 16 heads 771 -> 626 us, 1 x 8192, 32 / 8 heads 2733 -> 2047.
-// What bounds it: shared memory. The five MMAs of a pair read 2560 cycles' worth of operands there, which is what they need at full
-// rate; P, dS, the dQ boxes (written and sent) and the next Q and dO are another 2000.
+// What bounds it: the chain, no unit is full. A pair takes 7400 cycles (8 x 2048 tokens, 16 heads), of which the five MMAs need 2560
+// (tensor pipe 35 %); the way of the dQ sums to L2 is busy for 45 %, the data banks of shared memory and L1 read for 20 % and written
+// for 10 %. A softmax warp spends half of its time waiting for tensor memory: dP(i+1) follows the read of dQ(i), which follows dS(i),
+// which follows dP(i).
 #include "attn_bwd.cuh"
 
 namespace pb {

@@ -465,9 +465,9 @@ __global__ void attn_bwd_finish_kernel(const float* __restrict__ dq_acc, __nv_bf
 // nq[kv_tile] = number of query tiles that can see the kv tile: the diagonal tile plus every later tile whose first
 // row's sequence starts at or before the tile's last kv row (seq_start is non-decreasing). One warp per kv tile, 32
 // candidate tiles per step (one load latency per 32 tiles instead of one per tile). Also zeroes the work counter and
-// the dQ accumulator (n16 vectors of 16 bytes): a memset would break the chain of early launches and cost a launch of its own. Whole
-// backward with the memset and with this, L2 flushed: 16 x 1024 tokens, 8 heads of 64 152.5 -> 150.5 us; 8 x 2048, 16 heads of
-// 128 767 -> 769; 64 x 1024, 16 heads of 64 (268 MB to zero) 974 -> 977, where the memset streams a little better.
+// the dQ accumulator (n16 vectors of 16 bytes): a memset would break the chain of early launches and cost a launch of its own. Against
+// the memset, L2 flushed, a whole backward takes 2 us less at 16 x 1024 tokens, 8 heads of 64, 2 us more at 8 x 2048, 16 heads of 128, and
+// 3 us more at 64 x 1024, 16 heads of 64 (268 MB to zero), where the memset streams a little better.
 __global__ void __launch_bounds__(256) attn_bwd_span_kernel(const int* __restrict__ seq_start, int n_tiles, int* __restrict__ nq, int* counter,
                                                             uint4* __restrict__ dq_acc, long long n16) {
     pdl_sync();

@@ -26,7 +26,7 @@ struct AttnFwd128Cfg {
     // TMEM columns of the two query tiles: S (fp32) 128 each from 0, O (fp32) 128 each from 256. P (bf16 pairs, A operand of the PV
     // MMA) takes the place of S, whose row the softmax thread already holds, and the next S follows PV. Two CTAs per SM with
     // a tile each (the earlier form) had the same overlap, but fetched every K and V tile twice, into one stage:
-    // 8 x 2048 tokens, 16 heads 227 -> 205 us; 1 x 8192, 32 / 8 heads 712 -> 675.
+    // 8 x 2048 tokens, 16 heads 227 -> 190 us; 1 x 8192, 32 / 8 heads 702 -> 606.
 };
 
 __device__ __forceinline__ void fwd_reg_dealloc_56() { asm volatile("setmaxnreg.dec.sync.aligned.u32 56;"); }
@@ -426,9 +426,9 @@ attn_fwd128_kernel(const __grid_constant__ CUtensorMap tm, const AttnFwdParams p
 
 // Two tiles per CTA, but one where every tile then has an SM to itself. CTAs are numbered with the head running fastest, so that the
 // long rows of all heads start first and the short ones fill the end: with the tiles running fastest the last heads' longest pairs
-// started late, and from 150 to 1000 tiles of long rows two to a CTA lost 5-8 % against one each. One CTA per tile; tiles fastest; heads
+// started late, and from 150 to 800 tiles of long rows two to a CTA lost 2-8 % against one each. One CTA per tile; tiles fastest; heads
 // fastest, us: 1 x 4096 tokens, 16 heads 140, 149, 100; 1 x 8192, 8 heads 246, 268, 187; 32 / 8 heads 703, 666, 606; 64 x 1024, 16 heads
-// 503, 441, 429. What still loses to one CTA per tile: up to two tiles per SM of one long row (1 x 4096, 8 heads 94 and 98; one
+// 503, 441, 429. What still loses to one CTA per tile: up to two tiles per SM of long rows (1 x 4096, 8 heads 94 and 98; one
 // tile per CTA takes 72 there, but 45 instead of 35 at 37 x 777, one head, and the launch does not know where rows end), and rows of
 // 128 tokens (8 x 128, 8 heads, one launch behind the other, 7.3 and 7.8).
 int launch_attn_fwd128(const CUtensorMap& tm, const AttnFwdParams& p, cudaStream_t st) {

@@ -926,11 +926,12 @@ class FusedLlama:
     def _graphable(self, tokens, labels, seq_start, n_micro: int) -> bool:
         """Small steps without peers are replayed as one graph launch: a launch costs the host 14 us through the Python wrappers, so
         a step whose kernels average less than that waits for the host (two-block model, 512 tokens: 60 launches of this
-        package, 0.86 ms of host and 0.91 ms in all, replayed 0.37; debug model of 16 x 1024: 131 launches, 1.83 of 1.91 ms,
-        replayed 1.39). The line: twice the host time, at 13 us a launch, against the step's operations at a middling
+        package, 0.86 ms of host and 0.92 ms in all, replayed 0.27; debug model of 16 x 1024: 131 launches, 1.83 of 1.97 ms,
+        replayed 1.17). The line: twice the host time, at 13 us a launch, against the step's operations at a middling
         600 TFLOP/s. Above it the queue does not run dry, and what a graph saves is the 0.3 ms around each step's read of its
-        loss, in ms, replayed and one by one: below the line 70M 4 x 1024 tokens 2.47 and 2.77, 8 x 1024 3.5 and 3.65, 150M
-        2 x 1024 6.25 and 6.57; above it 70M 16 x 1024 6.2 and 6.4, 150M 4 x 1024 9.1 and 9.4, 6 x 1024 12.8 and 13.2."""
+        loss and what its branch of weight gradients gains; in ms, replayed and one by one: below the line 70M 4 x 1024 tokens
+        2.30 and 2.85, 8 x 1024 3.37 and 3.65, 150M 2 x 1024 5.91 and 6.57; above it 70M 16 x 1024 5.98 and 6.21, 150M 4 x 1024
+        8.69 and 9.04, 6 x 1024 12.6 and 12.9, 16 x 1024 29.0 and 28.8."""
         if not (self._direct_update and self.wgrad_stream is None and not self._accum and tokens.is_cuda and labels.is_cuda
                 and tokens.dtype == torch.int64 and labels.dtype == torch.int64 and tokens.device == self._counters.device
                 and (seq_start is None or (seq_start.is_cuda and seq_start.dtype == torch.int32))):
